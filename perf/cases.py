@@ -86,8 +86,9 @@ def draw(rng):
     n = _pick_n(rng, dim, 208 if dim == 2 else 48 if k == 1 else 24)
     if kind == "precond":
         return dict(kind="precond", dim=dim, n=n, k=k, nu=rng.choice([1, 2, 3]), precision=rng.choice(["fp32", "df", "fp64"]))
-    if kind in ("condense", "post"):
-        return dict(kind=kind, dim=dim, n=n, k=k)
+    if kind in ("condense", "post"):   # no hierarchy below the mesh: any size
+        lo, hi = (12, 256) if dim == 2 else (6, 48 if k == 1 else 24)
+        return dict(kind=kind, dim=dim, n=int(round(lo * (hi / lo) ** rng.random())), k=k)
     case = _solve("", dim=dim, n=n, k=k, precision=rng.choice(["fp64", "df", "fp32"]), nu=rng.choice([1, 1, 2, 3]),
                   io=rng.choice(["host", "device"]), autotune=rng.random() < 0.25)
     del case["name"]
@@ -295,14 +296,10 @@ def _run_condense(s):
 def _face_solution(case):
     """The discrete solution of the sine source, in the given numbering."""
     def make():
-        H = hho.Hierarchy(case["dim"], case["n"], case["k"])
-        As, Ps = [H.A(l) for l in range(H.levels)], [H.P(l) for l in range(H.levels - 1)]
-        b, bs = H.b(), H.block_size
+        H = hho.Hierarchy(case["dim"], case["n"], case["k"], max_levels=1)
+        A, b = H.A(0), H.b()
         H.close()
-        solver = S.fcg_mg(As, Ps, bs, precision="df")
-        x = solver.Solve(b)
-        solver.Context().close()
-        return x
+        return _pcg(A, b)
     return _keep(("face solution", case["dim"], case["n"], case["k"]), make)
 
 
