@@ -23,13 +23,12 @@ from fhhos4_gb300 import hho
 from fhhos4_gb300 import learned as LN
 from fhhos4_gb300 import solver as S
 
-TOL = 1e-8
 MAXIT = 200
 
 
 def _solve(name, **kw):
     case = dict(name=name, kind="solve", dim=3, n=16, k=1, coefficient="identity", contrast=1.0, precision="fp64",
-                nu=1, coarse_nu=-1, galerkin=False, p_multigrid=False, learned=False, autotune=False, io="device")
+                nu=1, coarse_nu=-1, galerkin=False, p_multigrid=False, learned=False, autotune=False, tol=1e-8, io="device")
     case.update(kw)
     return case
 
@@ -79,7 +78,7 @@ def draw(rng):
     """One more case of the listed ranges."""
     kind = rng.choice(["solve"] * 7 + ["batch", "precond", "condense", "post"])
     if kind == "batch":
-        return dict(kind="batch", problems=rng.randint(2, 32), n_max=16 * rng.randint(2, 6),
+        return dict(kind="batch", problems=rng.randint(2, 32), n_max=16 * rng.randint(3, 6),
                     precision=rng.choice(["fp32", "df", "fp64"]), spec_seed=rng.randint(1, 10 ** 6))
     dim = rng.choice([2, 3, 3])
     k = rng.choice([1, 2, 3]) if dim == 2 else rng.choice([1, 1, 2])
@@ -90,7 +89,7 @@ def draw(rng):
         lo, hi = (12, 256) if dim == 2 else (6, 48 if k == 1 else 24)
         return dict(kind=kind, dim=dim, n=int(round(lo * (hi / lo) ** rng.random())), k=k)
     case = _solve("", dim=dim, n=n, k=k, precision=rng.choice(["fp64", "df", "fp32"]), nu=rng.choice([1, 1, 2, 3]),
-                  io=rng.choice(["host", "device"]), autotune=rng.random() < 0.25)
+                  io=rng.choice(["host", "device"]), autotune=rng.random() < 0.25, tol=rng.choice([1e-6, 1e-7, 1e-8, 1e-8, 1e-9]))
     del case["name"]
     if case["nu"] == 3:
         case["coarse_nu"] = 4
@@ -172,7 +171,7 @@ def _hierarchy(case):
 def _solver(case):
     def make():
         As, Ps, bs, cnu = (got := _hierarchy(case))[:4]
-        solver = S.fcg_mg(As, Ps, bs, tol=TOL, maxit=MAXIT, precision=case["precision"], nu=(case["nu"], case["nu"]),
+        solver = S.fcg_mg(As, Ps, bs, tol=case.get("tol", 1e-8), maxit=MAXIT, precision=case["precision"], nu=(case["nu"], case["nu"]),
                           coarse_nu=cnu, galerkin=case.get("galerkin", False), autotune=case.get("autotune", False),
                           replace_residual=case.get("galerkin", False))
         if case.get("learned"):
