@@ -13,12 +13,12 @@
 //      S = A_FF - A_TF^T (A_TT^{-1} A_TF) and the source map G = -A_TF^T A_TT^{-1}
 //      (n_face_dofs x n_cell) are kept;
 //   2. per face block row: the sorted union of the unknown faces of its two elements is the row's
-//      block columns (counted, then offsets by a three-pass scan);
+//      block columns (counted per CTA, then the CTAs' offsets by a scan);
 //   3. per face block row: the values, S of the first element then of the second added into the
 //      row's positions in that order, and b_I = sum over the two elements of G b_T, restricted to
 //      the face's rows (the same order as the host assembly, so off-diagonal blocks are copies and
 //      diagonal blocks one addition).
-// Every row is written by one thread: no atomics, the result is bitwise reproducible. The output is
+// Every entry is written once by one thread: no atomics, the result is bitwise reproducible. The output is
 // the scalar CSR the solve phase takes (fhg_set_level): rows I * nf + a, columns J * nf + c.
 #include <cuda_runtime.h>
 
@@ -49,65 +49,78 @@ struct CondData {
     int* status;           // 1: a singular A_TT
 };
 
-// Step 1, one thread per class: Gauss-Jordan elimination with partial pivoting of [A_TT | I] gives
-// A_TT^{-1}; then S = A_FF - A_TF^T (A_TT^{-1} A_TF) and G = -A_TF^T A_TT^{-1}. NC = cell unknowns.
+// Step 1, one CTA per class: Gauss-Jordan elimination with partial pivoting of [A_TT | I] in shared
+// memory gives A_TT^{-1}; then X = A_TT^{-1} A_TF, S = A_FF - A_TF^T X and G = -A_TF^T A_TT^{-1}, one
+// entry per thread. NC = cell unknowns. A mesh has a few classes (tens), so a class is a serial chain
+// of NC pivots whatever the launch: spreading a pivot's rows and the products over a CTA leaves NC
+// barriers (one thread per class ran all of it, nFF NC (NC + nFF) multiply-adds, one after another).
+// The sums run in the same order, so the values are the same bits.
+constexpr int kClassThreads = 128;
+
 template <int NC>
-__global__ void __launch_bounds__(64) k_condense_classes(CondData D)
+__global__ void __launch_bounds__(kClassThreads) k_condense_classes(CondData D)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= D.ncls) return;
+    __shared__ double M[NC][NC], V[NC][NC], f[NC], X[NC][kCondMaxFaceDofs];
+    __shared__ int piv;
+    const int c = blockIdx.x, tid = threadIdx.x;
     const int nFF = D.nFF, nH = NC + nFF;
     const double* A = D.local + (long long)c * nH * nH;
-    double M[NC][NC], V[NC][NC];
-    for (int i = 0; i < NC; i++)
-        for (int j = 0; j < NC; j++) {
-            M[i][j] = A[i * nH + j];
-            V[i][j] = i == j ? 1.0 : 0.0;
-        }
+    for (int e = tid; e < NC * NC; e += kClassThreads) {
+        const int i = e / NC, j = e % NC;
+        M[i][j] = A[i * nH + j];
+        V[i][j] = i == j ? 1.0 : 0.0;
+    }
+    __syncthreads();
     for (int k = 0; k < NC; k++) {
-        int piv = k;
-        for (int i = k + 1; i < NC; i++)
-            if (fabs(M[i][k]) > fabs(M[piv][k])) piv = i;
-        if (M[piv][k] == 0.0) {
-            atomicExch(D.status, 1);
+        if (tid == 0) {
+            int p = k;
+            for (int i = k + 1; i < NC; i++)
+                if (fabs(M[i][k]) > fabs(M[p][k])) p = i;
+            piv = M[p][k] == 0.0 ? -1 : p;
+        }
+        __syncthreads();
+        const int p = piv;
+        if (p < 0) {   // the whole CTA leaves together
+            if (tid == 0) atomicExch(D.status, 1);
             return;
         }
-        if (piv != k)
-            for (int j = 0; j < NC; j++) {
-                double t = M[k][j]; M[k][j] = M[piv][j]; M[piv][j] = t;
-                t = V[k][j]; V[k][j] = V[piv][j]; V[piv][j] = t;
-            }
-        const double inv = 1.0 / M[k][k];
-        for (int j = 0; j < NC; j++) { M[k][j] *= inv; V[k][j] *= inv; }
-        for (int i = 0; i < NC; i++) {
-            if (i == k) continue;
-            const double f = M[i][k];
-            if (f == 0.0) continue;
-            for (int j = 0; j < NC; j++) { M[i][j] -= f * M[k][j]; V[i][j] -= f * V[k][j]; }
+        if (tid < NC && p != k) {
+            double t = M[k][tid]; M[k][tid] = M[p][tid]; M[p][tid] = t;
+            t = V[k][tid]; V[k][tid] = V[p][tid]; V[p][tid] = t;
         }
+        __syncthreads();
+        const double inv = 1.0 / M[k][k];
+        if (tid < NC && tid != k) f[tid] = M[tid][k];
+        __syncthreads();
+        if (tid < NC) { M[k][tid] *= inv; V[k][tid] *= inv; }
+        __syncthreads();
+        for (int e = tid; e < NC * NC; e += kClassThreads) {
+            const int i = e / NC, j = e % NC;
+            if (i == k || f[i] == 0.0) continue;
+            M[i][j] -= f[i] * M[k][j];
+            V[i][j] -= f[i] * V[k][j];
+        }
+        __syncthreads();
     }
-    // V = A_TT^{-1}; X(:, j) = V A_TF(:, j) formed column by column
     double* S = D.S + (long long)c * nFF * nFF;
     double* G = D.G + (long long)c * nFF * NC;
-    for (int j = 0; j < nFF; j++) {
-        double x[NC];
-        for (int t = 0; t < NC; t++) {
-            double v = 0.0;
-            for (int u = 0; u < NC; u++) v += V[t][u] * A[u * nH + NC + j];
-            x[t] = v;
-        }
-        for (int i = 0; i < nFF; i++) {
-            double s = A[(NC + i) * nH + NC + j];
-            for (int t = 0; t < NC; t++) s -= A[t * nH + NC + i] * x[t];
-            S[i * nFF + j] = s;
-        }
+    for (int e = tid; e < NC * nFF; e += kClassThreads) {
+        const int t = e / nFF, j = e % nFF;
+        double v = 0.0;
+        for (int u = 0; u < NC; u++) v += V[t][u] * A[u * nH + NC + j];
+        X[t][j] = v;
+        double g = 0.0;
+        const int i = e / NC, q = e % NC;
+        for (int u = 0; u < NC; u++) g += A[u * nH + NC + i] * V[u][q];
+        G[e] = -g;   // entry (i, q)
     }
-    for (int i = 0; i < nFF; i++)
-        for (int j = 0; j < NC; j++) {
-            double v = 0.0;
-            for (int t = 0; t < NC; t++) v += A[t * nH + NC + i] * V[t][j];
-            G[i * NC + j] = -v;
-        }
+    __syncthreads();
+    for (int e = tid; e < nFF * nFF; e += kClassThreads) {
+        const int i = e / nFF, j = e % nFF;
+        double v = A[(NC + i) * nH + NC + j];
+        for (int t = 0; t < NC; t++) v -= A[t * nH + NC + i] * X[t][j];
+        S[e] = v;
+    }
 }
 
 // The sorted block columns of face row I (the unknown faces of its two elements).
@@ -134,107 +147,152 @@ __device__ int row_columns(const CondData& D, int I, int* cols)
     return n;
 }
 
-// Step 2: block columns per face row.
-__global__ void __launch_bounds__(kCondThreads) k_count(CondData D, int* counts)
+// Step 2: block columns of the kCondThreads face rows of every CTA, summed.
+__global__ void __launch_bounds__(kCondThreads) k_count(CondData D, long long* totals)
 {
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
-    if (I >= D.nI) return;
+    __shared__ int sh[kCondThreads / 32];
+    const int I = blockIdx.x * kCondThreads + threadIdx.x;
     int cols[kCondMaxRowBlocks];
-    counts[I] = row_columns(D, I, cols);
-}
-
-// Three-pass exclusive scan: per-CTA totals, a scan of the totals by one CTA, per-CTA scans with
-// the offsets added. out[n] = total.
-__global__ void __launch_bounds__(kCondThreads) k_scan_totals(const int* in, int n, long long* totals)
-{
-    __shared__ long long sh[kCondThreads];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    sh[threadIdx.x] = i < n ? in[i] : 0;
+    int n = I < D.nI ? row_columns(D, I, cols) : 0;
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = n;
     __syncthreads();
-    for (int o = kCondThreads / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        long long t = 0;
+        for (int w = 0; w < kCondThreads / 32; w++) t += sh[w];
+        totals[blockIdx.x] = t;
     }
-    if (threadIdx.x == 0) totals[blockIdx.x] = sh[0];
 }
 
-__global__ void k_scan_offsets(long long* totals, int nblocks)
+// Exclusive scan of the totals by one CTA, in place; totals[nblocks] = the sum. Each thread sums a
+// contiguous chunk, the chunk sums are scanned, and the chunk is written back.
+constexpr int kScanThreads = 1024;
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_offsets(long long* totals, int nblocks)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    long long run = 0;
-    for (int b = 0; b < nblocks; b++) {
+    __shared__ long long warp_sum[kScanThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int chunk = (nblocks + kScanThreads - 1) / kScanThreads;
+    const int lo = min(tid * chunk, nblocks), hi = min(lo + chunk, nblocks);
+    long long sum = 0;
+    for (int b = lo; b < hi; b++) sum += totals[b];
+    long long run = sum;   // inclusive scan over the warp, then over the warps
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long t = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += t;
+    }
+    if (lane == 31) warp_sum[warp] = run;
+    __syncthreads();
+    if (warp == 0) {
+        long long w = warp_sum[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long t = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += t;
+        }
+        warp_sum[lane] = w;
+    }
+    __syncthreads();
+    if (tid == kScanThreads - 1) totals[nblocks] = warp_sum[kScanThreads / 32 - 1];
+    run += (warp ? warp_sum[warp - 1] : 0) - sum;
+    for (int b = lo; b < hi; b++) {
         const long long t = totals[b];
         totals[b] = run;
         run += t;
     }
-    totals[nblocks] = run;
 }
 
-__global__ void __launch_bounds__(kCondThreads) k_scan_apply(const int* in, int n, const long long* offsets, long long* out)
-{
-    __shared__ long long sh[kCondThreads];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const long long v = i < n ? in[i] : 0;
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < kCondThreads; o <<= 1) {   // inclusive Hillis-Steele scan
-        const long long t = (int)threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-        __syncthreads();
-        sh[threadIdx.x] += t;
-        __syncthreads();
-    }
-    if (i < n) out[i] = offsets[blockIdx.x] + sh[threadIdx.x] - v;
-    if (i == n - 1) out[n] = offsets[blockIdx.x] + sh[threadIdx.x];
-}
-
-// Step 3: row I's scalar rows, column indices, values and right-hand side.
-__global__ void __launch_bounds__(kCondThreads) k_fill(CondData D, const long long* block_start, int* rowptr,
+// Step 3: the scalar rows, column indices, values and right-hand side of kCondThreads face rows. The
+// output is 12 bytes per entry and far larger than anything read (the class tables stay in L1), so
+// the writes decide: a CTA first finds its rows' columns and sources one thread per row (shared
+// memory), then each warp writes one face row's entries, which are contiguous, 32 at a time. One
+// thread per face row, which cleared and then added to its own ~63 entries, and a serial scan of the
+// offsets took a 48^3, k = 1 assembly (82 M entries, 0.98 GB) 2.56 ms; now 0.55 ms. NF: face DOFs (0: any).
+template <int NF>
+__global__ void __launch_bounds__(kCondThreads) k_fill(CondData D, const long long* offsets, int* rowptr,
                                                        int* colidx, double* vals, double* b)
 {
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
-    if (I >= D.nI) return;
-    const int nf = D.nf, nC = D.nC, nFF = D.nFF;
-    int cols[kCondMaxRowBlocks];
-    const int nb = row_columns(D, I, cols);
-    const long long base = block_start[I] * nf * nf;   // first scalar entry of the block row
-    const int width = nb * nf;                         // scalar entries per row
-    for (int a = 0; a < nf; a++) {
-        const long long r0 = base + (long long)a * width;
-        rowptr[(long long)I * nf + a] = (int)r0;
-        for (int q = 0; q < nb; q++)
-            for (int cc = 0; cc < nf; cc++) {
-                colidx[r0 + q * nf + cc] = cols[q] * nf + cc;
-                vals[r0 + q * nf + cc] = 0.0;
+    struct Row {
+        int col[kCondMaxRowBlocks];     // block columns
+        unsigned lf0, lf1;              // 4 bits per column: its local face in element 1 / 2 (15: none)
+        long long s0, s1;               // first entry of S of element 1 / 2 at the face's rows
+        int nb, start;                  // block columns; blocks before this row in the CTA
+    };
+    __shared__ Row rows[kCondThreads];
+    __shared__ int warp_sum[kCondThreads / 32];
+    const int nf = NF ? NF : D.nf, nC = D.nC, nFF = D.nFF;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int I = blockIdx.x * kCondThreads + tid;
+    const long long block0 = offsets[blockIdx.x];
+    Row& R = rows[tid];
+    int nb = 0;
+    if (I < D.nI) {
+        int cols[kCondMaxRowBlocks];
+        nb = row_columns(D, I, cols);
+#pragma unroll
+        for (int q = 0; q < kCondMaxRowBlocks; q++) R.col[q] = q < nb ? cols[q] : 0;
+        unsigned lfs[2] = {0xffffffffu, 0xffffffffu};
+        long long first[2] = {0, 0};
+        double acc[NF ? NF : kCondMaxFaceDofs];
+        for (int a = 0; a < nf; a++) acc[a] = 0.0;
+        for (int side = 0; side < 2; side++) {
+            const int e = D.face_elems[(long long)I * 4 + 2 * side];
+            const int lfi = D.face_elems[(long long)I * 4 + 2 * side + 1];
+            if (e < 0 || lfi < 0) continue;
+            const int c = D.cls[e];
+            first[side] = ((long long)c * nFF + lfi * nf) * nFF;
+            for (int lf = 0; lf < D.nF; lf++) {
+                const int g = D.elem_faces[(long long)e * D.nF + lf];
+                if (g < 0) continue;
+                int q = 0;
+                while (q < nb && cols[q] != g) q++;
+                lfs[side] = (lfs[side] & ~(15u << (4 * q))) | ((unsigned)lf << (4 * q));
             }
-    }
-    if (I == D.nI - 1) rowptr[(long long)D.nI * nf] = (int)(base + (long long)nf * width);
-    double bI[kCondMaxFaceDofs];
-    for (int a = 0; a < nf; a++) bI[a] = 0.0;
-    for (int side = 0; side < 2; side++) {
-        const int e = D.face_elems[(long long)I * 4 + 2 * side];
-        const int lfi = D.face_elems[(long long)I * 4 + 2 * side + 1];
-        if (e < 0 || lfi < 0) continue;
-        const int c = D.cls[e];
-        const double* S = D.S + (long long)c * nFF * nFF;
-        const double* G = D.G + (long long)c * nFF * nC;
-        for (int lf = 0; lf < D.nF; lf++) {
-            const int g = D.elem_faces[(long long)e * D.nF + lf];
-            if (g < 0) continue;
-            int q = 0;
-            while (q < nb && cols[q] != g) q++;
+            const double* G = D.G + ((long long)c * nFF + lfi * nf) * nC;
+            const double* bT = D.b_cell + (long long)e * nC;
             for (int a = 0; a < nf; a++) {
-                double* dst = vals + base + (long long)a * width + q * nf;
-                for (int cc = 0; cc < nf; cc++) dst[cc] += S[(lfi * nf + a) * nFF + lf * nf + cc];
+                double s = 0.0;
+                for (int t = 0; t < nC; t++) s += G[a * nC + t] * bT[t];
+                acc[a] += s;
             }
         }
-        const double* bT = D.b_cell + (long long)e * nC;
-        for (int a = 0; a < nf; a++) {
-            double s = 0.0;
-            for (int t = 0; t < nC; t++) s += G[(lfi * nf + a) * nC + t] * bT[t];
-            bI[a] += s;
+        for (int a = 0; a < nf; a++) b[(long long)I * nf + a] = acc[a];
+        R.lf0 = lfs[0]; R.lf1 = lfs[1];
+        R.s0 = first[0]; R.s1 = first[1];
+    }
+    R.nb = nb;
+    int run = nb;   // blocks of the CTA's rows up to this one
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += t;
+    }
+    if (lane == 31) warp_sum[warp] = run;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) run += warp_sum[w];
+    R.start = run - nb;
+    if (I < D.nI) {
+        const long long base = (block0 + R.start) * nf * nf;
+        for (int a = 0; a < nf; a++) rowptr[(long long)I * nf + a] = (int)(base + (long long)a * nb * nf);
+        if (I == D.nI - 1) rowptr[(long long)D.nI * nf] = (int)(base + (long long)nb * nf * nf);
+    }
+    __syncthreads();
+    const int n = min(kCondThreads, D.nI - (int)blockIdx.x * kCondThreads);
+    for (int r = warp; r < n; r += kCondThreads / 32) {
+        const Row& W = rows[r];
+        const long long base = (block0 + W.start) * nf * nf;
+        const int width = W.nb * nf, count = width * nf;
+        // e / width by a rounded-up reciprocal: exact for e < 2^20 / width (count <= 8 * 13 * 13)
+        const unsigned inv = ((1u << 20) + width - 1) / max(width, 1);
+        for (int e = lane; e < count; e += 32) {
+            const int a = (int)(((unsigned)e * inv) >> 20), j = e - a * width;
+            const int q = j / nf, cc = j - q * nf;
+            const unsigned f0 = (W.lf0 >> (4 * q)) & 15u, f1 = (W.lf1 >> (4 * q)) & 15u;
+            double v = 0.0;
+            if (f0 != 15u) v += D.S[W.s0 + a * nFF + (int)f0 * nf + cc];
+            if (f1 != 15u) v += D.S[W.s1 + a * nFF + (int)f1 * nf + cc];
+            colidx[base + e] = W.col[q] * nf + cc;
+            vals[base + e] = v;
         }
     }
-    for (int a = 0; a < nf; a++) b[(long long)I * nf + a] = bI[a];
 }
 
 }  // namespace
@@ -244,9 +302,7 @@ struct fhg_cond {
     std::string err;
     CondData D{};
     std::vector<void*> allocs;
-    int* counts = nullptr;
-    long long* block_start = nullptr;
-    long long* totals = nullptr;
+    long long* totals = nullptr;   // block columns before every CTA's rows, then their sum
     int* rowptr = nullptr;
     int* colidx = nullptr;
     double* vals = nullptr;
@@ -347,8 +403,7 @@ int fhg_cond_create(fhg_cond** out, int device, int dim, int n_elements, int n_c
         (rc = dev_upload(p, face_elems, (size_t)n_face_blocks * 4, &D.face_elems)) ||
         (rc = dev_upload(p, local, nc * nH * nH, &D.local)) || (rc = dev_upload(p, b_cell, ne * n_cell, &D.b_cell)) ||
         (rc = dev_alloc(p, &D.S, nc * n_face_dofs * n_face_dofs)) || (rc = dev_alloc(p, &D.G, nc * n_face_dofs * n_cell)) ||
-        (rc = dev_alloc(p, &D.status, 1)) || (rc = dev_alloc(p, &p->counts, (size_t)n_face_blocks)) ||
-        (rc = dev_alloc(p, &p->block_start, (size_t)n_face_blocks + 1)) ||
+        (rc = dev_alloc(p, &D.status, 1)) ||
         (rc = dev_alloc(p, &p->totals, (size_t)(n_face_blocks + kCondThreads - 1) / kCondThreads + 1)) ||
         (rc = dev_alloc(p, &p->b, (size_t)n_face_blocks * D.nf)) ||
         (rc = dev_alloc(p, &p->rowptr, (size_t)n_face_blocks * D.nf + 1)))
@@ -369,23 +424,20 @@ int fhg_cond_run(fhg_cond* p, long long* nnz, double* elapsed_ms)
     cudaStream_t s = p->stream;
     DCK(cudaMemsetAsync(D.status, 0, sizeof(int), s));
     DCK(cudaEventRecord(p->ev0, s));
-    const int cgrid = (D.ncls + 63) / 64;
     switch (D.nC) {
-    case 3: k_condense_classes<3><<<cgrid, 64, 0, s>>>(D); break;
-    case 4: k_condense_classes<4><<<cgrid, 64, 0, s>>>(D); break;
-    case 6: k_condense_classes<6><<<cgrid, 64, 0, s>>>(D); break;
-    case 10: k_condense_classes<10><<<cgrid, 64, 0, s>>>(D); break;
-    case 20: k_condense_classes<20><<<cgrid, 64, 0, s>>>(D); break;
+    case 3: k_condense_classes<3><<<D.ncls, kClassThreads, 0, s>>>(D); break;
+    case 4: k_condense_classes<4><<<D.ncls, kClassThreads, 0, s>>>(D); break;
+    case 6: k_condense_classes<6><<<D.ncls, kClassThreads, 0, s>>>(D); break;
+    case 10: k_condense_classes<10><<<D.ncls, kClassThreads, 0, s>>>(D); break;
+    case 20: k_condense_classes<20><<<D.ncls, kClassThreads, 0, s>>>(D); break;
     default: return cond_fail(p, FHG_ERR_UNSUPPORTED, "%d cell unknowns per element", D.nC);
     }
-    k_count<<<grid, kCondThreads, 0, s>>>(D, p->counts);
-    k_scan_totals<<<grid, kCondThreads, 0, s>>>(p->counts, nI, p->totals);
-    k_scan_offsets<<<1, 32, 0, s>>>(p->totals, grid);
-    k_scan_apply<<<grid, kCondThreads, 0, s>>>(p->counts, nI, p->totals, p->block_start);
+    k_count<<<grid, kCondThreads, 0, s>>>(D, p->totals);
+    k_scan_offsets<<<1, kScanThreads, 0, s>>>(p->totals, grid);
     DCK(cudaGetLastError());
     long long blocks = 0;
     int status = 0;
-    DCK(cudaMemcpyAsync(&blocks, p->block_start + nI, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    DCK(cudaMemcpyAsync(&blocks, p->totals + grid, sizeof(long long), cudaMemcpyDeviceToHost, s));
     DCK(cudaMemcpyAsync(&status, D.status, sizeof(int), cudaMemcpyDeviceToHost, s));
     DCK(cudaStreamSynchronize(s));
     if (status) return cond_fail(p, FHG_ERR_SINGULAR_BLOCK, "singular cell block in a local operator");
@@ -403,7 +455,13 @@ int fhg_cond_run(fhg_cond* p, long long* nnz, double* elapsed_ms)
         if ((rc = dev_alloc(p, &p->colidx, (size_t)n_scalar)) || (rc = dev_alloc(p, &p->vals, (size_t)n_scalar))) return rc;
         p->nnz = n_scalar;
     }
-    k_fill<<<grid, kCondThreads, 0, s>>>(D, p->block_start, p->rowptr, p->colidx, p->vals, p->b);
+    switch (nf) {   // the face blocks of the supported degrees; any other size by the general kernel
+    case 2: k_fill<2><<<grid, kCondThreads, 0, s>>>(D, p->totals, p->rowptr, p->colidx, p->vals, p->b); break;
+    case 3: k_fill<3><<<grid, kCondThreads, 0, s>>>(D, p->totals, p->rowptr, p->colidx, p->vals, p->b); break;
+    case 4: k_fill<4><<<grid, kCondThreads, 0, s>>>(D, p->totals, p->rowptr, p->colidx, p->vals, p->b); break;
+    case 6: k_fill<6><<<grid, kCondThreads, 0, s>>>(D, p->totals, p->rowptr, p->colidx, p->vals, p->b); break;
+    default: k_fill<0><<<grid, kCondThreads, 0, s>>>(D, p->totals, p->rowptr, p->colidx, p->vals, p->b); break;
+    }
     DCK(cudaGetLastError());
     DCK(cudaEventRecord(p->ev1, s));
     DCK(cudaStreamSynchronize(s));

@@ -161,3 +161,33 @@ def test_gpu_condensation_one_class_per_element():
         assert np.abs(A.data - A0.data).max() <= 1e-13 * np.abs(A0.data).max()
     finally:
         cond.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,n,k", [(2, 9, 1), (2, 10, 2), (2, 11, 3), (3, 4, 1), (3, 3, 2), (3, 3, 3)])
+def test_gpu_condensation_of_distinct_elements(dim, n, k):
+    """Every face block size (the general fill kernel for 3D, k = 3), every cell size of the class kernel
+    but none shared between elements, and face counts around and off the 256 rows of a CTA, against the numpy
+    condensation. Tolerance: as the host assembly's, scaled by the elements' spread of values."""
+    from fhhos4_gb300 import _native as N
+    H = hho.Hierarchy(dim, n, k, max_levels=1)
+    try:
+        t = H.condense_tables()
+    finally:
+        H.close()
+    nH, ne = t["n_cell"] + t["n_face_dofs"], t["n_elements"]
+    rng = np.random.default_rng(7)
+    local = t["local"].reshape(-1, nH, nH)[t["elem_class"]] * np.exp(rng.standard_normal(ne))[:, None, None]
+    u = dict(t, n_classes=ne, local=local.ravel().copy(), elem_class=np.arange(ne, dtype=np.int32),
+             b_cell=rng.standard_normal(t["b_cell"].size))
+    A0, b0 = numpy_condense(u)
+    A0.sort_indices()
+    cond = N.Condense(u)
+    try:
+        nnz, _ = cond.run()
+        A, b = cond.result(nnz)
+    finally:
+        cond.close()
+    assert np.array_equal(A.indptr, A0.indptr) and np.array_equal(A.indices, A0.indices)
+    assert np.abs(A.data - A0.data).max() <= 1e-12 * np.abs(A0.data).max()
+    assert np.abs(b - b0).max() <= 1e-12 * np.abs(b0).max()
