@@ -130,3 +130,41 @@ def test_gpu_post_of_gpu_solve():
         assert 1e-4 < err < 1e-2   # the discretisation error of 8^3, k = 1
     finally:
         post.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tables", ["shared", "distinct"])
+@pytest.mark.parametrize("dim,n,k", [(2, 8, 1), (2, 12, 1), (2, 9, 2), (2, 12, 3), (3, 3, 1), (3, 4, 1), (3, 4, 2), (3, 4, 3)])
+def test_gpu_post_with_factorised_and_pointwise_tables(dim, n, k, tables):
+    """Both forms of the L2 sums against numpy at the points, for every element size: "shared" tables
+    are factorised; "distinct" ones (another rule of weights per element) are factorised up to 256 of them
+    (2D n = 8 and n = 9, 3D n = 3) and evaluated at the points above. Face values far from a solution, so
+    nothing cancels: 1e-12 covers the rounding of sums of a few 10^4 positive terms."""
+    import torch
+    from fhhos4_gb300 import _native as N
+    H = hho.Hierarchy(dim, n, k, max_levels=1)
+    try:
+        t = H.post_tables()
+        rows = H.A_rows(0)
+    finally:
+        H.close()
+    ne, nq = t["n_elements"], t["n_points"]
+    rng = np.random.default_rng(11)
+    if tables == "distinct":
+        cls = t["elem_class"]
+        for name, m in (("solve_cells", t["n_cell"] * t["n_face_dofs"]),
+                        ("recon", t["n_recon"] * (t["n_cell"] + t["n_face_dofs"])), ("offsets", nq * 3),
+                        ("basis", nq * t["n_recon"]), ("weights", nq)):
+            t[name] = t[name].reshape(-1, m)[cls].copy()
+        t["weights"] *= 1.0 + 1e-3 * np.arange(ne)[:, None]
+        t["n_classes"], t["elem_class"] = ne, np.arange(ne, dtype=np.int32)
+    x = rng.standard_normal(rows)
+    xc_ref, err_ref = numpy_post(t, x)
+    post = N.Post({k_: (v.ravel() if isinstance(v, np.ndarray) else v) for k_, v in t.items()})
+    try:
+        cells = torch.zeros(ne * t["n_cell"], dtype=torch.float64, device="cuda")
+        err, _ = post.run(torch.tensor(x, device="cuda").data_ptr(), cells.data_ptr(), "sine")
+    finally:
+        post.close()
+    assert np.abs(cells.cpu().numpy().reshape(xc_ref.shape) - xc_ref).max() <= 1e-12 * np.abs(xc_ref).max()
+    assert err == pytest.approx(err_ref, rel=1e-12)
