@@ -69,6 +69,11 @@ struct Level {
     DevBsr<float> A32s;         // FP32 A slot-major (all blocks, one thread per row), when built
     // FP32-pair copies (FHG_PREC_DF: FP64-class V-cycle on the FP32 pipe), same views as FP32
     DevBsr<dfl> A2, P2, R2, G2, A2p, G2s, A2s;
+    // Row-class views of A and of the outer operator (every value type: the dictionaries are small; the
+    // classes and columns are shared), built where the rows repeat often enough (setup).
+    DevBsr<double> C64, Co64;
+    DevBsr<float> C32;
+    DevBsr<dfl> C2, Co2;
     // jagged (JDS) views of the transfers, levels 0 and 1 (the large ones), and whether the products
     // use them (per V-cycle precision, chosen by timing at setup)
     DevBsr<float> P32j, R32j;
@@ -473,6 +478,47 @@ int upload_jds(fhg_ctx* ctx, const HostBsr& B, DevBsr<T>& D)
     return FHG_OK;
 }
 
+// The dictionary of a row-class view in T over classes and columns already on the device.
+template <class T>
+int upload_classes(fhg_ctx* ctx, const HostBsr& B, const RowClasses& C, const std::vector<double>& dict,
+                   const unsigned short* cls, const int* col, DevBsr<T>& D)
+{
+    std::vector<T> vals(dict.size());
+    for (size_t i = 0; i < dict.size(); i++) vals[i] = (T)dict[i];
+    D = DevBsr<T>();
+    int rc = upload(ctx, &D.vals, vals.data(), vals.size());
+    if (rc) return rc;
+    D.owns_index = false;
+    D.v.nbr = B.nbr; D.v.nbc = B.nbc; D.v.bs = B.bs; D.v.nnzb = B.nnzb(); D.v.ld = C.ncls; D.v.ell = C.W;
+    D.v.colidx = col; D.v.vals = D.vals; D.v.cls = cls;
+    D.v.lanes = 1;
+    return FHG_OK;
+}
+
+// Where rows repeat: at least kClassRows rows to a class (the dictionary is then a small part of the
+// streamed operator) and at most kMaxClasses (its FP32 form, 258 KB at 3 x 3 blocks and 6 neighbours, stays
+// in L1 and L2). The operators of a 64^3 mesh with one tensor have 77 classes, of a 4 x 4 x 4
+// checkerboard about 200; one tensor per 4^3 cubes makes 25 to 30 rows to a class, which stay with the
+// stored-block views.
+constexpr int kClassRows = 64, kMaxClasses = 1024;
+
+// Row-class views of B in FP64, FP32 (d32, nullable) and pairs; inv: the inverted diagonal blocks or null.
+int build_class_views(fhg_ctx* ctx, const HostBsr& B, const double* inv, DevBsr<double>& d64, DevBsr<float>* d32,
+                      DevBsr<dfl>& d2)
+{
+    RowClasses C;
+    if (!row_classes(B, kMaxClasses, kClassRows, C)) return FHG_OK;
+    std::vector<double> dict;
+    class_dictionary(B, C, inv, dict);
+    unsigned short* cls = nullptr;
+    int* col = nullptr;
+    int rc;
+    if ((rc = upload(ctx, &cls, C.cls.data(), C.cls.size())) || (rc = upload(ctx, &col, C.col.data(), C.col.size())) ||
+        (rc = upload_classes(ctx, B, C, dict, cls, col, d64)) || (rc = upload_classes(ctx, B, C, dict, cls, col, d2)))
+        return rc;
+    return d32 ? upload_classes(ctx, B, C, dict, cls, col, *d32) : FHG_OK;
+}
+
 // Outer operator as an FP32 pair: hi = fl32(a), lo = fl32(a - hi), entry-major like upload_bsr.
 int upload_bsr_split(fhg_ctx* ctx, const HostBsr& B, DevBsr<float>& D, float** lo_out, const DevBsr<double>& share_index)
 {
@@ -573,14 +619,14 @@ template <> struct LevelVecs<double> {
     static double* x(Level& L) { return L.x; }
     static double* b(Level& L) { return L.b; }
     static double* r(Level& L) { return L.r; }
-    static const BsrView<double>& A(Level& L) { return L.A.v; }
+    static const BsrView<double>& A(Level& L) { return L.C64.vals ? L.C64.v : L.A.v; }
     static const BsrView<double>& P(Level& L) { return L.P.v; }
     static const BsrView<double>& R(Level& L) { return L.R.v; }
     static const BsrView<double>& Pcsr(Level& L) { return L.P.v; }
     static const BsrView<double>& Rcsr(Level& L) { return L.R.v; }
     static const double* dinv(Level& L) { return L.dinv; }
     static double* k(Level& L, int i) { return L.kv64[i]; }
-    static const BsrView<double>& gs(Level& L) { return L.A.v; }
+    static const BsrView<double>& gs(Level& L) { return L.C64.vals ? L.C64.v : L.A.v; }
     static const BsrView<double>& Acsr(Level& L) { return L.A.v; }
 };
 template <> struct LevelVecs<float> {
@@ -588,9 +634,10 @@ template <> struct LevelVecs<float> {
     static float* x(Level& L) { return L.x32; }
     static float* b(Level& L) { return L.b32; }
     static float* r(Level& L) { return L.r32; }
-    // products with A: the slot-major or the row-major padded view when setup built one
+    // products with A: the row-class, slot-major or row-major padded view when setup built one
     static const BsrView<float>& A(Level& L)
     {
+        if (L.C32.vals) return L.C32.v;
         if (L.prod_slot[kPrec] && L.A32s.vals) return L.A32s.v;
         return L.A32p.vals ? L.A32p.v : L.A32.v;
     }
@@ -602,9 +649,10 @@ template <> struct LevelVecs<float> {
     static const BsrView<float>& Rcsr(Level& L) { return L.R32.v; }
     static const float* dinv(Level& L) { return L.dinv32; }
     static float* k(Level& L, int i) { return L.kv32[i]; }
-    // GS sweeps: the slot-major or padded off-diagonal view when setup built one
+    // GS sweeps: the row-class, slot-major or padded off-diagonal view when setup built one
     static const BsrView<float>& gs(Level& L)
     {
+        if (L.C32.vals) return L.C32.v;
         if (L.gs_slot[kPrec] && L.G32s.vals) return L.G32s.v;
         return L.G32.vals ? L.G32.v : L.A32.v;
     }
@@ -618,6 +666,7 @@ template <> struct LevelVecs<dfl> {
     static dfl* r(Level& L) { return L.r2; }
     static const BsrView<dfl>& A(Level& L)
     {
+        if (L.C2.vals) return L.C2.v;
         if (L.prod_slot[kPrec] && L.A2s.vals) return L.A2s.v;
         return L.A2p.vals ? L.A2p.v : L.A2.v;
     }
@@ -629,6 +678,7 @@ template <> struct LevelVecs<dfl> {
     static dfl* k(Level& L, int i) { return L.kv2[i]; }
     static const BsrView<dfl>& gs(Level& L)
     {
+        if (L.C2.vals) return L.C2.v;
         if (L.gs_slot[kPrec] && L.G2s.vals) return L.G2s.v;
         return L.G2.vals ? L.G2.v : L.A2.v;
     }
@@ -1128,13 +1178,25 @@ void precondition(fhg_ctx* ctx, const double* r, double* z)
 
 double* part(fhg_ctx* ctx, int i) { return ctx->partials + (size_t)i * fhg::kReduceCtas; }
 
-// Ad = Â d in pair arithmetic with the partials of d.Ad and r.d: on the slot-major pair view when
-// setup built one and the autotuner kept it, else on the row-major split view.
+// The FP64 outer operator Â: its row-class view, else CSR with the tuned lanes.
+BsrView<double> outer_operator(const Level& L)
+{
+    if (L.Co64.vals) return L.Co64.v;
+    BsrView<double> Ah = L.ahat_is_a ? L.A.v : L.Ahat.v;
+    if (L.outer_lanes) Ah.lanes = L.outer_lanes;
+    return Ah;
+}
+
+// Ad = Â d in pair arithmetic with the partials of d.Ad and r.d: on the row-class view where Â's rows
+// repeat, on the slot-major pair view when setup built one and the autotuner kept it, else on the
+// row-major split view.
 void outer_product_df(fhg_ctx* ctx, const float* dh, const float* dl, const float* rh, const float* rl, float* Adh,
                       float* Adl, double* partials)
 {
     Level& L0 = ctx->levels[0];
-    if (L0.Ahat2s.vals && (L0.outer_slot || !L0.ahat_lo))
+    if (L0.Co2.vals)
+        fhg::launch_spmv_dots_df_slot(L0.Co2.v, dh, dl, rh, rl, Adh, Adl, partials, ctx->stream);
+    else if (L0.Ahat2s.vals && (L0.outer_slot || !L0.ahat_lo))
         fhg::launch_spmv_dots_df_slot(L0.Ahat2s.v, dh, dl, rh, rl, Adh, Adl, partials, ctx->stream);
     else
         fhg::launch_spmv_dots_df(L0.Ahat_hi.v, L0.ahat_lo, dh, dl, rh, rl, Adh, Adl, partials, ctx->stream);
@@ -1146,7 +1208,7 @@ bool outer_df(const fhg_ctx* ctx)
 {
     const int p = ctx->opts.vcycle_precision;
     return (p == FHG_PREC_FP32 || (p == FHG_PREC_DF && ctx->rhi)) && ctx->opts.krylov == FHG_KRYLOV_FCG &&
-           (ctx->levels[0].ahat_lo || ctx->levels[0].Ahat2s.vals) && ctx->rlo;
+           (ctx->levels[0].ahat_lo || ctx->levels[0].Ahat2s.vals || ctx->levels[0].Co2.vals) && ctx->rlo;
 }
 
 // High part of the outer residual pair: the FP32 V-cycle reads it as its right-hand side.
@@ -1219,11 +1281,7 @@ void fcg_iteration(fhg_ctx* ctx, int p)
         fhg::launch_dot(n, z, Adp, part(ctx, 0), s);
         fhg::launch_fcg_direction(n, z, dp, part(ctx, 0), ctx->scal + 1, z, s);
     }
-    {
-        BsrView<double> Ah = L0.ahat_is_a ? L0.A.v : L0.Ahat.v;
-        if (L0.outer_lanes) Ah.lanes = L0.outer_lanes;
-        fhg::launch_spmv_dots(Ah, z, ctx->kr, Ad, part(ctx, 1), s);
-    }
+    fhg::launch_spmv_dots(outer_operator(L0), z, ctx->kr, Ad, part(ctx, 1), s);
     // parts 1 = d.Ad, 2 = r.d
     fhg::launch_krylov_step(n, ctx->kx, ctx->kr, z, Ad, part(ctx, 2), part(ctx, 1), ctx->scal + 1, part(ctx, 3), s,
                             fp32 ? L0.b32 : nullptr);
@@ -1241,7 +1299,7 @@ void cg_iteration(fhg_ctx* ctx)
     double* d = ctx->kz[1];
     double* Ad = ctx->kAd[0];
     fhg::launch_cg_direction(n, z, ctx->scal + 4, d, s);
-    fhg::launch_spmv_dots(ctx->levels[0].A.v, d, ctx->kr, Ad, part(ctx, 1), s);
+    fhg::launch_spmv_dots(LevelVecs<double>::A(ctx->levels[0]), d, ctx->kr, Ad, part(ctx, 1), s);
     fhg::launch_cg_step(n, ctx->kx, ctx->kr, d, Ad, ctx->scal + 3, part(ctx, 1), part(ctx, 3), s);
     precondition(ctx, ctx->kr, z);
     fhg::launch_dot(n, ctx->kr, z, part(ctx, 0), s);
@@ -1349,12 +1407,12 @@ int time_candidate(fhg_ctx* ctx, F run, float* ms_out)
 // mesh size and degree, whatever their coefficients) share the best shape, so a process that sets up
 // many of them times each structure once.
 struct TuneKey {
-    int prec, bs, nb, ncol, gs_w, prod_w, p_nbr, r_nbr;
+    int prec, bs, nb, ncol, gs_w, prod_w, p_nbr, r_nbr, classes;
     long long nnzb, p_blocks;
     bool operator<(const TuneKey& o) const
     {
-        return std::tie(prec, bs, nb, ncol, gs_w, prod_w, p_nbr, r_nbr, nnzb, p_blocks) <
-               std::tie(o.prec, o.bs, o.nb, o.ncol, o.gs_w, o.prod_w, o.p_nbr, o.r_nbr, o.nnzb, o.p_blocks);
+        return std::tie(prec, bs, nb, ncol, gs_w, prod_w, p_nbr, r_nbr, classes, nnzb, p_blocks) <
+               std::tie(o.prec, o.bs, o.nb, o.ncol, o.gs_w, o.prod_w, o.p_nbr, o.r_nbr, o.classes, o.nnzb, o.p_blocks);
     }
 };
 struct TuneShapes {
@@ -1387,7 +1445,7 @@ int tune_level(fhg_ctx* ctx, int l)
     L.gs_slot[PR] = false;
     BsrView<T>& A = const_cast<BsrView<T>&>(V::A(L));
     TuneKey key{PR, L.bs, L.nb, L.ncolours, V::gs(L).ell, A.ell, coarsest ? 0 : V::Pcsr(L).nbr,
-                coarsest ? 0 : V::Rcsr(L).nbr, A.nnzb, coarsest ? 0 : V::Pcsr(L).nnzb};
+                coarsest ? 0 : V::Rcsr(L).nbr, A.cls ? 1 : 0, A.nnzb, coarsest ? 0 : V::Pcsr(L).nnzb};
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
@@ -1444,8 +1502,9 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
     const bool forced_prod_slot = L.prod_slot[V::kPrec];
     L.prod_slot[V::kPrec] = false;
     BsrView<T>& A = const_cast<BsrView<T>&>(V::A(L));
+    const bool classes = A.cls != nullptr;   // row-class views have no launch shape to choose
     float row_prod_ms = 0.f;
-    int rc = tune(ctx, bs, A.lanes, A.unroll, [&](int G, int U) {
+    int rc = classes ? FHG_OK : tune(ctx, bs, A.lanes, A.unroll, [&](int G, int U) {
         BsrView<T> v = A; v.lanes = G; v.unroll = U;
         fhg::launch_spmv<T>(v, fhg::kSpmvResidual, V::x(L), V::b(L), V::r(L), s);
     }, &row_prod_ms);
@@ -1473,14 +1532,16 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
         L.gs_slot[PR] = false;
         float row_ms = 0.f;
         if (V::gs(L).ell > 0) { g = V::gs(L).lanes; gu = 1; }
-        rc = tune(ctx, bs, g, gu, [&](int G, int U) {
+        rc = classes ? FHG_OK : tune(ctx, bs, g, gu, [&](int G, int U) {
             BsrView<T> v = V::gs(L); v.lanes = G; v.unroll = U;
             for (int c = 0; c < L.ncolours; c++)
                 fhg::launch_gs<T>(v, L.colour_start[c], L.colour_start[c + 1], V::dinv(L), L.nb, V::b(L), V::x(L), s);
         }, &row_ms);
         if (rc) return rc;
-        L.gs_lanes[PR] = g;
-        L.gs_unroll[PR] = gu;
+        if (!classes) {
+            L.gs_lanes[PR] = g;
+            L.gs_unroll[PR] = gu;
+        }
         L.gs_slot[PR] = forced_slot;
         if constexpr (!std::is_same<T, double>::value) {
             const BsrView<T>* slot = nullptr;
@@ -1571,6 +1632,11 @@ void reset_device_state(Level& L)
     L.A32p = DevBsr<float>();
     L.G32s = DevBsr<float>();
     L.A32s = DevBsr<float>();
+    L.C64 = DevBsr<double>();
+    L.Co64 = DevBsr<double>();
+    L.C32 = DevBsr<float>();
+    L.C2 = DevBsr<dfl>();
+    L.Co2 = DevBsr<dfl>();
     L.A2 = DevBsr<dfl>();
     L.P2 = DevBsr<dfl>();
     L.R2 = DevBsr<dfl>();
@@ -1717,7 +1783,7 @@ int run_solve(fhg_ctx* ctx, double* history, fhg_solve_info* info)
         if (learned_its > 0 && status == FHG_OK) status = check_learned_status(ctx);
         if (status != FHG_OK) break;
         // The FP64 true residual ||b - A x|| / ||b|| judges the solve (A the full level-0 operator).
-        fhg::launch_spmv<double>(L0.A.v, fhg::kSpmvResidual, ctx->kx, ctx->kb, ctx->kt, s);
+        fhg::launch_spmv<double>(LevelVecs<double>::A(L0), fhg::kSpmvResidual, ctx->kx, ctx->kb, ctx->kt, s);
         fhg::launch_dot(n, ctx->kt, ctx->kt, part(ctx, 0), s);
         fhg::launch_sqrt_sum(part(ctx, 0), ctx->scal + 5, s);
         double h[6];
@@ -2047,25 +2113,6 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
         if ((rc = upload_bsr<double>(ctx, Ap, L.A, nullptr))) return rc;
         if (fp32 && (rc = upload_bsr<float>(ctx, Ap, L.A32, &L.A))) return rc;
         if (pair && (rc = upload_bsr<dfl>(ctx, Ap, L.A2, &L.A))) return rc;
-        // slot-major views (GS sweeps and products): when forced, or for the autotuner to compare
-        const bool want_slot = o.colouring && (o.gs_layout == FHG_GS_SLOT || (o.gs_layout == FHG_GS_AUTO && o.autotune));
-        if (fp32 && l < nlevels - 1) {
-            if (o.colouring && (rc = upload_padded(ctx, Ap, L.G32, true, 8))) return rc;
-            if ((rc = upload_padded(ctx, Ap, L.A32p, false, 8))) return rc;
-            if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G32s))) return rc;
-            if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A32s))) return rc;
-            L.gs_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.G32s.vals;
-            L.prod_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.A32s.vals;
-        }
-        if (pair && l < nlevels - 1) {
-            if (o.colouring && (rc = upload_padded(ctx, Ap, L.G2, true, 8))) return rc;
-            if ((rc = upload_padded(ctx, Ap, L.A2p, false, 8))) return rc;
-            if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G2s))) return rc;
-            if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A2s))) return rc;
-            L.gs_slot[FHG_PREC_DF] = o.gs_layout == FHG_GS_SLOT && L.G2s.vals;
-            L.prod_slot[FHG_PREC_DF] = o.gs_layout == FHG_GS_SLOT && L.A2s.vals;
-        }
-        if ((rc = upload(ctx, &L.perm_d, L.perm.data(), L.perm.size()))) return rc;
         if (l < nlevels - 1) {
             // Pre-inverted diagonal blocks (FP64, rounded for the FP32 copy).
             const int bs = L.bs;
@@ -2091,6 +2138,36 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                 for (size_t q = 0; q < soa.size(); q++) s2[q] = dfl(soa[q]);
                 if ((rc = upload(ctx, &L.dinv2, s2.data(), s2.size()))) return rc;
             }
+            // Where rows repeat, the row-class views serve the sweeps and the products in every precision
+            // (a forced layout keeps the stored-block views).
+            if (o.colouring && o.gs_layout == FHG_GS_AUTO &&
+                (rc = build_class_views(ctx, Ap, inv.data(), L.C64, &L.C32, L.C2)))
+                return rc;
+        }
+        // The row- and slot-major views of stored blocks: not beside class views, but for the padded rows of
+        // levels >= 1, which the one-launch coarse sub-cycle reads.
+        const bool classes = L.C64.vals != nullptr;
+        const bool padded = !classes || (l > 0 && o.fused_coarse);
+        // slot-major views (GS sweeps and products): when forced, or for the autotuner to compare
+        const bool want_slot = o.colouring && !classes && (o.gs_layout == FHG_GS_SLOT || (o.gs_layout == FHG_GS_AUTO && o.autotune));
+        if (fp32 && l < nlevels - 1) {
+            if (o.colouring && padded && (rc = upload_padded(ctx, Ap, L.G32, true, 8))) return rc;
+            if (padded && (rc = upload_padded(ctx, Ap, L.A32p, false, 8))) return rc;
+            if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G32s))) return rc;
+            if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A32s))) return rc;
+            L.gs_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.G32s.vals;
+            L.prod_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.A32s.vals;
+        }
+        if (pair && l < nlevels - 1) {
+            if (o.colouring && padded && (rc = upload_padded(ctx, Ap, L.G2, true, 8))) return rc;
+            if (padded && (rc = upload_padded(ctx, Ap, L.A2p, false, 8))) return rc;
+            if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G2s))) return rc;
+            if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A2s))) return rc;
+            L.gs_slot[FHG_PREC_DF] = o.gs_layout == FHG_GS_SLOT && L.G2s.vals;
+            L.prod_slot[FHG_PREC_DF] = o.gs_layout == FHG_GS_SLOT && L.A2s.vals;
+        }
+        if ((rc = upload(ctx, &L.perm_d, L.perm.data(), L.perm.size()))) return rc;
+        if (l < nlevels - 1) {
             if (L.inject) {
                 // The natural injection: block row i of this level is block row map[i] of the next.
                 std::vector<int> map(L.nb);
@@ -2100,7 +2177,7 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
             } else {
                 // Transfers: P' = Pi_l P Pi_{l+1}^T, R' = P'^T.
                 HostBsr Pb, Pp, Rp;
-                csr_to_bsr(L.P_in, bs, Pb);
+                csr_to_bsr(L.P_in, L.bs, Pb);
                 permute_bsr(Pb, L.perm, iperm[l + 1], Pp);
                 Pb = HostBsr();
                 transpose_bsr(Pp, Rp);
@@ -2149,9 +2226,13 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                 HostBsr Sb, Sp;
                 csr_to_bsr(S, L.bs, Sb);
                 permute_bsr(Sb, L.perm, iperm[0], Sp);
-                if ((rc = upload_bsr<double>(ctx, Sp, L.Ahat, nullptr))) return rc;
-                if (split && (rc = upload_bsr_split(ctx, Sp, L.Ahat_hi, &L.ahat_lo, L.Ahat))) return rc;
-                if (split && (rc = upload_slot_major_all(ctx, Sp, L.Ahat2s))) return rc;
+                if (L.C64.vals && (rc = build_class_views(ctx, Sp, nullptr, L.Co64, nullptr, L.Co2))) return rc;
+                if (!L.Co64.vals && (rc = upload_bsr<double>(ctx, Sp, L.Ahat, nullptr))) return rc;
+                if (split && !L.Co64.vals && (rc = upload_bsr_split(ctx, Sp, L.Ahat_hi, &L.ahat_lo, L.Ahat))) return rc;
+                if (split && !L.Co64.vals && (rc = upload_slot_major_all(ctx, Sp, L.Ahat2s))) return rc;
+            } else if (L.C64.vals) {   // Â = A: its views
+                L.Co64 = L.C64;
+                L.Co2 = L.C2;
             } else if (split) {
                 if ((rc = upload_bsr_split(ctx, Ap, L.Ahat_hi, &L.ahat_lo, L.A))) return rc;
                 if ((rc = upload_slot_major_all(ctx, Ap, L.Ahat2s))) return rc;
@@ -2227,8 +2308,8 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
         // the outer operator's choices, kept per structure like the levels' shapes
         const std::vector<long long> okey = {L0.bs, L0.nb, (long long)Ah.nnzb, L0.ahat_is_a ? 1 : 0,
                                              L0.ahat_lo ? 1 : 0, L0.Ahat2s.vals ? 1 : 0, o.gs_layout};
-        bool cached = false;
-        if (o.gs_layout == FHG_GS_AUTO) {
+        bool cached = L0.Co64.vals != nullptr;   // a row-class view has no launch shape
+        if (!cached && o.gs_layout == FHG_GS_AUTO) {
             std::lock_guard<std::mutex> lock(g_tune_mutex);
             auto it = g_outer_cache.find(okey);
             if (it != g_outer_cache.end()) {
@@ -2375,9 +2456,7 @@ static int apply_device(fhg_ctx* ctx, int level, int op, double* in, double* aux
     cudaStream_t s = ctx->stream;
     if (op == FHG_OP_SYM_SPMV) {
         if (level != 0) return fail(ctx, FHG_ERR_INVALID_ARG, "symmetric operator exists on level 0 only");
-        BsrView<double> Ah = L.ahat_is_a ? L.A.v : L.Ahat.v;
-        if (L.outer_lanes) Ah.lanes = L.outer_lanes;
-        fhg::launch_spmv_dots(Ah, in, in, out, part(ctx, 4), s);
+        fhg::launch_spmv_dots(outer_operator(L), in, in, out, part(ctx, 4), s);
         return FHG_OK;
     }
     if (op == FHG_OP_VCYCLE) {
@@ -2527,7 +2606,7 @@ int fhg_time_op(fhg_ctx* ctx, int level, int op, int precision, int warmup, int 
         // FP32 or DF: the outer operator in double-FP32 arithmetic (the one product both use)
         const bool split = op == FHG_OP_SYM_SPMV && (precision == FHG_PREC_FP32 || precision == FHG_PREC_DF);
         if (precision != FHG_PREC_FP64 && !split) return fail(ctx, FHG_ERR_INVALID_ARG, "op %d is timed in FP64 only", op);
-        if (split && ((!L0.ahat_lo && !L0.Ahat2s.vals) || !ctx->rlo))
+        if (split && ((!L0.ahat_lo && !L0.Ahat2s.vals && !L0.Co2.vals) || !ctx->rlo))
             return fail(ctx, FHG_ERR_NOT_READY, "the double-FP32 outer operator was not built at setup");
         const size_t n0 = L0.n;
         double* t = nullptr;
@@ -3088,7 +3167,7 @@ void device_true_residual(fhg_ctx* ctx, int replace)
     const long long n = L0.n;
     cudaStream_t s = ctx->stream;
     const double tol = ctx->opts.tolerance;
-    fhg::launch_spmv<double>(L0.A.v, fhg::kSpmvResidual, ctx->kx, ctx->kb, ctx->kt, s);
+    fhg::launch_spmv<double>(LevelVecs<double>::A(L0), fhg::kSpmvResidual, ctx->kx, ctx->kb, ctx->kt, s);
     fhg::launch_dot(n, ctx->kt, ctx->kt, part(ctx, 0), s);
     fhg::launch_check_fp64(part(ctx, 0), ctx->scal, tol, ctx->loop_state, s);
     fhg::launch_residual_comp(L0.A.v, ctx->kx, ctx->kb, ctx->kt, part(ctx, 1), s, ctx->loop_state + fhg::kLoopNeedComp);

@@ -594,6 +594,134 @@ __global__ void __launch_bounds__(kThreads, 2) k_bsr_residual_dinv_slot(int nbr,
     }
 }
 
+// ---------------------------------------------------------------------------
+// Row-class views. On a mesh of translated elements a block row is one of a few dozen (classes: see
+// row_classes in fhg_host.h), so the values stay in L1 and only the class (2 bytes), the off-diagonal
+// columns and the vectors are streamed: 62 bytes a row for an FP32 sweep with 3 x 3 blocks where the stored
+// blocks take 312. One thread per block row; the column indices and then every neighbour's x entries are
+// loaded before the sums, with registers for that (kClsBlocks CTAs of 128 threads per SM: at the compiler's
+// own choice of 32 registers the x loads follow one another, and a launch too small to hide them
+// takes twice as long). The sums run over the off-diagonal blocks in column order. What bounds a sweep now
+// is the L1's rate of gathered lines (a warp's x loads of one slot touch 7 lines) and L2; FP64 stays bound
+// by its pipe. 64^3, k = 1 (3.1 M rows, 77 classes), one sweep of stored blocks against classes:
+// FP32 188 -> 86 us, pairs 331 -> 149 us, FP64 402 -> 370 us (836 us with the row-major kernel's lanes).
+constexpr int kClsThreads = 128;
+
+// CTAs per SM of a class kernel: 64, 80 or 128 registers, what W x BS gathered values in flight and
+// 2 BS sums take without spills.
+template <class T, int BS, int W>
+constexpr int kClsBlocks = BS <= 3 ? 8 : sizeof(T) == 4 ? 6 : 4;
+
+// The x entries of a row's off-diagonal slots; zeros for an empty slot (the row's own column) and, in a
+// zero-start sweep, for a column outside [col_lo, col_hi).
+template <class T, int BS, int W, bool ZERO>
+__device__ __forceinline__ void gather_slots(const int (&col)[W], int row, int col_lo, int col_hi, const T* x, T (&xv)[W][BS])
+{
+#pragma unroll
+    for (int s = 0; s < W; s++) {
+        const int j = col[s];
+        const bool use = j != row && (!ZERO || (j >= col_lo && j < col_hi));
+#pragma unroll
+        for (int c = 0; c < BS; c++) xv[s][c] = use ? x[(long long)j * BS + c] : T(0);
+    }
+}
+
+// acc += sum over the off-diagonal slots of dict x (dict: the row's class).
+template <class T, int BS, int W>
+__device__ __forceinline__ void class_row(const T* __restrict__ dict, int ld, const T (&xv)[W][BS], T (&acc)[BS])
+{
+#pragma unroll
+    for (int s = 0; s < W; s++)
+#pragma unroll
+        for (int r = 0; r < BS; r++)
+#pragma unroll
+            for (int c = 0; c < BS; c++) acc[r] = fma(dict[((s * BS + r) * BS + c) * ld], xv[s][c], acc[r]);
+}
+
+// v = M w, M the bs x bs block `slot` of the row's class.
+template <class T, int BS>
+__device__ __forceinline__ void class_block(const T* __restrict__ dict, int ld, int slot, const T (&w)[BS], T (&v)[BS])
+{
+#pragma unroll
+    for (int r = 0; r < BS; r++)
+#pragma unroll
+        for (int c = 0; c < BS; c++) v[r] = fma(dict[((slot * BS + r) * BS + c) * ld], w[c], v[r]);
+}
+
+// One colour of block GS / SOR (the column rules of k_bsr_gs).
+template <class T, int BS, int W, bool ZERO>
+__global__ void __launch_bounds__(kClsThreads, kClsBlocks<T, BS, W>)
+    k_bsr_gs_cls(int row0, int row1, int nbr, const unsigned short* __restrict__ cls, const int* __restrict__ colidx,
+                 const T* __restrict__ dict, int ld, const T* __restrict__ b, T* x, int col_lo, int col_hi, T omega)
+{
+    const int row = row0 + (int)(blockIdx.x * kClsThreads + threadIdx.x);
+    const bool in = row < row1;
+    int col[W];   // the classes and columns never change after setup: read ahead of the wait
+    const T* d = dict + (in ? cls[row] : 0);
+#pragma unroll
+    for (int s = 0; s < W; s++) col[s] = in ? colidx[(long long)s * nbr + row] : row;
+    pdl_wait();
+    if (!in) return;
+    T xv[W][BS], t[BS], acc[BS], v[BS];
+    gather_slots<T, BS, W, ZERO>(col, row, col_lo, col_hi, x, xv);
+#pragma unroll
+    for (int c = 0; c < BS; c++) {
+        t[c] = b[(long long)row * BS + c];
+        acc[c] = T(0);
+        v[c] = T(0);
+    }
+    class_row<T, BS, W>(d, ld, xv, acc);
+#pragma unroll
+    for (int c = 0; c < BS; c++) t[c] = t[c] - acc[c];
+    class_block<T, BS>(d, ld, W, t, v);
+#pragma unroll
+    for (int r = 0; r < BS; r++) {
+        const long long i = (long long)row * BS + r;
+        if (omega != T(1)) v[r] = fma(omega, v[r], (T(1) - omega) * x[i]);   // block SOR
+        x[i] = fin(v[r]);
+    }
+}
+
+// y = A x | y = aux - A x; with DINV y = D^-1 (aux - A x) (the learned step's input).
+template <class T, int BS, int W, int MODE, bool DINV>
+__global__ void __launch_bounds__(kClsThreads, kClsBlocks<T, BS, W>)
+    k_bsr_spmv_cls(int nbr, const unsigned short* __restrict__ cls, const int* __restrict__ colidx,
+                   const T* __restrict__ dict, int ld, const T* __restrict__ x, const T* aux, T* y)
+{
+    const int row = (int)(blockIdx.x * kClsThreads + threadIdx.x);
+    const bool in = row < nbr;
+    int col[W];
+    const T* d = dict + (in ? cls[row] : 0);
+#pragma unroll
+    for (int s = 0; s < W; s++) col[s] = in ? colidx[(long long)s * nbr + row] : row;
+    pdl_wait();
+    if (!in) return;
+    T xv[W][BS], xd[BS], acc[BS], av[BS];
+    gather_slots<T, BS, W, false>(col, row, 0, 0, x, xv);
+#pragma unroll
+    for (int c = 0; c < BS; c++) {
+        xd[c] = x[(long long)row * BS + c];
+        av[c] = MODE == kSpmvAssign ? T(0) : aux[(long long)row * BS + c];
+        acc[c] = T(0);
+    }
+    class_row<T, BS, W>(d, ld, xv, acc);
+    class_block<T, BS>(d, ld, W + 1, xd, acc);
+    if (DINV) {
+        T v[BS];
+#pragma unroll
+        for (int c = 0; c < BS; c++) {
+            av[c] = av[c] - acc[c];
+            v[c] = T(0);
+        }
+        class_block<T, BS>(d, ld, W, av, v);
+#pragma unroll
+        for (int r = 0; r < BS; r++) y[(long long)row * BS + r] = fin(v[r]);
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < BS; r++) y[(long long)row * BS + r] = MODE == kSpmvAssign ? fin(acc[r]) : av[r] - acc[r];
+}
+
 // Block Jacobi: xnew_i = D_i^{-1} (omega b_i + (1-omega) D_i xold_i - omega sum_{j!=i} A_ij xold_j)
 template <class T, int BS, int G>
 __global__ void __launch_bounds__(kThreads) k_bsr_jacobi(int nbr, const int* __restrict__ rowptr,
@@ -840,10 +968,37 @@ void spmv_slot_w(const BsrView<T>& A, unsigned grid, int mode, const T* x, const
     }
 }
 
+// Row-class views: dispatch on the block size and the slot count (setup builds 4 and 6).
+#define FHG_DISPATCH_CLS(BSV, WV, ...)                                     \
+    switch (BSV * 10 + WV) {                                               \
+    case 24: { constexpr int BS = 2, W = 4; __VA_ARGS__; } break;          \
+    case 26: { constexpr int BS = 2, W = 6; __VA_ARGS__; } break;          \
+    case 34: { constexpr int BS = 3, W = 4; __VA_ARGS__; } break;          \
+    case 36: { constexpr int BS = 3, W = 6; __VA_ARGS__; } break;          \
+    case 44: { constexpr int BS = 4, W = 4; __VA_ARGS__; } break;          \
+    case 46: { constexpr int BS = 4, W = 6; __VA_ARGS__; } break;          \
+    case 64: { constexpr int BS = 6, W = 4; __VA_ARGS__; } break;          \
+    case 66: { constexpr int BS = 6, W = 6; __VA_ARGS__; } break;          \
+    default: break;                                                        \
+    }
+
 template <class T>
 void launch_spmv(const BsrView<T>& A, int mode, const T* x, const T* aux, T* y, cudaStream_t s)
 {
     if (A.nbr == 0) return;
+    if (A.cls) {   // operators only (assign, residual)
+        const unsigned grid = grid_for(A.nbr, kClsThreads);
+        FHG_DISPATCH_CLS(A.bs, A.ell, {
+            if (mode == kSpmvAssign)
+                pdl_launch(k_bsr_spmv_cls<T, BS, W, kSpmvAssign, false>, grid, kClsThreads, 0, s, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, x, aux, y);
+            else
+                pdl_launch(k_bsr_spmv_cls<T, BS, W, kSpmvResidual, false>, grid, kClsThreads, 0, s, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, x, aux, y);
+        });
+        g_kernel_launches++;
+        return;
+    }
     if (A.jds_perm) {
         // jagged views exist only for the transfers (assign, add-to) with at most kMaxJdsSlots blocks
         // a row (setup builds no other); they have no row pointers to fall back on
@@ -936,6 +1091,19 @@ void launch_gs(const BsrView<T>& A, int row0, int row1, const T* dinv, long long
                int col_lo, int col_hi, T omega)
 {
     if (row1 <= row0) return;
+    if (A.cls) {
+        const unsigned grid = grid_for((long long)(row1 - row0), kClsThreads);
+        FHG_DISPATCH_CLS(A.bs, A.ell, {
+            if (col_lo > 0 || col_hi < 0x7fffffff)
+                pdl_launch(k_bsr_gs_cls<T, BS, W, true>, grid, kClsThreads, 0, s, row0, row1, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, b, x, col_lo, col_hi, omega);
+            else
+                pdl_launch(k_bsr_gs_cls<T, BS, W, false>, grid, kClsThreads, 0, s, row0, row1, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, b, x, col_lo, col_hi, omega);
+        });
+        g_kernel_launches++;
+        return;
+    }
     if constexpr (!std::is_same<T, double>::value) {
         if (A.slot_major) {   // FP32 and pair views (setup builds no FP64 slot-major view)
             launch_gs_slot<T>(A, row0, row1, dinv, dld, b, x, s, col_lo, col_hi, omega);

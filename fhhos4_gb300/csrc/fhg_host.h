@@ -8,7 +8,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <system_error>
 #include <thread>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -379,6 +381,132 @@ inline bool invert_block(const double* a_in, int n, double* inv)
     for (int k = 0; k < n; k++)
         for (int j = 0; j < n; j++) inv[colperm[k] * n + j] = b[k * n + j];
     return true;
+}
+
+// Rows of a block operator that hold the same values: on the meshes whose elements are translations of
+// a few (n^3 cubes cut alike, with a coefficient that is constant on patches) every row of the face
+// system is one of a few dozen to a few hundred, whatever n. A class is a row's blocks, bit for bit: the
+// off-diagonal ones in column order, then the diagonal one.
+struct RowClasses {
+    int W = 0;                          // off-diagonal slots of every row (4 or 6)
+    int ncls = 0;
+    std::vector<unsigned short> cls;    // class of each row, numbered by first appearance
+    std::vector<int> col;               // off-diagonal columns, slot s of row i at s * nbr + i; empty: i
+    std::vector<int> rep;               // the first row of each class
+};
+
+// Run f(lo, hi) over [0, n) on the host's threads.
+template <class F>
+void parallel_rows(int n, F f)
+{
+    const int nt = (int)std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
+    const int chunk = std::max(4096, (n + nt - 1) / nt);
+    std::vector<std::thread> th;
+    for (int lo = chunk; lo < n; lo += chunk) {
+        const int hi = std::min(n, lo + chunk);
+        try {
+            th.emplace_back(f, lo, hi);
+        } catch (const std::system_error&) {   // no thread to be had
+            f(lo, hi);
+        }
+    }
+    f(0, std::min(n, chunk));
+    for (auto& t : th) t.join();
+}
+
+// The classes of B's rows, when there are few: at most max_classes, at least min_rows rows to a class on
+// average, at most 6 off-diagonal blocks a row, and a diagonal block in every row. False otherwise.
+inline bool row_classes(const HostBsr& B, int max_classes, int min_rows, RowClasses& C)
+{
+    const int n = B.nbr;
+    const size_t bb = (size_t)B.bs * B.bs;
+    const int limit = std::min(max_classes, n / min_rows);
+    if (limit < 1) return false;
+    std::vector<unsigned long long> hash(n);
+    std::vector<unsigned char> width(n);
+    parallel_rows(n, [&](int lo, int hi) {
+        for (int i = lo; i < hi; i++) {
+            int w = 0, diag = 0;
+            unsigned long long h = 0x9E3779B97F4A7C15ull, hd = 0;
+            for (int p = B.rowptr[i]; p < B.rowptr[i + 1]; p++) {
+                unsigned long long g = 0x2545F4914F6CDD1Dull;
+                for (size_t e = 0; e < bb; e++) {
+                    unsigned long long u;
+                    std::memcpy(&u, &B.vals[p * bb + e], 8);
+                    g = (g ^ u) * 0xBF58476D1CE4E5B9ull;
+                    g ^= g >> 29;
+                }
+                if (B.colidx[p] == i) { hd = g; diag++; continue; }
+                h = (h ^ g) * 0x94D049BB133111EBull;
+                h ^= h >> 31;
+                w = std::min(w + 1, 255);
+            }
+            width[i] = (unsigned char)(diag == 1 ? w : 255);
+            hash[i] = (h ^ hd) * 0x9E3779B97F4A7C15ull + (unsigned long long)w;
+        }
+    });
+    int W = 0;
+    for (int i = 0; i < n; i++) W = std::max(W, (int)width[i]);
+    if (W > 6) return false;
+    C.W = W <= 4 ? 4 : 6;
+    C.rep.clear();
+    C.cls.assign(n, 0);
+    std::unordered_map<unsigned long long, int> ids;
+    for (int i = 0; i < n; i++) {
+        const auto it = ids.find(hash[i]);
+        if (it != ids.end()) { C.cls[i] = (unsigned short)it->second; continue; }
+        if ((int)C.rep.size() == limit) return false;
+        ids[hash[i]] = (int)C.rep.size();
+        C.cls[i] = (unsigned short)C.rep.size();
+        C.rep.push_back(i);
+    }
+    C.ncls = (int)C.rep.size();
+    C.col.assign((size_t)C.W * n, 0);
+    std::vector<unsigned char> same(n, 1);   // every row against its class's first (hashes can collide)
+    parallel_rows(n, [&](int lo, int hi) {
+        for (int i = lo; i < hi; i++) {
+            const int r = C.rep[C.cls[i]];
+            int k = 0, q = B.rowptr[r];
+            const int q1 = B.rowptr[r + 1];
+            int pd = -1, qd = -1;
+            bool eq = width[i] == width[r];
+            for (int p = B.rowptr[i]; p < B.rowptr[i + 1]; p++) {
+                if (B.colidx[p] == i) { pd = p; continue; }
+                while (q < q1 && B.colidx[q] == r) qd = q++;
+                eq = eq && q < q1 && std::memcmp(&B.vals[p * bb], &B.vals[q * bb], bb * sizeof(double)) == 0;
+                q++;
+                C.col[(size_t)k++ * n + i] = B.colidx[p];
+            }
+            for (; k < C.W; k++) C.col[(size_t)k * n + i] = i;
+            if (qd < 0)
+                for (int p = B.rowptr[r]; p < q1; p++)
+                    if (B.colidx[p] == r) qd = p;
+            same[i] = eq && pd >= 0 && qd >= 0 &&
+                      std::memcmp(&B.vals[pd * bb], &B.vals[qd * bb], bb * sizeof(double)) == 0;
+        }
+    });
+    for (int i = 0; i < n; i++)
+        if (!same[i]) return false;
+    return true;
+}
+
+// The dictionary of the classes, entry by entry (entry e of class c at e * ncls + c): the W off-diagonal
+// blocks (zero where a row has fewer), D^-1 of the diagonal block (inv: nbr x bs^2, null: zeros), and
+// the diagonal block.
+inline void class_dictionary(const HostBsr& B, const RowClasses& C, const double* inv, std::vector<double>& dict)
+{
+    const size_t bb = (size_t)B.bs * B.bs, n = C.ncls;
+    dict.assign((C.W + 2) * bb * n, 0.0);
+    for (size_t c = 0; c < n; c++) {
+        const int r = C.rep[c];
+        size_t k = 0;
+        for (int p = B.rowptr[r]; p < B.rowptr[r + 1]; p++) {
+            const size_t slot = B.colidx[p] == r ? C.W + 1 : k++;
+            for (size_t e = 0; e < bb; e++) dict[(slot * bb + e) * n + c] = B.vals[p * bb + e];
+        }
+        if (inv)
+            for (size_t e = 0; e < bb; e++) dict[(C.W * bb + e) * n + c] = inv[r * bb + e];
+    }
 }
 
 // Dense Cholesky A = L L^T in place (lower), then A^{-1} = L^{-T} L^{-1}; multithreaded over columns.

@@ -38,6 +38,12 @@ struct BsrView {
     const int* jds_perm = nullptr;
     const int* jds_start = nullptr;
     int jds_slots = 0;
+    // Row-class view (operators whose rows repeat): cls[i] is the class of row i, vals the dictionary of
+    // the classes, entry e of class c at e * ld + c: the ell off-diagonal blocks in column order, D^-1, the
+    // diagonal block; the off-diagonal columns of row i at s * nbr + i (the row itself in an empty slot);
+    // rowptr unused (accepted by launch_spmv but for add-to, launch_gs, launch_residual_dinv and the outer
+    // products).
+    const unsigned short* cls = nullptr;
 };
 
 // Fixed number of CTAs of the reduction kernels: the partial-sum arrays they write
@@ -95,7 +101,7 @@ void launch_fcg_direction_mixed(long long n, const float* z, const double* dp, c
 void launch_spmv_dots_df(const BsrView<float>& Ahi, const float* vlo, const float* dhi, const float* dlo,
                          const float* rhi, const float* rlo, float* Adhi, float* Adlo, double* partials,
                          cudaStream_t s);
-// The same on the slot-major pair view of Â (ell = 5..8 slots; bs 2, 3, 4, 6).
+// The same on the slot-major pair view of Â (ell = 5..8 slots; bs 2, 3, 4, 6) or on its row-class view.
 void launch_spmv_dots_df_slot(const BsrView<dfl>& A, const float* dhi, const float* dlo, const float* rhi,
                               const float* rlo, float* Adhi, float* Adlo, double* partials, cudaStream_t s);
 // partials of z.Adp (z FP32, or z2 non-null: the pair V-cycle's output as interleaved pairs).

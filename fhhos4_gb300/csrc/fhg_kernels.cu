@@ -243,6 +243,107 @@ __global__ void __launch_bounds__(kReduceThreads, 2) k_bsr_spmv_dots_df_slot(int
     }
 }
 
+// The outer products on the row-class view of Â (fhg_bsr_kernels.cuh): one thread per block row over the
+// fixed grid, the values from the class dictionary. In pairs the 64^3, k = 1 product is bound by its FP32
+// pair arithmetic (13 instructions a term) instead of the 1.6 GB of stored pairs.
+template <int BS, int W>
+__global__ void __launch_bounds__(kReduceThreads, BS <= 3 ? 4 : 2) k_bsr_spmv_dots_df_cls(int nbr, const unsigned short* __restrict__ cls,
+                                                                         const int* __restrict__ colidx,
+                                                                         const dfl* __restrict__ dict, int ld,
+                                                                         const float* __restrict__ dhi,
+                                                                         const float* __restrict__ dlo,
+                                                                         const float* __restrict__ rhi,
+                                                                         const float* __restrict__ rlo,
+                                                                         float* __restrict__ Adhi,
+                                                                         float* __restrict__ Adlo,
+                                                                         double* __restrict__ partials)
+{
+    pdl_wait();
+    __shared__ double sh_red[33];
+    float dad_h = 0.f, dad_l = 0.f, rd_h = 0.f, rd_l = 0.f;
+    for (long long row = (long long)blockIdx.x * kReduceThreads + threadIdx.x; row < nbr; row += kRedStride) {
+        const dfl* t = dict + cls[row];
+        int col[W];
+#pragma unroll
+        for (int s = 0; s < W; s++) col[s] = colidx[(long long)s * nbr + row];
+        dfl xv[W][BS], xd[BS], acc[BS];
+#pragma unroll
+        for (int s = 0; s < W; s++)
+#pragma unroll
+            for (int c = 0; c < BS; c++) {
+                const long long j = (long long)col[s] * BS + c;
+                xv[s][c] = col[s] != (int)row ? dfl(dhi[j], dlo[j]) : dfl(0.f, 0.f);
+            }
+#pragma unroll
+        for (int c = 0; c < BS; c++) {
+            xd[c] = dfl(dhi[row * BS + c], dlo[row * BS + c]);
+            acc[c] = dfl(0.f, 0.f);
+        }
+        class_row<dfl, BS, W>(t, ld, xv, acc);
+        class_block<dfl, BS>(t, ld, W + 1, xd, acc);
+#pragma unroll
+        for (int r = 0; r < BS; r++) {
+            const long long i = row * BS + r;
+            const dfl a = fin(acc[r]);
+            float ph, pl;
+            Adhi[i] = a.h;
+            Adlo[i] = a.l;
+            df_mul(xd[r].h, xd[r].l, a.h, a.l, ph, pl);
+            df_add(dad_h, dad_l, ph, pl);
+            df_mul(rhi[i], rlo[i], xd[r].h, xd[r].l, ph, pl);
+            df_add(rd_h, rd_l, ph, pl);
+        }
+    }
+    const double s1 = block_sum((double)dad_h + (double)dad_l, sh_red);
+    const double s2 = block_sum((double)rd_h + (double)rd_l, sh_red);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = s1;
+        partials[kReduceCtas + blockIdx.x] = s2;
+    }
+}
+
+template <int BS, int W>
+__global__ void __launch_bounds__(kReduceThreads, BS <= 3 ? 4 : 2) k_bsr_spmv_dots_cls(int nbr, const unsigned short* __restrict__ cls,
+                                                                      const int* __restrict__ colidx,
+                                                                      const double* __restrict__ dict, int ld,
+                                                                      const double* __restrict__ d,
+                                                                      const double* __restrict__ rvec,
+                                                                      double* __restrict__ Ad,
+                                                                      double* __restrict__ partials)
+{
+    pdl_wait();
+    __shared__ double sh[33];
+    double dad = 0.0, rd = 0.0;
+    for (long long row = (long long)blockIdx.x * kReduceThreads + threadIdx.x; row < nbr; row += kRedStride) {
+        const double* t = dict + cls[row];
+        int col[W];
+#pragma unroll
+        for (int s = 0; s < W; s++) col[s] = colidx[(long long)s * nbr + row];
+        double xv[W][BS], xd[BS], acc[BS];
+        gather_slots<double, BS, W, false>(col, (int)row, 0, 0, d, xv);
+#pragma unroll
+        for (int c = 0; c < BS; c++) {
+            xd[c] = d[row * BS + c];
+            acc[c] = 0.0;
+        }
+        class_row<double, BS, W>(t, ld, xv, acc);
+        class_block<double, BS>(t, ld, W + 1, xd, acc);
+#pragma unroll
+        for (int r = 0; r < BS; r++) {
+            const long long i = row * BS + r;
+            Ad[i] = acc[r];
+            dad = fma(xd[r], acc[r], dad);
+            rd = fma(rvec[i], xd[r], rd);
+        }
+    }
+    const double s1 = block_sum(dad, sh);
+    const double s2 = block_sum(rd, sh);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = s1;
+        partials[kReduceCtas + blockIdx.x] = s2;
+    }
+}
+
 // r = b - A x with compensated summation (Ogita, Rump and Oishi 2005, "Accurate sum and dot
 // product", Dot2): every product split exactly by an FMA (TwoProduct), the running sum kept exact by
 // TwoSum, the rounding errors summed apart and added once, so r_i carries an error of about one unit
@@ -617,6 +718,15 @@ void launch_residual_dinv(const BsrView<float>& A, const float* dinv, long long 
                           float* w, cudaStream_t s)
 {
     if (A.nbr == 0) return;
+    if (A.cls) {
+        const unsigned grid = grid_for(A.nbr, kClsThreads);
+        FHG_DISPATCH_CLS(A.bs, A.ell, {
+            pdl_launch(k_bsr_spmv_cls<float, BS, W, kSpmvResidual, true>, grid, kClsThreads, 0, s, A.nbr, A.cls, A.colidx,
+                       A.vals, (int)A.ld, x, b, w);
+        });
+        g_kernel_launches++;
+        return;
+    }
     if (A.slot_major) {   // block sizes of the learned step (2..4)
         if (A.bs == 2) residual_dinv_slot<2>(A, dinv, dld, x, b, w, s);
         else if (A.bs == 3) residual_dinv_slot<3>(A, dinv, dld, x, b, w, s);
@@ -634,6 +744,14 @@ void launch_residual_dinv(const BsrView<float>& A, const float* dinv, long long 
 void launch_spmv_dots(const BsrView<double>& A, const double* d, const double* r, double* Ad, double* partials,
                       cudaStream_t s)
 {
+    if (A.cls) {
+        FHG_DISPATCH_CLS(A.bs, A.ell, {
+            pdl_launch(k_bsr_spmv_dots_cls<BS, W>, kReduceCtas, kReduceThreads, 0, s, A.nbr, A.cls, A.colidx, A.vals,
+                       (int)A.ld, d, r, Ad, partials);
+        });
+        g_kernel_launches++;
+        return;
+    }
     FHG_DISPATCH_BS_G(A.bs, A.lanes, {
         pdl_launch(k_bsr_spmv_dots<BS, G>, kReduceCtas, kReduceThreads, 0, s, A.nbr, A.rowptr, A.colidx, A.vals, A.ld, d, r,
                                                                       Ad, partials);
@@ -718,6 +836,14 @@ void launch_spmv_dots_df(const BsrView<float>& Ahi, const float* vlo, const floa
 void launch_spmv_dots_df_slot(const BsrView<dfl>& A, const float* dhi, const float* dlo, const float* rhi,
                               const float* rlo, float* Adhi, float* Adlo, double* partials, cudaStream_t s)
 {
+    if (A.cls) {
+        FHG_DISPATCH_CLS(A.bs, A.ell, {
+            pdl_launch(k_bsr_spmv_dots_df_cls<BS, W>, kReduceCtas, kReduceThreads, 0, s, A.nbr, A.cls, A.colidx, A.vals,
+                       (int)A.ld, dhi, dlo, rhi, rlo, Adhi, Adlo, partials);
+        });
+        g_kernel_launches++;
+        return;
+    }
 #define FHG_OUTER_SLOT(BSV, WV)                                                                              \
     if (A.bs == BSV && A.ell == WV) {                                                                       \
         pdl_launch(k_bsr_spmv_dots_df_slot<BSV, WV>, kReduceCtas, kReduceThreads, 0, s, A.nbr, A.colidx, A.vals, A.ld, \

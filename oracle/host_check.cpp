@@ -94,6 +94,25 @@ long long hc_symmetrise_lower(int n, const int* rp, const int* ci, const double*
     return unwrap(S, &rows, &cols, out_rp, out_ci, out_v, cap);
 }
 
+// The row classes of A (block size bs): their number, 0 when setup would not use them. W: off-diagonal
+// slots; cls, rep: n / bs entries each; col: 6 n / bs; dict: cap values, written when it holds them.
+int hc_row_classes(int n, const int* rp, const int* ci, const double* v, int bs, int max_classes, int min_rows, int* W,
+                   int* cls, int* rep, int* col, double* dict, long long cap)
+{
+    HostBsr B;
+    csr_to_bsr(wrap(n, n, rp, ci, v), bs, B);
+    RowClasses C;
+    if (!row_classes(B, max_classes, min_rows, C)) return 0;
+    *W = C.W;
+    std::copy(C.cls.begin(), C.cls.end(), cls);
+    std::copy(C.rep.begin(), C.rep.end(), rep);
+    std::copy(C.col.begin(), C.col.end(), col);
+    std::vector<double> d;
+    class_dictionary(B, C, nullptr, d);
+    if ((long long)d.size() <= cap) std::copy(d.begin(), d.end(), dict);
+    return C.ncls;
+}
+
 // Inverse of an n x n block (full pivoting); 0 when singular.
 int hc_invert_block(const double* a, int n, double* inv) { return invert_block(a, n, inv) ? 1 : 0; }
 

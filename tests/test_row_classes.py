@@ -1,0 +1,163 @@
+"""Row-class views (operators whose block rows repeat): the classes and dictionary that setup finds
+give the operator back bit for bit and are refused where rows do not repeat (CPU, through
+oracle/host_check.cpp); the sweeps, products and solves on them against the oracle in colour order, in every
+value type and block size, and against the stored-block views (GPU)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import oracle as O
+from test_host_setup import csr, dp, ip, lib
+
+from fhhos4_gb300 import hho
+
+MAX_CLASSES, MIN_ROWS = 1024, 64   # the limits of setup
+
+
+def classes(A, bs, max_classes=MAX_CLASSES, min_rows=MIN_ROWS):
+    """(W, cls, rep, col, dictionary (W + 2, bs, bs, ncls)) or None."""
+    rp, ci, va = csr(A)
+    n, nb = A.shape[0], A.shape[0] // bs
+    W, cls, rep, col = C.c_int(), np.zeros(nb, np.int32), np.zeros(nb, np.int32), np.zeros(6 * nb, np.int32)
+    dic = np.zeros(8 * bs * bs * max_classes)
+    k = lib().hc_row_classes(n, ip(rp), ip(ci), dp(va), bs, max_classes, min_rows, C.byref(W), ip(cls), ip(rep), ip(col),
+                             dp(dic), C.c_longlong(dic.size))
+    if k == 0:
+        return None
+    w = W.value
+    return w, cls, rep[:k], col[:w * nb].reshape(w, nb), dic[:(w + 2) * bs * bs * k].reshape(w + 2, bs, bs, k)
+
+
+def rebuild(n, bs, view):
+    """The operator the view stands for (empty slots: the row's own column)."""
+    W, cls, _, col, dic = view
+    nb = n // bs
+    rows, cols, vals = [], [], []
+    i = np.arange(nb)
+    for s in range(W + 1):
+        j = col[s] if s < W else i
+        keep = (j != i) if s < W else np.ones(nb, bool)
+        b = dic[s if s < W else W + 1][:, :, cls].transpose(2, 0, 1)[keep]
+        r = i[keep][:, None, None] * bs + np.arange(bs)[None, :, None]
+        c = j[keep][:, None, None] * bs + np.arange(bs)[None, None, :]
+        rows.append(np.broadcast_to(r, b.shape).ravel())
+        cols.append(np.broadcast_to(c, b.shape).ravel())
+        vals.append(b.ravel())
+    return sp.csr_matrix((np.concatenate(vals), (np.concatenate(rows), np.concatenate(cols))), shape=(n, n))
+
+
+@pytest.mark.parametrize("dim,n,k,coefficient", [(2, 40, 1, "identity"), (2, 41, 2, "identity"), (2, 40, 3, "identity"),
+                                                 (3, 8, 1, "identity"), (3, 12, 2, "checkerboard")])
+def test_classes_give_the_operator_back(dim, n, k, coefficient):
+    H = hho.Hierarchy(dim, n, k, max_levels=1, coefficient=coefficient, contrast=1e3)
+    A, bs = H.A(0), H.block_size
+    H.close()
+    got = classes(A, bs)
+    assert got is not None
+    assert got[0] == (4 if dim == 2 else 6)
+    assert abs(rebuild(A.shape[0], bs, got) - A).max() == 0.0
+    # first appearance: the representatives ascend and belong to their classes
+    assert np.all(np.diff(got[2]) > 0) and np.array_equal(got[1][got[2]], np.arange(len(got[2])))
+
+
+def test_operators_without_repeating_rows_are_refused():
+    H = hho.Hierarchy(3, 8, 1, max_levels=1)
+    A, bs = H.A(0), H.block_size
+    H.close()
+    got = classes(A, bs)
+    assert classes(A, bs, max_classes=len(got[2]) - 1) is None               # one class too many
+    assert classes(A, bs, max_classes=len(got[2])) is not None
+    assert classes(A, bs, min_rows=A.shape[0] // bs // len(got[2]) + 1) is None   # too few rows a class
+    noise = A.copy()
+    noise.data *= 1.0 + 1e-15 * np.random.default_rng(0).integers(0, 4, A.nnz)   # rows equal to rounding only
+    assert classes(noise, bs) is None
+    P = hho.Hierarchy(3, 8, 1)
+    G = (P.P(0).T @ P.A(0) @ P.P(0)).tocsr()                                  # more than 6 neighbours
+    P.close()
+    assert classes(G, bs, min_rows=1) is None
+    B = A.tolil()
+    B[0:bs, 0:bs] = 0
+    B = B.tocsr()
+    B.eliminate_zeros()                                                        # a row without a diagonal block
+    assert classes(B, bs) is None
+
+
+PREC = {"fp64": (np.float64, 1e-13), "df": (None, 1e-12), "fp32": (np.float32, 1e-5)}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "df", "fp32"])
+@pytest.mark.parametrize("dim,n,k,omega", [(2, 36, 1, 1.0), (2, 36, 2, 1.0), (2, 36, 3, 1.3), (3, 8, 1, 1.0), (3, 8, 1, 1.3),
+                                           (3, 8, 2, 1.0)])
+def test_gpu_sweeps_and_products_on_class_views(dim, n, k, omega, precision):
+    """Level-0 sweeps, SpMV and residual against the oracle in FP64 and colour order. Tolerance: a row
+    of up to 42 products in FP64 (2^-53), pairs (2^-47) or FP32 (2^-24), scaled by the operator."""
+    torch = pytest.importorskip("torch")
+    from fhhos4_gb300 import _native as N
+    from fhhos4_gb300 import solver as S
+    from test_gpu_parity import scalar_perm
+    As, Ps, _, bs = hho.generate(dim, n, k)
+    assert classes(As[0], bs) is not None
+    solver = S.fcg_mg(As, Ps, bs, precision=precision, omega=omega)
+    ctx = solver.Context()
+    rows = As[0].shape[0]
+    s = scalar_perm(ctx.permutation(0, rows // bs), bs)
+    Ap = O.as_csr(As[0][s][:, s])
+    rng = np.random.default_rng(5)
+    x, b = rng.standard_normal(rows), rng.standard_normal(rows)
+
+    def put(v):
+        if precision == "df":
+            hi = v.astype(np.float32)
+            return torch.tensor(np.stack([hi, (v - hi).astype(np.float32)], 1), device="cuda")
+        return torch.tensor(v.astype(PREC[precision][0]), device="cuda")
+
+    def get(t):
+        a = t.cpu().numpy().astype(np.float64)
+        return a[:, 0] + a[:, 1] if precision == "df" else a
+
+    xd, bd = put(x), put(b)
+    x, b = get(xd), get(bd)
+    out = torch.empty_like(xd)
+    tol = PREC[precision][1]
+    scale = abs(Ap).sum(axis=1).max() * np.abs(x).max() + np.abs(b).max()
+    ctx.apply_internal(0, N.OP_SPMV, precision, xd.data_ptr(), None, out.data_ptr())
+    assert np.abs(get(out) - Ap @ x).max() <= tol * scale
+    ctx.apply_internal(0, N.OP_RESIDUAL, precision, xd.data_ptr(), bd.data_ptr(), out.data_ptr())
+    assert np.abs(get(out) - (b - Ap @ x)).max() <= tol * scale
+    for op, backward in ((N.OP_GS_FORWARD, False), (N.OP_GS_BACKWARD, True)):
+        ctx.apply_internal(0, op, precision, xd.data_ptr(), bd.data_ptr(), out.data_ptr())
+        ref = O.block_gs(Ap, bs, b, x, backward=backward) if omega == 1.0 else None
+        if ref is None:   # block SOR: a forced row-major layout of the same precision
+            other = S.fcg_mg(As, Ps, bs, precision=precision, omega=omega, gs_layout="row")
+            o2 = torch.empty_like(xd)
+            other.Context().apply_internal(0, op, precision, xd.data_ptr(), bd.data_ptr(), o2.data_ptr())
+            ref = get(o2)
+            other.Context().close()
+        assert np.abs(get(out) - ref).max() <= 50 * tol * np.abs(ref).max()
+    ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "df", "fp32"])
+@pytest.mark.parametrize("dim,n,k", [(2, 48, 3), (3, 16, 1), (3, 8, 2)])
+def test_gpu_solves_on_class_views_track_stored_blocks(dim, n, k, precision):
+    """The same solve on class views and on the stored-block views (row-major): FP64 and pairs to 1e-10 of
+    the solution with equal iterations, FP32 within one iteration."""
+    from fhhos4_gb300 import solver as S
+    As, Ps, b, bs = hho.generate(dim, n, k)
+    kw = dict(precision=precision, nu=(2, 2), fused=False)
+    a = S.fcg_mg(As, Ps, bs, **kw)
+    r = S.fcg_mg(As, Ps, bs, gs_layout="row", **kw)
+    xa, xr = a.Solve(b), r.Solve(b)
+    if precision == "fp32":
+        assert abs(a.IterationCount - r.IterationCount) <= 1
+        assert np.linalg.norm(b - As[0] @ xa) <= 1e-8 * (1 + 1e-6) * np.linalg.norm(b)
+    else:
+        assert a.IterationCount == r.IterationCount
+        assert np.linalg.norm(xa - xr) <= 1e-10 * np.linalg.norm(xr)
+        assert a.TrueRelativeResidual == pytest.approx(r.TrueRelativeResidual, rel=1e-3)
+    for s in (a, r):
+        s.Context().close()
