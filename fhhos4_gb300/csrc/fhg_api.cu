@@ -800,13 +800,21 @@ void kcycle_fcg(fhg_ctx* ctx, int m, T* r, T* x)
     fhg::launch_lincomb<T>(n, alpha1 / rho1 - gamma * alpha2 / (rho1 * rho2), c, alpha2 / rho2, d, x, s);
 }
 
-// Lanes of the fused kernel per block row of an operator: enough for the average row's blocks to be
-// loaded together, a power of two from 4 to 16.
-template <class T>
-int fused_lanes(const BsrView<T>& B)
+// Threads per block row of a phase of the one-launch sub-cycle: `each` blocks of the average row to a thread
+// (2 to 32 threads), but no more threads than leave the phase's rows in one pass of the cluster.
+int fused_lanes(double blocks_per_row, int each, int rows, int threads)
 {
-    const double avg = B.nbr ? (double)B.nnzb / B.nbr : 1.0;
-    return avg <= 5.0 ? 4 : avg <= 12.0 ? 8 : 16;
+    int g = 2;
+    while (g < 32 && g * each < blocks_per_row) g *= 2;
+    while (g > 2 && (long long)rows * g > threads) g /= 2;
+    return g;
+}
+
+int largest_colour(const Level& L)
+{
+    int m = 0;
+    for (int c = 0; c < L.ncolours; c++) m = std::max(m, L.colour_start[c + 1] - L.colour_start[c]);
+    return m;
 }
 
 // The coarse sub-cycle from level l down as one cluster launch (fhg_coarse.cu), when setup found the
@@ -820,11 +828,12 @@ bool fused_cycle(fhg_ctx* ctx, int l, const T* b, T* x, bool x_zero)
     } else {
         using V = LevelVecs<T>;
         const fhg_options& o = ctx->opts;
-        if (!o.fused_coarse || l != ctx->fused_from[V::kPrec] || l <= 0 || o.w_loops == FHG_CYCLE_K ||
-            !is_gs(o.pre_smoother) || !is_gs(o.post_smoother))
+        const int from = ctx->fused_from[V::kPrec];
+        if (!o.fused_coarse || l != from || l <= 0 || o.w_loops == FHG_CYCLE_K || !is_gs(o.pre_smoother) ||
+            !is_gs(o.post_smoother))
             return false;
-        Level& L0 = ctx->levels[l];
-        if (b != V::b(L0) || x != V::x(L0)) return false;
+        const int npre_c = o.coarse_pre_iterations >= 0 ? o.coarse_pre_iterations : o.pre_iterations;
+        const int npost_c = o.coarse_post_iterations >= 0 ? o.coarse_post_iterations : o.post_iterations;
         auto dir = [](int code) {
             switch (code) {
             case FHG_SMOOTHER_BGS: return fhg::kFusedForward;
@@ -834,25 +843,27 @@ bool fused_cycle(fhg_ctx* ctx, int l, const T* b, T* x, bool x_zero)
             default: return fhg::kFusedAlternatingBackward;
             }
         };
+        const int ctas = ctx->fused_ctas[V::kPrec], cta_threads = ctx->fused_threads[V::kPrec], threads = ctas * cta_threads;
         fhg::FusedCycle<T> P;
         P.nlev = ctx->nlevels - l;
         P.pre = dir(o.pre_smoother);
         P.post = dir(o.post_smoother);
-        P.npre = o.coarse_pre_iterations >= 0 ? o.coarse_pre_iterations : o.pre_iterations;
-        P.npost = o.coarse_post_iterations >= 0 ? o.coarse_post_iterations : o.post_iterations;
+        P.npre = npre_c;
+        P.npost = npost_c;
         P.w_loops = o.w_loops > 1 ? o.w_loops : 1;
         P.x_zero = x_zero ? 1 : 0;
         P.omega = T(o.omega);
+        auto mean = [](const BsrView<T>& B) { return B.nbr ? (double)B.nnzb / B.nbr : 1.0; };
         for (int k = 0; k < P.nlev; k++) {
             Level& L = ctx->levels[l + k];
             fhg::FusedLevel<T>& F = P.lev[k];
             F.nb = L.nb;
-            F.x = V::x(L);
-            F.b = V::b(L);
-            F.r = V::r(L);
+            F.x = k == 0 ? x : nullptr;
+            F.b = k == 0 ? b : nullptr;
             if (l + k == ctx->nlevels - 1) {
                 P.n_coarse = L.n;
                 P.cinv = L.cinv;
+                P.c_lanes = fused_lanes(L.n, 16, L.n, threads);
                 continue;
             }
             F.ncol = L.ncolours;
@@ -864,45 +875,61 @@ bool fused_cycle(fhg_ctx* ctx, int l, const T* b, T* x, bool x_zero)
             F.p_rowptr = Pv.rowptr; F.p_colidx = Pv.colidx; F.p_vals = Pv.vals; F.p_ld = Pv.ld;
             const BsrView<T>& Rv = V::Rcsr(L);
             F.r_rowptr = Rv.rowptr; F.r_colidx = Rv.colidx; F.r_vals = Rv.vals; F.r_ld = Rv.ld;
-            F.lanes = fused_lanes(A);
-            F.t_lanes = fused_lanes(Rv);
-            const BsrView<T>* G = nullptr;
-            const BsrView<T>* Ap = nullptr;
-            if constexpr (std::is_same<T, float>::value) {
-                if (L.G32.vals) G = &L.G32.v;
-                if (L.A32p.vals) Ap = &L.A32p.v;
-            } else {
-                if (L.G2.vals) G = &L.G2.v;
-                if (L.A2p.vals) Ap = &L.A2p.v;
-            }
-            if (G && G->ell > 0 && G->ell <= F.lanes) {
-                F.g_ell = G->ell; F.g_colidx = G->colidx; F.g_vals = G->vals; F.g_ld = G->ld;
-            }
-            if (Ap && Ap->ell > 0 && Ap->ell <= F.lanes) {
-                F.ap_ell = Ap->ell; F.ap_colidx = Ap->colidx; F.ap_vals = Ap->vals; F.ap_ld = Ap->ld;
-            }
+            F.lanes = fused_lanes(mean(A), 1, largest_colour(L), threads);
+            F.a_lanes = fused_lanes(mean(A), 1, L.nb, threads);
+            F.p_lanes = fused_lanes(mean(Pv), 1, L.nb, threads);
+            F.r_lanes = fused_lanes(mean(Rv), 1, Rv.nbr, threads);
         }
-        if (fhg::launch_fused_cycle<T>(P, L0.bs, ctx->fused_ctas[V::kPrec], ctx->fused_threads[V::kPrec], ctx->stream) !=
-            cudaSuccess)
+        const int smem = fhg::fused_layout<T>(P, ctx->levels[l].bs, ctas);
+        if (smem < 0 || fhg::launch_fused_cycle<T>(P, ctx->levels[l].bs, ctas, cta_threads, smem, ctx->stream) != cudaSuccess)
             return false;
         fhg::g_kernel_launches++;
         return true;
     }
 }
 
-// First level (>= 1, above the coarsest) from which every level has at most max_rows block rows and
-// at most kFusedMaxColours colours, within kFusedMaxLevels levels, all of one block size and joined by
-// products with P (no natural injection); -1 when there is none.
-int fused_first_level(const fhg_ctx* ctx, int max_rows)
+// Whether the one-launch sub-cycle can take levels l and below: at most kFusedMaxLevels, of one block
+// size, joined by products with P (no natural injection), each of at most kFusedMaxRows block rows and
+// kFusedMaxColours colours.
+bool fused_eligible(const fhg_ctx* ctx, int l)
 {
     const int nlevels = ctx->nlevels;
-    for (int l = 1; l + 1 < nlevels; l++) {
-        bool ok = nlevels - l <= fhg::kFusedMaxLevels;
-        for (int k = l; k < nlevels && ok; k++)
-            ok = ctx->levels[k].nb <= max_rows && ctx->levels[k].bs == ctx->levels[l].bs &&
-                 (k == nlevels - 1 || (ctx->levels[k].ncolours <= fhg::kFusedMaxColours && !ctx->levels[k].inject));
-        if (ok) return l;
+    if (l + 1 >= nlevels || nlevels - l > fhg::kFusedMaxLevels) return false;
+    for (int k = l; k < nlevels; k++) {
+        const Level& L = ctx->levels[k];
+        if (L.nb > fhg::kFusedMaxRows || L.bs != ctx->levels[l].bs ||
+            (k < nlevels - 1 && (L.ncolours > fhg::kFusedMaxColours || L.inject)))
+            return false;
     }
+    return true;
+}
+
+// Clusters of the sub-cycle from level l that fit on the device at once, with `ctas` CTAs of `threads`
+// threads: 0 where its vectors do not fit the CTAs' shared memory or the device does not run the shape.
+template <class T>
+int fused_clusters(fhg_ctx* ctx, int l, int ctas, int threads)
+{
+    using V = LevelVecs<T>;
+    fhg::FusedCycle<T> P;
+    P.nlev = ctx->nlevels - l;
+    P.n_coarse = ctx->levels[ctx->nlevels - 1].n;
+    for (int k = 0; k < P.nlev; k++) {
+        Level& L = ctx->levels[l + k];
+        P.lev[k].nb = L.nb;
+        if (k + 1 == P.nlev) continue;
+        P.lev[k].a_ld = V::Acsr(L).ld;
+        P.lev[k].p_ld = V::Pcsr(L).ld;
+        P.lev[k].r_ld = V::Rcsr(L).ld;
+    }
+    const int bs = ctx->levels[l].bs;
+    return fhg::fused_cycle_clusters<T>(bs, ctas, threads, fhg::fused_layout<T>(P, bs, ctas));
+}
+
+// First level (>= 1, above the coarsest) that the sub-cycle can start from; -1 when there is none.
+int fused_first_level(const fhg_ctx* ctx)
+{
+    for (int l = 1; l + 1 < ctx->nlevels; l++)
+        if (fused_eligible(ctx, l)) return l;
     return -1;
 }
 
@@ -915,6 +942,7 @@ struct FusedKey {
 struct FusedChoice {
     int from = -1, ctas = fhg::kClusterCtasPortable, threads = fhg::kFusedThreads;
 };
+
 std::mutex g_fused_mutex;
 std::map<FusedKey, FusedChoice> g_fused_cache;
 
@@ -931,12 +959,12 @@ int choose_fused(fhg_ctx* ctx)
     constexpr int PR = V::kPrec;
     const fhg_options& o = ctx->opts;
     const int nlevels = ctx->nlevels;
-    const int first = fused_first_level(ctx, fhg::kFusedMaxRows);
+    const int first = fused_first_level(ctx);
     ctx->fused_from[PR] = -1;
     ctx->fused_ctas[PR] = fhg::kClusterCtasPortable;
     ctx->fused_threads[PR] = fhg::kFusedThreads;
     if (first < 0) return FHG_OK;
-    const int bs = ctx->levels[first].bs;   // every candidate level's (fused_first_level)
+    const int bs = ctx->levels[first].bs;
     FusedKey key;
     key.sig = {PR, ctx->levels[0].bs, bs, nlevels, o.pre_smoother, o.post_smoother, o.pre_iterations, o.post_iterations,
                o.coarse_pre_iterations, o.coarse_post_iterations, o.w_loops, o.omega == 1.0 ? 1 : 0};
@@ -978,8 +1006,8 @@ int choose_fused(fhg_ctx* ctx)
     FusedChoice choice;
     for (int threads : {fhg::kFusedThreads, fhg::kFusedThreadsWide}) {
         for (int ctas : {fhg::kClusterCtasPortable, fhg::kClusterCtasLarge}) {
-            if (fhg::fused_cycle_clusters<T>(bs, ctas, threads) < 1) continue;
             for (int l = first; l + 1 < nlevels; l++) {
+                if (fused_clusters<T>(ctx, l, ctas, threads) < 1) continue;
                 ctx->fused_from[PR] = l;
                 ctx->fused_ctas[PR] = ctas;
                 ctx->fused_threads[PR] = threads;
@@ -1022,15 +1050,13 @@ void release_unused_views(fhg_ctx* ctx)
 {
     for (int l = 0; l + 1 < ctx->nlevels; l++) {
         Level& L = ctx->levels[l];
-        // levels >= 1 keep their padded-row views: the one-launch coarse sub-cycle reads them
-        const bool keep_padded = l > 0;
-        if (L.G32s.vals && L.gs_slot[FHG_PREC_FP32]) { if (!keep_padded) release_bsr(ctx, L.G32); }
+        if (L.G32s.vals && L.gs_slot[FHG_PREC_FP32]) release_bsr(ctx, L.G32);
         else if (L.G32s.vals) release_bsr(ctx, L.G32s);
-        if (L.A32s.vals && L.prod_slot[FHG_PREC_FP32]) { if (!keep_padded) release_bsr(ctx, L.A32p); }
+        if (L.A32s.vals && L.prod_slot[FHG_PREC_FP32]) release_bsr(ctx, L.A32p);
         else if (L.A32s.vals) release_bsr(ctx, L.A32s);
-        if (L.G2s.vals && L.gs_slot[FHG_PREC_DF]) { if (!keep_padded) release_bsr(ctx, L.G2); }
+        if (L.G2s.vals && L.gs_slot[FHG_PREC_DF]) release_bsr(ctx, L.G2);
         else if (L.G2s.vals) release_bsr(ctx, L.G2s);
-        if (L.A2s.vals && L.prod_slot[FHG_PREC_DF]) { if (!keep_padded) release_bsr(ctx, L.A2p); }
+        if (L.A2s.vals && L.prod_slot[FHG_PREC_DF]) release_bsr(ctx, L.A2p);
         else if (L.A2s.vals) release_bsr(ctx, L.A2s);
         if (L.P32j.vals && !L.p_jds[FHG_PREC_FP32]) release_bsr(ctx, L.P32j);
         if (L.R32j.vals && !L.r_jds[FHG_PREC_FP32]) release_bsr(ctx, L.R32j);
@@ -1052,9 +1078,23 @@ void release_unused_views(fhg_ctx* ctx)
 // on several host threads do their host work concurrently without disturbing each other's timings.
 std::recursive_mutex g_timing_mutex;
 
-// The coarse sub-cycle of every V-cycle precision the context holds: off, by timing (autotuning), or
-// from the first level of at most kFusedDefaultRows block rows with 8 CTAs. Called at setup and when
-// the cycle changes.
+// The sub-cycle's start without timing: the first level from which no level has more than
+// kFusedDefaultRows block rows, with 8 CTAs. A phase takes about 2 us, as much as a colour's launch on
+// such a level; above it the whole GPU's launches are faster (32^3 k = 1, FP32: a cycle from 5,760 rows down
+// 123 us in one launch of 16 CTAs, 55 us launch by launch).
+template <class T>
+void default_fused(fhg_ctx* ctx, int threads)
+{
+    constexpr int PR = LevelVecs<T>::kPrec;
+    int from = -1;
+    for (int l = ctx->nlevels - 2; l >= 1 && ctx->levels[l].nb <= fhg::kFusedDefaultRows && fused_eligible(ctx, l); l--) from = l;
+    if (from < 0 || fused_clusters<T>(ctx, from, fhg::kClusterCtasPortable, threads) < 1) return;
+    ctx->fused_from[PR] = from;
+    ctx->fused_threads[PR] = threads;
+}
+
+// The coarse sub-cycle of every V-cycle precision the context holds: off, by timing (autotuning), or by
+// default_fused. Called at setup and when the cycle changes.
 int refresh_fused(fhg_ctx* ctx)
 {
     std::lock_guard<std::recursive_mutex> timing(g_timing_mutex);
@@ -1067,25 +1107,16 @@ int refresh_fused(fhg_ctx* ctx)
     }
     if (!o.fused_coarse || o.w_loops == FHG_CYCLE_K || !is_gs(o.pre_smoother) || !is_gs(o.post_smoother))
         return FHG_OK;
-    int rc = FHG_OK;
+    const int threads = !o.autotune && o.fused_coarse == 2 ? fhg::kFusedThreadsWide : fhg::kFusedThreads;
     if (o.autotune) {
+        int rc = FHG_OK;
         if (fp32 && (rc = choose_fused<float>(ctx))) return rc;
         if (pair && (rc = choose_fused<dfl>(ctx))) return rc;
         return cudaStreamSynchronize(ctx->stream) == cudaSuccess ? FHG_OK
                                                                  : fail(ctx, FHG_ERR_CUDA, "coarse sub-cycle timing failed");
     }
-    const int first = fused_first_level(ctx, fhg::kFusedDefaultRows);
-    if (first < 0) return FHG_OK;
-    const int bs = ctx->levels[first].bs;
-    const int threads = o.fused_coarse == 2 ? fhg::kFusedThreadsWide : fhg::kFusedThreads;
-    if (fp32 && fhg::fused_cycle_clusters<float>(bs, fhg::kClusterCtasPortable, threads) >= 1) {
-        ctx->fused_from[FHG_PREC_FP32] = first;
-        ctx->fused_threads[FHG_PREC_FP32] = threads;
-    }
-    if (pair && fhg::fused_cycle_clusters<dfl>(bs, fhg::kClusterCtasPortable, threads) >= 1) {
-        ctx->fused_from[FHG_PREC_DF] = first;
-        ctx->fused_threads[FHG_PREC_DF] = threads;
-    }
+    if (fp32) default_fused<float>(ctx, threads);
+    if (pair) default_fused<dfl>(ctx, threads);
     return FHG_OK;
 }
 
@@ -2144,23 +2175,21 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                 (rc = build_class_views(ctx, Ap, inv.data(), L.C64, &L.C32, L.C2)))
                 return rc;
         }
-        // The row- and slot-major views of stored blocks: not beside class views, but for the padded rows of
-        // levels >= 1, which the one-launch coarse sub-cycle reads.
+        // The row- and slot-major views of stored blocks: not beside class views.
         const bool classes = L.C64.vals != nullptr;
-        const bool padded = !classes || (l > 0 && o.fused_coarse);
         // slot-major views (GS sweeps and products): when forced, or for the autotuner to compare
         const bool want_slot = o.colouring && !classes && (o.gs_layout == FHG_GS_SLOT || (o.gs_layout == FHG_GS_AUTO && o.autotune));
         if (fp32 && l < nlevels - 1) {
-            if (o.colouring && padded && (rc = upload_padded(ctx, Ap, L.G32, true, 8))) return rc;
-            if (padded && (rc = upload_padded(ctx, Ap, L.A32p, false, 8))) return rc;
+            if (o.colouring && !classes && (rc = upload_padded(ctx, Ap, L.G32, true, 8))) return rc;
+            if (!classes && (rc = upload_padded(ctx, Ap, L.A32p, false, 8))) return rc;
             if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G32s))) return rc;
             if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A32s))) return rc;
             L.gs_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.G32s.vals;
             L.prod_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.A32s.vals;
         }
         if (pair && l < nlevels - 1) {
-            if (o.colouring && padded && (rc = upload_padded(ctx, Ap, L.G2, true, 8))) return rc;
-            if (padded && (rc = upload_padded(ctx, Ap, L.A2p, false, 8))) return rc;
+            if (o.colouring && !classes && (rc = upload_padded(ctx, Ap, L.G2, true, 8))) return rc;
+            if (!classes && (rc = upload_padded(ctx, Ap, L.A2p, false, 8))) return rc;
             if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G2s))) return rc;
             if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A2s))) return rc;
             L.gs_slot[FHG_PREC_DF] = o.gs_layout == FHG_GS_SLOT && L.G2s.vals;

@@ -1,30 +1,35 @@
 // The coarse part of a multigrid cycle in one kernel launch.
 //
-// Below some level the operators are small (tens of thousands of block rows or fewer) and a cycle
-// there is a long chain of short phases: every colour of every smoothing sweep, the residual, the
-// restriction, the coarsest solve, the prolongation. Launched one kernel per phase, each costs a
-// launch slot of a few microseconds while its work takes a fraction of that. Here one thread-block
-// cluster (8 or 16 CTAs, co-scheduled by the hardware) runs the whole sub-cycle: every phase
-// spreads its rows over all threads of the cluster, and phases are separated by the hardware
-// cluster barrier (barrier.cluster with release/acquire semantics at cluster scope, which orders the
-// global-memory writes of one phase before the reads of the next across the cluster's CTAs). The
-// barrier cannot wait forever: all CTAs of a cluster are resident together and every thread takes
-// the same path through the cycle.
+// Below some level the operators are small (thousands of block rows) and a cycle there is a long chain
+// of short phases: every colour of every smoothing sweep, the residual, the restriction, the coarsest
+// solve, the prolongation. Launched one kernel per phase, each costs 1.7 us or more (2.5 in pairs) while its
+// work takes a fraction of that. Here one thread-block cluster (8 or 16 CTAs, co-scheduled by the
+// hardware) runs the whole sub-cycle: every phase spreads its rows over the CTAs, and phases are separated
+// by the hardware cluster barrier. The barrier cannot wait forever: all CTAs of a cluster are resident
+// together and every thread takes the same path through the cycle.
 //
-// A block row is walked by a group of `lanes` threads (block p of the row by lane p mod lanes,
-// partial sums added by shuffles), and each group keeps up to four rows in flight (all their loads
-// issued before the sums), so that loads overlap: one thread per row waits for them one after another,
-// and a phase of a few rows per thread is a chain of memory round trips. The cycle runs as a loop over levels with a
-// count of coarse corrections per level (no device recursion, so the stack is fixed at compile time).
+// The vectors x, b and r of every level live in the cluster's distributed shared memory, so what one phase
+// writes the next reads without a trip through L2: a store to global memory, the release and the load back
+// take 0.9 us between two barriers, through distributed shared memory 0.4 us (measured, 512-thread CTAs; the
+// barrier alone 0.24 us, with 8 CTAs as with 16). Block row i belongs to one CTA (chunks of kChunk rows dealt
+// out in turn), which holds its entries and computes it; only the entries of other rows that a row walk
+// gathers are remote. Matrix data stays in L2 and never changes: row bounds are loaded two phases ahead and
+// block columns one, so that a phase waits for one round trip (values, D^-1 and the gathered entries
+// together), the sums and the barrier. A block row is walked by a group of 2 to 32 threads, partial sums
+// added by shuffles; warps without a row of the phase go straight to the barrier. The cycle runs as a loop
+// over levels with a count of coarse corrections per level (no device recursion, so the stack is fixed at
+// compile time).
 //
 // The arithmetic is the multigrid cycle of Multigrid::MultigridCycle (src/Solver/Multigrid/
 // Multigrid.h:438-608) on the levels it covers: block Gauss-Seidel / SOR sweeps in colour order
 // (BlockGaussSeidel.h:84-120, BlockSOR.h:199-227), r = b - A x (Multigrid.h:478), R r (Level.h:139-143),
 // the coarse correction (V, or W with WLoops: repeated on the same right-hand side, except directly
 // above the coarsest level), the coarsest dense solve, x += P e (Level.h:150-154, Multigrid.h:554).
-// The FP32 and pair (dfl) value types are instantiated.
+// The FP32 and pair (dfl) value types are instantiated: in FP64 the phases are bound by the FP64 pipe of the
+// cluster's SMs, and the launches are faster.
 #include "fhg_coarse.h"
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -32,13 +37,11 @@ namespace fhg {
 
 namespace {
 
-// Every thread of the cluster arrives (release) and waits (acquire); the non-aligned form does not
-// require the threads of a warp to arrive together.
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release;\n"
-                 "barrier.cluster.wait.acquire;\n" ::: "memory");
-}
+// Every thread of the cluster arrives (release) when its writes of a phase are done and waits (acquire)
+// before it reads what others wrote; the non-aligned form does not require the threads of a warp to
+// arrive together. Each arrive is followed by exactly one wait.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
 
 __device__ __forceinline__ void pdl_wait_coarse() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
@@ -65,201 +68,337 @@ __device__ __forceinline__ double lanes_sum(double v, int g)
     return v;
 }
 
+// One block's BS values from distributed shared memory (address of the CTA that holds them, aligned to
+// their own size), in the widest loads their size allows. Volatile: not moved across the barrier.
+template <class T, int BS>
+__device__ __forceinline__ void load_remote(unsigned addr, T (&out)[BS])
+{
+    constexpr int kBytes = BS * (int)sizeof(T);
+    float f[kBytes / 4];
+    if constexpr (kBytes % 16 == 0) {
+#pragma unroll
+        for (int q = 0; q < kBytes / 16; q++)
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                         : "=f"(f[4 * q]), "=f"(f[4 * q + 1]), "=f"(f[4 * q + 2]), "=f"(f[4 * q + 3]) : "r"(addr + 16 * q));
+    } else if constexpr (kBytes % 8 == 0) {
+#pragma unroll
+        for (int q = 0; q < kBytes / 8; q++)
+            asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];\n" : "=f"(f[2 * q]), "=f"(f[2 * q + 1]) : "r"(addr + 8 * q));
+    } else {
+#pragma unroll
+        for (int q = 0; q < kBytes / 4; q++)
+            asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(f[q]) : "r"(addr + 4 * q));
+    }
+#pragma unroll
+    for (int c = 0; c < BS; c++) {
+        if constexpr (std::is_same<T, float>::value) out[c] = f[c];
+        else if constexpr (std::is_same<T, double>::value)
+            out[c] = __hiloint2double(__float_as_int(f[2 * c + 1]), __float_as_int(f[2 * c]));
+        else out[c] = T(f[2 * c], f[2 * c + 1]);
+    }
+}
+
 template <class T>
 struct Ctx {
     const FusedCycle<T>& P;
-    long long t, nthr;   // thread index within the cluster, threads of the cluster
+    char* smem;                // the CTA's dynamic shared memory
+    unsigned saddr;            // its shared-window address
+    int rank, log_ctas;        // this CTA in the cluster, log2 of the cluster's CTAs
+    int warp, nwarps, lane;    // of the CTA
+
+    // Block row of local row u, and how many of the block rows below row are this CTA's.
+    __device__ __forceinline__ int row(int u) const
+    {
+        return ((((u >> kChunkLog) << log_ctas) + rank) << kChunkLog) | (u & (kChunk - 1));
+    }
+    __device__ __forceinline__ int local_rows(int row) const
+    {
+        const int c = row >> kChunkLog, owner = c & ((1 << log_ctas) - 1), full = (c >> log_ctas) << kChunkLog;
+        return full + (owner > rank ? kChunk : owner == rank ? (row & (kChunk - 1)) : 0);
+    }
+    // Where block row j's entries of the vector at byte offset `off` are: an address in the cluster.
+    __device__ __forceinline__ unsigned remote(int off, int j, int bytes) const
+    {
+        const int c = j >> kChunkLog;
+        const unsigned a = saddr + off + ((((c >> log_ctas) << kChunkLog) | (j & (kChunk - 1))) * bytes);
+        unsigned r;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(a), "r"(c & ((1 << log_ctas) - 1)));
+        return r;
+    }
+    __device__ __forceinline__ T* local(int off) const { return reinterpret_cast<T*>(smem + off); }
 };
 
-// Rows [r0, r1) of a phase, `g` lanes per row: calls f(i, valid, lane) in passes that every thread
-// of the cluster takes the same number of times (the shuffles of a group need all lanes of the warp).
-template <class T, class F>
-__device__ __forceinline__ void row_passes(const Ctx<T>& C, long long r0, long long r1, int g, F f)
+// A block operator in CSR form, entry-major values.
+template <class T>
+struct Rows {
+    const int* rowptr;
+    const int* colidx;
+    const T* vals;
+    unsigned ld;   // entries of the levels here fit 32 bits (fused_layout)
+};
+
+// The local rows [lo, hi) of a phase, and a lane's place in its first row: the row's bounds (p: the lane's
+// first block; it takes p, p + g, ...) and its first columns (-1: none).
+struct Span {
+    int lo = 0, hi = 0;
+};
+struct Bounds {
+    int p = 0, p1 = 0;
+};
+template <int N>
+struct Columns {
+    int col[N];
+};
+
+template <class T>
+__device__ __forceinline__ Bounds row_bounds(const Ctx<T>& C, const Rows<T>& M, int u, int hi, int g)
 {
-    const long long gid = C.t / g, ngroups = C.nthr / g;
-    const int lane = (int)(C.t % g);
-    const long long passes = (r1 - r0 + ngroups - 1) / ngroups;
-    for (long long ps = 0; ps < passes; ps++) {
-        const long long i = r0 + ps * ngroups + gid;
-        f(i, i < r1, lane);
+    Bounds b;
+    if (u < hi) {
+        const int i = C.row(u);
+        b.p = M.rowptr[i] + (C.lane & (g - 1));
+        b.p1 = M.rowptr[i + 1];
     }
+    return b;
 }
 
-// Rows [r0, r1) of a phase with `g` lanes per row and R rows per group in flight: in each pass a group
-// takes R rows, loads the row bounds of all R, then each step loads one block of every row (column
-// index, the x entries it names, the values) before any sum, so the loads of R rows overlap instead of
-// following one another. A row is summed block by block in each lane's order (blocks lane, lane + g,
-// ...), then over the lanes by shuffles. emit(i, lane, acc) runs for every valid row after the sums.
-template <class T, int BS, int R, class Emit>
-__device__ __forceinline__ void rows_multi(const Ctx<T>& C, long long r0, long long r1, int g, int ell,
-                                           const int* __restrict__ rowptr, const int* __restrict__ colidx,
-                                           const T* __restrict__ vals, long long ld, const T* x, bool skip_diag,
-                                           Emit emit)
+template <int N, class T>
+__device__ __forceinline__ Columns<N> row_columns(const Rows<T>& M, const Bounds& b, int g)
 {
-    const long long gid = C.t / g, ngroups = C.nthr / g;
-    const int lane = (int)(C.t % g);
-    const long long span = ngroups * R;
-    const long long passes = (r1 - r0 + span - 1) / span;
-    for (long long ps = 0; ps < passes; ps++) {
-        int i[R];   // rows and columns fit in 32 bits (at most kFusedMaxRows block rows)
-        int p0[R], p1[R];
+    Columns<N> c;
 #pragma unroll
-        for (int q = 0; q < R; q++) {
-            const long long iq = r0 + ps * span + (long long)q * ngroups + gid;
-            i[q] = (int)iq;
-            const bool v = iq < r1;
-            if (ell > 0) {   // padded rows: no row-pointer round trip
-                p0[q] = v ? i[q] * ell : 0;
-                p1[q] = v ? p0[q] + ell : 0;
-            } else {
-                p0[q] = v ? rowptr[i[q]] : 0;
-                p1[q] = v ? rowptr[i[q] + 1] : 0;
+    for (int q = 0; q < N; q++) c.col[q] = b.p + q * g < b.p1 ? M.colidx[b.p + q * g] : -1;
+    return c;
+}
+
+// Blocks of a row a lane has in flight at once (columns ahead, then values and gathered entries), by the
+// bytes of a block: 128 registers of a 512-thread CTA, 64 of a 1024-thread one. kHold: the values in registers
+// (else as the sums reach them).
+template <class T, int BS, int TH>
+constexpr int kLaneBlocks = TH > kFusedThreads ? 1
+                            : BS * BS * (int)sizeof(T) <= 16 ? 4 : BS * BS * (int)sizeof(T) <= 36 ? 2 : 1;
+template <class T, int BS, int TH>
+constexpr bool kHold = BS * BS * (int)sizeof(T) <= (TH > kFusedThreads ? 16 : 36);
+
+enum { kRowAssign = 0, kRowAdd = 1, kRowResidual = 2, kRowSweep = 3 };
+
+// One phase over this CTA's rows `span` of M, `g` lanes per row, src: the byte offset of the gathered vector:
+//   kRowAssign    out_i = (M src)_i, and zero_i = 0 (the next level's first x)
+//   kRowAdd       out_i += (M src)_i
+//   kRowResidual  out_i = b_i - (M src)_i
+//   kRowSweep     out_i = omega D_i^-1 (b_i - sum_{j != i} M_ij src_j) + (1 - omega) out_i, out = src
+// b, out and zero are the CTA's own parts. Output r of a row is written by lane r mod g. bounds, cols: the
+// warp's first row, loaded ahead; on return those of the span `next`, with the bounds of `after` (the next
+// two phases on M, empty spans where there are none). Waits for the barrier that the phase before arrived at,
+// and arrives at the next.
+template <class T, int BS, int TH, int KIND>
+__device__ __forceinline__ void rows_phase(const Ctx<T>& C, Span span, int g, const Rows<T>& M, Bounds& bounds,
+                                           Columns<kLaneBlocks<T, BS, TH>>& cols,
+                                           Bounds& next_bounds, Span next, Span after, int src, const T* dinv, int nb,
+                                           const T* b, T* out, T* zero)
+{
+    constexpr int NB = kLaneBlocks<T, BS, TH>;
+    constexpr bool HOLD = kHold<T, BS, TH>, SWEEP = KIND == kRowSweep;
+    const int lane = C.lane & (g - 1), group = C.warp * (32 / g) + C.lane / g, stride = C.nwarps * (32 / g);
+    cluster_wait();
+    bool ahead = false;   // the next phases' data asked for
+    for (int base = span.lo + C.warp * (32 / g); base < span.hi || !ahead; base += stride) {   // warp-uniform
+        const int u = base + C.lane / g;
+        const bool in = u < span.hi;
+        const int i = C.row(u);
+        Bounds at = bounds;
+        Columns<NB> now = cols;
+        T acc[BS], dv[BS];
+#pragma unroll
+        for (int r = 0; r < BS; r++) acc[r] = T(0);
+        if (base < span.hi) {
+            if (SWEEP) {
+                unsigned dld = nb;
+                asm volatile("" : "+r"(dld));
+#pragma unroll
+                for (int c = 0; c < BS; c++) dv[c] = in && lane < BS ? dinv[(unsigned)(lane * BS + c) * dld + (unsigned)i] : T(0);
             }
         }
-        T acc[R][BS];
+        bool first = true;
+        while (true) {
+            unsigned ld = M.ld;   // opaque, so that the entries' offsets are not kept in registers between rows
+            asm volatile("" : "+r"(ld));
+            if (SWEEP) {
 #pragma unroll
-        for (int q = 0; q < R; q++)
-#pragma unroll
-            for (int r = 0; r < BS; r++) acc[q][r] = T(0);
-        for (int base = lane;; base += g) {
-            bool ok[R], any = false;
-            int col[R];
-#pragma unroll
-            for (int q = 0; q < R; q++) {
-                ok[q] = p0[q] + base < p1[q];
-                any |= ok[q];
-                col[q] = ok[q] ? colidx[p0[q] + base] : 0;
+                for (int q = 0; q < NB; q++)
+                    if (now.col[q] == i) now.col[q] = -1;   // the diagonal block: D^-1 instead
             }
-            if (!any) break;   // per lane; no shuffle inside the loop
-            T xv[R][BS], av[R][BS * BS];
+            T xv[NB][BS], v[HOLD ? NB : 1][BS * BS];
 #pragma unroll
-            for (int q = 0; q < R; q++) {
+            for (int q = 0; q < NB; q++) {
+                const int j = now.col[q];
 #pragma unroll
-                for (int c = 0; c < BS; c++) xv[q][c] = ok[q] ? x[(long long)col[q] * BS + c] : T(0);
+                for (int c = 0; c < BS; c++) xv[q][c] = T(0);
+                if (j >= 0) {
+                    if (HOLD) {
+                        const T* vp = M.vals + (at.p + q * g);
 #pragma unroll
-                for (int e = 0; e < BS * BS; e++) av[q][e] = ok[q] ? vals[(long long)e * ld + p0[q] + base] : T(0);
+                        for (int e = 0; e < BS * BS; e++, vp += ld) v[q][e] = *vp;
+                    }
+                    load_remote<T, BS>(C.remote(src, j, BS * (int)sizeof(T)), xv[q]);
+                }
+            }
+            if (first) {   // behind the loads this row waits for
+                first = false;
+                if (base + stride < span.hi) {   // another pass of this phase
+                    bounds = row_bounds(C, M, u + stride, span.hi, g);
+                } else if (!ahead) {
+                    ahead = true;
+                    bounds = next_bounds;
+                    cols = row_columns<NB>(M, bounds, g);
+                    next_bounds = row_bounds(C, M, after.lo + group, after.hi, g);
+                }
             }
 #pragma unroll
-            for (int q = 0; q < R; q++) {
-                if (!ok[q] || (skip_diag && col[q] == i[q])) continue;
+            for (int q = 0; q < NB; q++) {
+                if (now.col[q] < 0) continue;
 #pragma unroll
                 for (int r = 0; r < BS; r++)
 #pragma unroll
-                    for (int c = 0; c < BS; c++) acc[q][r] = fma(av[q][r * BS + c], xv[q][c], acc[q][r]);
+                    for (int c = 0; c < BS; c++) {
+                        const T a = HOLD ? v[q][r * BS + c] : M.vals[(unsigned)(r * BS + c) * ld + (unsigned)(at.p + q * g)];
+                        acc[r] = fma(a, xv[q][c], acc[r]);
+                    }
+            }
+            at.p += NB * g;
+            if (at.p >= at.p1) break;   // per lane; no shuffle inside the loop
+            now = row_columns<NB>(M, at, g);
+        }
+        if (base >= span.hi) break;   // a warp without a row: only asked for the next phases' data
+        if (base + stride < span.hi) cols = row_columns<NB>(M, bounds, g);
+#pragma unroll
+        for (int r = 0; r < BS; r++) acc[r] = lanes_sum(acc[r], g);
+        if (!in) continue;
+        if (SWEEP) {
+            const T w = C.P.omega;
+            T t[BS];
+#pragma unroll
+            for (int c = 0; c < BS; c++) t[c] = b[u * BS + c] - acc[c];
+            for (int r = lane; r < BS; r += g) {
+                T y = T(0);
+#pragma unroll
+                for (int c = 0; c < BS; c++)
+                    y = fma(r == lane ? dv[c] : dinv[(unsigned)(r * BS + c) * (unsigned)nb + (unsigned)i], t[c], y);
+                if (w != T(1)) y = fma(w, y, (T(1) - w) * out[u * BS + r]);
+                out[u * BS + r] = fin(y);
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < BS; r++) {
+                if (r % g != lane) continue;
+                const int k = u * BS + r;
+                if (KIND == kRowAssign) {
+                    out[k] = fin(acc[r]);
+                    zero[k] = T(0);
+                } else if (KIND == kRowResidual) {
+                    out[k] = b[k] - acc[r];
+                } else {
+                    out[k] = out[k] + acc[r];
+                }
             }
         }
-#pragma unroll
-        for (int q = 0; q < R; q++)
-#pragma unroll
-            for (int r = 0; r < BS; r++) acc[q][r] = lanes_sum(acc[q][r], g);
-#pragma unroll
-        for (int q = 0; q < R; q++)
-            if (i[q] < r1) emit((long long)i[q], lane, acc[q]);
     }
+    cluster_arrive();
 }
 
-// Rows in flight per lane group, by the bytes of a block: what fits in 128 registers (512-thread
-// CTAs) without spills; one row with 64 registers (1024-thread CTAs).
-template <class T, int BS, int THREADS>
-constexpr int kRowsInFlight = THREADS > kFusedThreads ? 1
-                              : BS * BS * (int)sizeof(T) <= 16 ? 4 : BS * BS * (int)sizeof(T) <= 36 ? 3
-                              : BS * BS * (int)sizeof(T) <= 72 ? 2 : 1;
-
-// One colour [c0, c1) of a block GS / SOR sweep on level L: x_i <- D_i^-1 (b_i - sum_{j != i} A_ij x_j),
-// relaxed by omega; output r of a row written by lane r (lanes loop when BS > lanes).
-template <class T, int BS, int TH>
-__device__ void gs_colour(const Ctx<T>& C, const FusedLevel<T>& L, int c0, int c1)
+// A phase of its own over all rows (residual, transfers): its first columns loaded between the barrier's
+// arrive and wait.
+template <class T, int BS, int TH, int KIND>
+__device__ __forceinline__ void product(const Ctx<T>& C, int rows, int g, const Rows<T>& M, int src, const T* b, T* out, T* zero)
 {
-    const T w = C.P.omega;
-    const bool pad = L.g_ell > 0;
-    rows_multi<T, BS, kRowsInFlight<T, BS, TH>>(C, c0, c1, L.lanes, L.g_ell, L.a_rowptr, pad ? L.g_colidx : L.a_colidx,
-                                            pad ? L.g_vals : L.a_vals, pad ? L.g_ld : L.a_ld, L.x, true,
-                                            [&](long long i, int lane, const T* acc) {
-        for (int r = lane; r < BS; r += L.lanes) {
-            T v = T(0);
-#pragma unroll
-            for (int c = 0; c < BS; c++) v = fma(L.dinv[(long long)(r * BS + c) * L.nb + i], L.b[i * BS + c] - acc[c], v);
-            if (w != T(1)) v = fma(w, v, (T(1) - w) * L.x[i * BS + r]);
-            L.x[i * BS + r] = fin(v);
-        }
-    });
-    cluster_sync();
+    constexpr int NB = kLaneBlocks<T, BS, TH>;
+    const Span span{0, C.local_rows(rows)};
+    Bounds bounds = row_bounds(C, M, C.warp * (32 / g) + C.lane / g, span.hi, g), none;
+    Columns<NB> cols = row_columns<NB>(M, bounds, g);
+    rows_phase<T, BS, TH, KIND>(C, span, g, M, bounds, cols, none, Span(), Span(), src, nullptr, 0, b, out, zero);
 }
 
-template <class T, int BS, int TH>
-__device__ void sweep(const Ctx<T>& C, const FusedLevel<T>& L, bool backward)
-{
-    if (!backward)
-        for (int c = 0; c < L.ncol; c++) gs_colour<T, BS, TH>(C, L, L.colour_start[c], L.colour_start[c + 1]);
-    else
-        for (int c = L.ncol - 1; c >= 0; c--) gs_colour<T, BS, TH>(C, L, L.colour_start[c], L.colour_start[c + 1]);
-}
-
-// The smoother directions of BlockGaussSeidel::ExecuteOneIteration (alternating ones by iteration parity).
+// `iters` smoothing steps on level L in the direction of the smoother code: the sweeps of
+// BlockGaussSeidel::ExecuteOneIteration (alternating ones by iteration parity), one phase per colour.
 template <class T, int BS, int TH>
 __device__ void smooth(const Ctx<T>& C, const FusedLevel<T>& L, int code, int iters)
 {
-    for (int it = 0; it < iters; it++) {
-        if (code == kFusedForward) sweep<T, BS, TH>(C, L, false);
-        else if (code == kFusedBackward) sweep<T, BS, TH>(C, L, true);
-        else if (code == kFusedSymmetric) { sweep<T, BS, TH>(C, L, false); sweep<T, BS, TH>(C, L, true); }
-        else if (code == kFusedAlternatingForward) sweep<T, BS, TH>(C, L, it % 2 != 0);
-        else sweep<T, BS, TH>(C, L, it % 2 == 0);
+    const Rows<T> A{L.a_rowptr, L.a_colidx, L.a_vals, (unsigned)L.a_ld};
+    const int sweeps = code == kFusedSymmetric ? 2 * iters : iters, g = L.lanes, group = C.warp * (32 / g) + C.lane / g;
+    if (sweeps == 0) return;
+    int s = 0, k = 0;   // sweep and colour of the next span
+    auto next_span = [&]() {
+        Span r;
+        if (s >= sweeps) return r;
+        const bool backward = code == kFusedBackward || (code == kFusedAlternatingBackward && !(s & 1)) ||
+                              ((code == kFusedSymmetric || code == kFusedAlternatingForward) && (s & 1));
+        const int c = backward ? L.ncol - 1 - k : k;
+        r.lo = C.local_rows(L.colour_start[c]);
+        r.hi = C.local_rows(L.colour_start[c + 1]);
+        if (++k == L.ncol) {
+            k = 0;
+            s++;
+        }
+        return r;
+    };
+    Span now = next_span(), next = next_span(), after = next_span();
+    Bounds bounds = row_bounds(C, A, now.lo + group, now.hi, g);
+    Bounds next_bounds = row_bounds(C, A, next.lo + group, next.hi, g);
+    Columns<kLaneBlocks<T, BS, TH>> cols = row_columns<kLaneBlocks<T, BS, TH>>(A, bounds, g);
+    for (int phase = sweeps * L.ncol; phase > 0; phase--) {
+        rows_phase<T, BS, TH, kRowSweep>(C, now, g, A, bounds, cols, next_bounds, next, after, L.x_off, L.dinv, L.nb,
+                                         C.local(L.b_off), C.local(L.x_off), nullptr);
+        now = next;
+        next = after;
+        after = next_span();
     }
 }
 
-// L.r = L.b - A x (all blocks, the diagonal included).
-template <class T, int BS, int TH>
-__device__ void residual(const Ctx<T>& C, const FusedLevel<T>& L)
-{
-    const bool pad = L.ap_ell > 0;
-    rows_multi<T, BS, kRowsInFlight<T, BS, TH>>(C, 0, L.nb, L.lanes, L.ap_ell, L.a_rowptr, pad ? L.ap_colidx : L.a_colidx,
-                                            pad ? L.ap_vals : L.a_vals, pad ? L.ap_ld : L.a_ld, L.x, false,
-                                            [&](long long i, int lane, const T* acc) {
-        for (int r = lane; r < BS; r += L.lanes) L.r[i * BS + r] = L.b[i * BS + r] - acc[r];
-    });
-    cluster_sync();
-}
-
-// out (rows of M) = M in, or out += M in: the transfers as block products over CSR operators.
-template <class T, int BS, int TH>
-__device__ void product(const Ctx<T>& C, int rows, int g, const int* rowptr, const int* colidx, const T* vals,
-                        long long ld, const T* in, T* out, bool add)
-{
-    rows_multi<T, BS, kRowsInFlight<T, BS, TH>>(C, 0, rows, g, 0, rowptr, colidx, vals, ld, in, false,
-                                            [&](long long i, int lane, const T* acc) {
-        for (int r = lane; r < BS; r += g) out[i * BS + r] = add ? out[i * BS + r] + acc[r] : fin(acc[r]);
-    });
-    cluster_sync();
-}
-
-template <class T>
-__device__ void zero(const Ctx<T>& C, T* x, long long n)
-{
-    for (long long i = C.t; i < n; i += C.nthr) x[i] = T(0);
-    cluster_sync();
-}
-
-// The coarsest level: x = C^{-1} b, C^{-1} dense FP64 row-major, FP64 accumulation; 8 lanes a row.
-template <class T>
+// The coarsest level: x = C^{-1} b, C^{-1} dense FP64 row-major, FP64 accumulation. Every CTA gathers all
+// of b in FP64, then computes its own rows, c_lanes lanes a row; the matrix is read eight entries a lane at
+// a time, the first eight ahead of the barrier.
+template <class T, int BS>
 __device__ void coarse_solve(const Ctx<T>& C, const FusedLevel<T>& L)
 {
-    const long long n = C.P.n_coarse;
-    row_passes(C, 0, n, 8, [&](long long i, bool valid, int lane) {
+    constexpr int kAtOnce = 8;
+    const int n = C.P.n_coarse, g = C.P.c_lanes, tid = C.warp * 32 + C.lane;
+    const int rows = C.local_rows(L.nb) * BS, lane = C.lane & (g - 1), stride = C.nwarps * (32 / g);
+    double* bc = reinterpret_cast<double*>(C.smem + C.P.bc_off);
+    T* x = C.local(L.x_off);
+    double a[kAtOnce];
+    auto load = [&](int k, int j) {
+        const double* row = C.P.cinv + (long long)(C.row(k / BS) * BS + k % BS) * n;
+#pragma unroll
+        for (int q = 0; q < kAtOnce; q++) a[q] = k < rows && j + q * g < n ? row[j + q * g] : 0.0;
+    };
+    int k = C.warp * (32 / g) + C.lane / g;
+    load(k, lane);
+    cluster_wait();
+    for (int j = tid; j < L.nb; j += C.nwarps * 32) {
+        T v[BS];
+        load_remote<T, BS>(C.remote(L.b_off, j, BS * (int)sizeof(T)), v);
+#pragma unroll
+        for (int c = 0; c < BS; c++) bc[j * BS + c] = (double)v[c];
+    }
+    __syncthreads();
+    for (int base = C.warp * (32 / g); base < rows; base += stride, k += stride) {   // warp-uniform
+        if (base >= stride) load(k, lane);
         double acc = 0.0;
-        if (valid) {
-            const double* a = C.P.cinv + i * n;
-            for (long long j = lane; j < n; j += 8) acc = fma(a[j], (double)L.b[j], acc);
+        for (int j = lane; j < n; j += kAtOnce * g) {
+            if (j != lane) load(k, j);
+#pragma unroll
+            for (int q = 0; q < kAtOnce; q++) acc = fma(a[q], j + q * g < n ? bc[j + q * g] : 0.0, acc);
         }
-        acc = lanes_sum(acc, 8);
-        if (valid && lane == 0) L.x[i] = T(acc);
-    });
-    cluster_sync();
+        acc = lanes_sum(acc, g);
+        if (k < rows && lane == 0) x[k] = T(acc);
+    }
+    cluster_arrive();
 }
 
-// The cycle from lev[0] down: descend (zero x on a fresh level, pre-smooth, residual, restrict) to the
+// The cycle from lev[0] down: descend (pre-smooth, residual, restrict and zero the next x) to the
 // coarsest, solve there, then ascend (prolongate, post-smooth) until a level still owes a coarse
-// correction (W-cycle), from which the next descent starts with the coarser level's x kept.
+// correction (W-cycle), from which the next descent starts with the coarser level's x kept. b and x of
+// lev[0] come from and x goes back to global memory.
 template <class T, int BS, int TH>
 __device__ void run_cycle(const Ctx<T>& C)
 {
@@ -267,19 +406,26 @@ __device__ void run_cycle(const Ctx<T>& C)
     const int last = P.nlev - 1;
     int done[kFusedMaxLevels];   // coarse corrections completed on each level of the current descent
     int l = 0;
-    bool xz = P.x_zero != 0;
+    const FusedLevel<T>& L0 = P.lev[0];
+    const int own = C.local_rows(L0.nb) * BS, tid = C.warp * 32 + C.lane;
+    for (int k = tid; k < own; k += C.nwarps * 32) {
+        const long long i = (long long)C.row(k / BS) * BS + k % BS;
+        C.local(L0.b_off)[k] = L0.b[i];
+        C.local(L0.x_off)[k] = P.x_zero ? T(0) : L0.x[i];
+    }
+    cluster_arrive();
     while (true) {
         for (; l < last; l++) {
             const FusedLevel<T>& L = P.lev[l];
             const FusedLevel<T>& N = P.lev[l + 1];
-            if (xz) zero(C, L.x, (long long)L.nb * BS);
             smooth<T, BS, TH>(C, L, P.pre, P.npre);
-            residual<T, BS, TH>(C, L);
-            product<T, BS, TH>(C, N.nb, L.t_lanes, L.r_rowptr, L.r_colidx, L.r_vals, L.r_ld, L.r, N.b, false);
+            product<T, BS, TH, kRowResidual>(C, L.nb, L.a_lanes, {L.a_rowptr, L.a_colidx, L.a_vals, (unsigned)L.a_ld}, L.x_off,
+                                             C.local(L.b_off), C.local(L.r_off), nullptr);
+            product<T, BS, TH, kRowAssign>(C, N.nb, L.r_lanes, {L.r_rowptr, L.r_colidx, L.r_vals, (unsigned)L.r_ld}, L.r_off, nullptr,
+                                           C.local(N.b_off), C.local(N.x_off));
             done[l] = 0;
-            xz = true;
         }
-        coarse_solve(C, P.lev[last]);
+        coarse_solve<T, BS>(C, P.lev[last]);
         bool again = false;
         while (l > 0) {
             l--;
@@ -291,20 +437,24 @@ __device__ void run_cycle(const Ctx<T>& C)
             }
             const FusedLevel<T>& L = P.lev[l];
             const FusedLevel<T>& N = P.lev[l + 1];
-            product<T, BS, TH>(C, L.nb, L.lanes, L.p_rowptr, L.p_colidx, L.p_vals, L.p_ld, N.x, L.x, true);
+            product<T, BS, TH, kRowAdd>(C, L.nb, L.p_lanes, {L.p_rowptr, L.p_colidx, L.p_vals, (unsigned)L.p_ld}, N.x_off, nullptr,
+                                        C.local(L.x_off), nullptr);
             smooth<T, BS, TH>(C, L, P.post, P.npost);
         }
-        if (!again) return;
-        l++;          // the next coarse correction of level l - 1 starts on level l
-        xz = false;   // from the x the previous one left
+        if (!again) break;
+        l++;   // the next coarse correction of level l - 1 starts on level l, from the x the last one left
     }
+    cluster_wait();   // the last phase's barrier: no CTA leaves before the others have read its memory
+    for (int k = tid; k < own; k += C.nwarps * 32) L0.x[(long long)C.row(k / BS) * BS + k % BS] = C.local(L0.x_off)[k];
 }
 
 template <class T, int BS, int TH>
 __global__ void __launch_bounds__(TH, 1) k_fused_cycle(const __grid_constant__ FusedCycle<T> P)
 {
+    extern __shared__ __align__(16) char fused_smem[];
     pdl_wait_coarse();
-    const Ctx<T> C{P, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x};
+    const Ctx<T> C{P, fused_smem, (unsigned)__cvta_generic_to_shared(fused_smem), (int)blockIdx.x, 31 - __clz((int)gridDim.x),
+                   (int)(threadIdx.x >> 5), (int)(blockDim.x >> 5), (int)(threadIdx.x & 31)};
     run_cycle<T, BS, TH>(C);
 }
 
@@ -328,11 +478,12 @@ void* kernel_for(int bs, int threads)
     return nullptr;
 }
 
-void fused_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ctas, int threads, cudaStream_t s)
+void fused_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ctas, int threads, int smem, cudaStream_t s)
 {
     cfg = {};
     cfg.gridDim = dim3(ctas);
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ctas;
@@ -344,29 +495,51 @@ void fused_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ctas, 
     cfg.numAttrs = 2;
 }
 
-// Clusters above the portable size need the kernel's opt-in attribute, set once per kernel.
+// Clusters above the portable size and shared memory above 48 KB need the kernel's opt-ins.
 std::mutex g_fused_attr_mutex;
 
-cudaError_t allow_large_clusters(const void* k)
+cudaError_t allow_fused(const void* k)
 {
     std::lock_guard<std::mutex> lock(g_fused_attr_mutex);
-    return cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedMaxSmem);
+    return e == cudaSuccess ? cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : e;
 }
 
 }  // namespace
 
 template <class T>
-int fused_cycle_clusters(int bs, int ctas, int threads)
+int fused_layout(FusedCycle<T>& P, int bs, int ctas)
+{
+    long long at = 0;
+    auto take = [&](long long bytes) {
+        const long long o = at;
+        at += (bytes + 15) / 16 * 16;
+        return (int)std::min<long long>(o, 1 << 30);
+    };
+    for (int k = 0; k < P.nlev; k++) {
+        FusedLevel<T>& L = P.lev[k];
+        if (std::max({L.a_ld, L.p_ld, L.r_ld, (long long)L.nb}) * bs * bs >= 1LL << 31) return -1;   // 32-bit indices
+        const long long chunks = (L.nb + kChunk - 1) / kChunk, own = (chunks + ctas - 1) / ctas * kChunk;
+        L.x_off = take(own * bs * (long long)sizeof(T));
+        L.b_off = take(own * bs * (long long)sizeof(T));
+        if (k + 1 < P.nlev) L.r_off = take(own * bs * (long long)sizeof(T));
+    }
+    P.bc_off = take(8LL * P.n_coarse);
+    return at <= kFusedMaxSmem ? (int)at : -1;
+}
+
+template <class T>
+int fused_cycle_clusters(int bs, int ctas, int threads, int smem)
 {
     const void* k = kernel_for<T>(bs, threads);
-    if (!k || (ctas != kClusterCtasPortable && ctas != kClusterCtasLarge)) return 0;
-    if (ctas > kClusterCtasPortable && allow_large_clusters(k) != cudaSuccess) {
+    if (!k || smem < 0 || (ctas != kClusterCtasPortable && ctas != kClusterCtasLarge)) return 0;
+    if (allow_fused(k) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    fused_config(cfg, attr, ctas, threads, nullptr);
+    fused_config(cfg, attr, ctas, threads, smem, nullptr);
     cfg.numAttrs = 1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
@@ -377,20 +550,23 @@ int fused_cycle_clusters(int bs, int ctas, int threads)
 }
 
 template <class T>
-cudaError_t launch_fused_cycle(const FusedCycle<T>& P, int bs, int ctas, int threads, cudaStream_t s)
+cudaError_t launch_fused_cycle(const FusedCycle<T>& P, int bs, int ctas, int threads, int smem, cudaStream_t s)
 {
     const void* k = kernel_for<T>(bs, threads);
     if (!k) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[2];
-    fused_config(cfg, attr, ctas, threads, s);
+    fused_config(cfg, attr, ctas, threads, smem, s);
     void* args[] = {const_cast<FusedCycle<T>*>(&P)};
     return cudaLaunchKernelExC(&cfg, k, args);
 }
 
-template cudaError_t launch_fused_cycle<float>(const FusedCycle<float>&, int, int, int, cudaStream_t);
-template cudaError_t launch_fused_cycle<dfl>(const FusedCycle<dfl>&, int, int, int, cudaStream_t);
-template int fused_cycle_clusters<float>(int, int, int);
-template int fused_cycle_clusters<dfl>(int, int, int);
+#define FHG_FUSED_INSTANCES(T)                                                                      \
+    template cudaError_t launch_fused_cycle<T>(const FusedCycle<T>&, int, int, int, int, cudaStream_t); \
+    template int fused_cycle_clusters<T>(int, int, int, int);                                      \
+    template int fused_layout<T>(FusedCycle<T>&, int, int);
+FHG_FUSED_INSTANCES(float)
+FHG_FUSED_INSTANCES(dfl)
+#undef FHG_FUSED_INSTANCES
 
 }  // namespace fhg

@@ -135,16 +135,16 @@ typedef struct {
                                    in the reference. */
     int fused_coarse;           /* 1 (default): with GS / SOR smoothers and a V or W cycle in FP32 or DF, the cycle
                                    below some level (>= 1) runs as one thread-block-cluster launch (8 or 16 CTAs,
-                                   phases separated by the cluster barrier) instead of one launch per colour and
-                                   product. With autotune, setup (and fhg_set_cycle / fhg_set_coarse_smoothing)
-                                   times one cycle below level 0 launch by launch and fused from every eligible
-                                   level (every level below it at most 65,536 block rows and 24 colours, at most
-                                   6 levels) and keeps the fastest, per precision and hierarchy structure;
-                                   without, it fuses from the first level of at most 8,192 block rows with 8
-                                   CTAs of 512 threads. Timing also tries CTAs of 1024 threads (twice the warps
-                                   per SM, one row in flight per lane group). 2: as 1, but without autotuning
-                                   the CTAs have 1024 threads. 0: launch by launch. Same arithmetic up to the
-                                   summation order of a row. */
+                                   the levels' vectors in distributed shared memory, phases separated by the
+                                   cluster barrier) instead of one launch per colour and product. With autotune,
+                                   setup (and fhg_set_cycle / fhg_set_coarse_smoothing) times one cycle below
+                                   level 0 launch by launch and fused from every eligible level (every level below
+                                   it at most 65,536 block rows and 64 colours, at most 6 levels, the vectors
+                                   within the CTAs' shared memory) and keeps the fastest, per precision and
+                                   hierarchy structure; without, it fuses from the first level of at most 768
+                                   block rows with 8 CTAs of 512 threads. Timing also tries CTAs of 1024 threads.
+                                   2: as 1, but without autotuning the CTAs have 1024 threads. 0: launch by
+                                   launch. Same arithmetic up to the summation order of a row. */
 } fhg_options;
 
 typedef struct {
