@@ -450,6 +450,94 @@ __global__ void __launch_bounds__(kThreads) k_bsr_gs(int row0, int row1, const i
     }
 }
 
+// One colour of block GS over long rows (the Galerkin operators, whose rows hold 25 to 130 blocks in
+// colours of tens to a thousand rows): TPR threads of a 128-thread CTA walk a row, one block each as far as
+// it goes. Such a launch is bound by latency, not by bytes: a warp per row took the row's blocks 32 at a
+// time, each step waiting for its columns and then for its x entries (9.5 us a colour of 40 rows of 124
+// blocks in pairs). Here a thread has its block's column, values and its D^-1 row on the way before it waits
+// for the kernel ahead, then one gather, the sums (shuffles, then shared memory across the row's warps) and
+// the store remain. Column rules as in k_bsr_gs.
+constexpr int kLongThreads = 128;
+
+template <class T, int BS, int TPR>
+__global__ void __launch_bounds__(kLongThreads) k_bsr_gs_long(int row0, int row1, const int* __restrict__ rowptr,
+                                                              const int* __restrict__ colidx,
+                                                              const T* __restrict__ vals, long long ld,
+                                                              const T* __restrict__ dinv, long long dld,
+                                                              const T* __restrict__ b, T* x, int col_lo, int col_hi, T omega)
+{
+    constexpr bool HOLD = BS * BS * (int)sizeof(T) <= 128;   // values in registers ahead of the wait
+    constexpr int kWarps = kLongThreads / 32, kRowWarps = TPR / 32;
+    __shared__ T part[kWarps][BS];
+    const int tid = threadIdx.x, lane = tid % TPR;
+    const int row = row0 + (int)blockIdx.x * (kLongThreads / TPR) + tid / TPR;
+    const bool in = row < row1;
+    int p = 0, p1 = 0;
+    if (in) {
+        p = rowptr[row] + lane;
+        p1 = rowptr[row + 1];
+    }
+    int col = -1;
+    T v[HOLD ? BS * BS : 1], dv[BS], bv[BS], acc[BS];
+    auto load = [&]() {
+        col = colidx[p];
+        if (HOLD) {
+#pragma unroll
+            for (int e = 0; e < BS * BS; e++) v[e] = vals[(long long)e * ld + p];
+        }
+    };
+    if (p < p1) load();
+    const bool writes = in && lane < BS;
+    if (writes)
+#pragma unroll
+        for (int c = 0; c < BS; c++) dv[c] = dinv[(long long)(lane * BS + c) * dld + row];
+    pdl_wait();
+    if (writes)
+#pragma unroll
+        for (int c = 0; c < BS; c++) bv[c] = b[(long long)row * BS + c];
+#pragma unroll
+    for (int r = 0; r < BS; r++) acc[r] = T(0);
+    while (p < p1) {
+        if (col != row && col >= col_lo && col < col_hi) {
+            T xv[BS];
+#pragma unroll
+            for (int c = 0; c < BS; c++) xv[c] = x[(long long)col * BS + c];
+#pragma unroll
+            for (int r = 0; r < BS; r++)
+#pragma unroll
+                for (int c = 0; c < BS; c++) {
+                    const T a = HOLD ? v[r * BS + c] : vals[(long long)(r * BS + c) * ld + p];
+                    acc[r] = fma(a, xv[c], acc[r]);
+                }
+        }
+        p += TPR;
+        if (p < p1) load();
+    }
+#pragma unroll
+    for (int r = 0; r < BS; r++) acc[r] = group_sum<32>(acc[r]);
+    if (kRowWarps > 1) {
+        const int warp = tid >> 5;
+        if ((tid & 31) == 0)
+#pragma unroll
+            for (int r = 0; r < BS; r++) part[warp][r] = fin(acc[r]);
+        __syncthreads();
+        if (writes) {   // the row's first warp
+#pragma unroll
+            for (int w = 1; w < kRowWarps; w++)
+#pragma unroll
+                for (int r = 0; r < BS; r++) acc[r] += part[warp + w][r];
+        }
+    }
+    if (writes) {
+        T y = T(0);
+#pragma unroll
+        for (int c = 0; c < BS; c++) y = fma(dv[c], bv[c] - acc[c], y);
+        const long long i = (long long)row * BS + lane;
+        if (omega != T(1)) y = fma(omega, y, (T(1) - omega) * x[i]);   // block SOR
+        x[i] = fin(y);
+    }
+}
+
 // One colour of block GS on a slot-major padded view (slot_major, ell = W): one thread per block
 // row. Slot s of row i of the colour [row0, row1) lives at row0 * W + s * (row1 - row0) + (i - row0),
 // so a warp's loads of one slot are 32 consecutive words. The W column indices, then the used
@@ -1086,6 +1174,38 @@ void launch_gs_slot(const BsrView<T>& A, int row0, int row1, const T* dinv, long
     }
 }
 
+// Threads per row of k_bsr_gs_long: one block to a thread, but a single warp per row where the colour's rows
+// fill the GPU by themselves (16 CTAs of 128 threads per SM).
+template <class T, int BS>
+void gs_long_bs(const BsrView<T>& A, int row0, int row1, const T* dinv, long long dld, const T* b, T* x, cudaStream_t s,
+                int col_lo, int col_hi, T omega)
+{
+    const double mean = (double)A.nnzb / A.nbr;
+    const int rows = row1 - row0;
+    const int tpr = rows > 152 * 16 * 4 || mean <= 32.0 ? 32 : mean <= 64.0 ? 64 : 128;
+    const unsigned grid = grid_for((long long)rows * tpr, kLongThreads);
+    auto go = [&](auto kernel) {
+        pdl_launch(kernel, grid, kLongThreads, 0, s, row0, row1, A.rowptr, A.colidx, A.vals, A.ld, dinv, dld, b, x, col_lo,
+                   col_hi, omega);
+    };
+    if (tpr == 32) go(k_bsr_gs_long<T, BS, 32>);
+    else if (tpr == 64) go(k_bsr_gs_long<T, BS, 64>);
+    else go(k_bsr_gs_long<T, BS, 128>);
+}
+
+template <class T>
+void gs_long(const BsrView<T>& A, int row0, int row1, const T* dinv, long long dld, const T* b, T* x, cudaStream_t s,
+             int col_lo, int col_hi, T omega)
+{
+    switch (A.bs) {
+    case 2: gs_long_bs<T, 2>(A, row0, row1, dinv, dld, b, x, s, col_lo, col_hi, omega); break;
+    case 3: gs_long_bs<T, 3>(A, row0, row1, dinv, dld, b, x, s, col_lo, col_hi, omega); break;
+    case 4: gs_long_bs<T, 4>(A, row0, row1, dinv, dld, b, x, s, col_lo, col_hi, omega); break;
+    case 6: gs_long_bs<T, 6>(A, row0, row1, dinv, dld, b, x, s, col_lo, col_hi, omega); break;
+    default: break;
+    }
+}
+
 template <class T>
 void launch_gs(const BsrView<T>& A, int row0, int row1, const T* dinv, long long dld, const T* b, T* x, cudaStream_t s,
                int col_lo, int col_hi, T omega)
@@ -1110,6 +1230,11 @@ void launch_gs(const BsrView<T>& A, int row0, int row1, const T* dinv, long long
             g_kernel_launches++;
             return;
         }
+    }
+    if (A.lanes == 32 && A.ell == 0) {   // long rows
+        gs_long<T>(A, row0, row1, dinv, dld, b, x, s, col_lo, col_hi, omega);
+        g_kernel_launches++;
+        return;
     }
     FHG_DISPATCH_BS_G(A.bs, A.lanes, {
         const unsigned grid = grid_for((long long)(row1 - row0) * G, kThreads);
