@@ -38,9 +38,9 @@ template <class T>
 struct DevBsr {
     BsrView<T> v;
     T* vals = nullptr;
-    int* rowptr = nullptr;   // row pointers (CSR), or the row permutation of a jagged view
+    int* rowptr = nullptr;   // row pointers (CSR), or the row permutation of a sliced view
     int* colidx = nullptr;
-    int* jds_start = nullptr;  // slot offsets of a jagged view
+    int* slices = nullptr;     // slice offsets of a sliced view
     bool owns_index = true;
 };
 
@@ -74,11 +74,12 @@ struct Level {
     DevBsr<double> C64, Co64;
     DevBsr<float> C32;
     DevBsr<dfl> C2, Co2;
-    // jagged (JDS) views of the transfers, levels 0 and 1 (the large ones), and whether the products
-    // use them (per V-cycle precision, chosen by timing at setup)
-    DevBsr<float> P32j, R32j;
-    DevBsr<dfl> P2j, R2j;
-    bool p_jds[3] = {false, false, false}, r_jds[3] = {false, false, false};
+    // sliced views of the transfers, and whether the products use them (per V-cycle precision: by rule, or
+    // chosen by timing at setup)
+    DevBsr<double> P64s, R64s;
+    DevBsr<float> P32s, R32s;
+    DevBsr<dfl> P2s, R2s;
+    bool p_sell[3] = {false, false, false}, r_sell[3] = {false, false, false};
     dfl* dinv2 = nullptr;
     dfl *x2 = nullptr, *b2 = nullptr, *r2 = nullptr;
     dfl* kv2[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -431,51 +432,72 @@ int upload_slot_major_all(fhg_ctx* ctx, const HostBsr& B, DevBsr<T>& D)
     return FHG_OK;
 }
 
-// Jagged (JDS) view of a transfer operator: rows stably sorted by decreasing block count, slot s of
-// sorted row k at start[s] + k, values entry-major with no padding. Not built above 64 blocks a row.
+// Sliced view of a transfer operator with `lanes` threads per row (BsrView::sell_perm): rows stably sorted by
+// decreasing block count within windows of kSellWindow rows, slices as long as their longest row. Left empty
+// when the padding adds more than a quarter.
+constexpr int kSellWindow = 1024;
+
 template <class T>
-int upload_jds(fhg_ctx* ctx, const HostBsr& B, DevBsr<T>& D)
+int upload_sell(fhg_ctx* ctx, const HostBsr& B, int lanes, DevBsr<T>& D)
 {
     D = DevBsr<T>();
-    const int nbr = B.nbr;
-    int W = 0;
-    for (int i = 0; i < nbr; i++) W = std::max(W, B.rowptr[i + 1] - B.rowptr[i]);
-    if (nbr == 0 || W == 0 || W > 64) return FHG_OK;
-    std::vector<int> perm(nbr);
-    for (int i = 0; i < nbr; i++) perm[i] = i;
-    std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) {
-        return B.rowptr[a + 1] - B.rowptr[a] > B.rowptr[b + 1] - B.rowptr[b];
-    });
-    std::vector<int> start(W + 1, 0);
-    for (int sl = 0; sl < W; sl++) {
-        int rows = 0;
-        while (rows < nbr && B.rowptr[perm[rows] + 1] - B.rowptr[perm[rows]] > sl) rows++;
-        start[sl + 1] = start[sl] + rows;
+    const int nbr = B.nbr, rows = 32 / lanes, slices = (nbr + rows - 1) / rows;
+    if (nbr == 0) return FHG_OK;
+    auto blocks = [&](int i) { return B.rowptr[i + 1] - B.rowptr[i]; };
+    std::vector<int> perm((size_t)slices * rows, -1), ptr(slices + 1, 0);
+    std::iota(perm.begin(), perm.begin() + nbr, 0);
+    for (int w = 0; w < nbr; w += kSellWindow)
+        std::stable_sort(perm.begin() + w, perm.begin() + std::min(nbr, w + kSellWindow),
+                         [&](int a, int b) { return blocks(a) > blocks(b); });
+    long long slots = 0;
+    for (int q = 0; q < slices; q++) {
+        int longest = 0;   // the first row's, but where a slice spans two windows
+        for (int k = q * rows; k < std::min(nbr, (q + 1) * rows); k++) longest = std::max(longest, blocks(perm[k]));
+        slots += 32LL * ((longest + lanes - 1) / lanes);
+        if (slots > INT32_MAX) return FHG_OK;
+        ptr[q + 1] = (int)slots;
     }
-    const long long nnzb = B.nnzb();
+    if (slots > B.nnzb() + B.nnzb() / 4 + 1024) return FHG_OK;
     const int bb = B.bs * B.bs;
-    const long long ld = round_up(std::max<long long>(nnzb, 1), 32);
-    std::vector<int> col((size_t)nnzb);
+    const long long ld = round_up(std::max<long long>(slots, 1), 32);
+    std::vector<int> col((size_t)ld, -1);
     std::vector<T> soa((size_t)ld * bb, T(0));
-    for (int sl = 0; sl < W; sl++)
-        for (int k = 0; k < start[sl + 1] - start[sl]; k++) {
-            const long long p = B.rowptr[perm[k]] + sl;
-            const long long q = start[sl] + k;
-            col[(size_t)q] = B.colidx[(size_t)p];
-            for (int e = 0; e < bb; e++) soa[(size_t)e * ld + q] = (T)B.vals[(size_t)p * bb + e];
+    parallel_rows(slices * rows, [&](int lo, int hi) {
+        for (int k = lo; k < hi; k++) {
+            if (perm[k] < 0) continue;
+            const long long first = ptr[k / rows] + (long long)(k % rows) * lanes;
+            const int p0 = B.rowptr[perm[k]];
+            for (int j = 0; j < blocks(perm[k]); j++) {
+                const long long q = first + j % lanes + 32LL * (j / lanes);
+                col[(size_t)q] = B.colidx[p0 + j];
+                for (int e = 0; e < bb; e++) soa[(size_t)e * ld + q] = (T)B.vals[(size_t)(p0 + j) * bb + e];
+            }
         }
+    });
     int rc;
-    int *dperm = nullptr, *dstart = nullptr;
-    if ((rc = upload(ctx, &dperm, perm.data(), perm.size())) || (rc = upload(ctx, &dstart, start.data(), start.size())) ||
+    int *dperm = nullptr, *dptr = nullptr;
+    if ((rc = upload(ctx, &dperm, perm.data(), perm.size())) || (rc = upload(ctx, &dptr, ptr.data(), ptr.size())) ||
         (rc = upload(ctx, &D.colidx, col.data(), col.size())) || (rc = upload(ctx, &D.vals, soa.data(), soa.size())))
         return rc;
-    D.rowptr = dperm;   // owned with the view (freed with it): the permutation and the slot offsets
-    D.v.nbr = B.nbr; D.v.nbc = B.nbc; D.v.bs = B.bs; D.v.nnzb = nnzb; D.v.ld = ld;
+    D.rowptr = dperm;   // owned with the view (freed with it): the permutation and the slice offsets
+    D.slices = dptr;
+    D.v.nbr = B.nbr; D.v.nbc = B.nbc; D.v.bs = B.bs; D.v.nnzb = B.nnzb(); D.v.ld = ld;
     D.v.rowptr = nullptr; D.v.colidx = D.colidx; D.v.vals = D.vals;
-    D.v.jds_perm = dperm; D.v.jds_start = dstart; D.v.jds_slots = W;
+    D.v.sell_lanes = lanes; D.v.sell_perm = dperm; D.v.sell_ptr = dptr;
     D.v.lanes = 1;
-    D.jds_start = dstart;
     return FHG_OK;
+}
+
+// Threads per row of a transfer's sliced view, 0 for CSR. The rows of P (at most 7 blocks) take a thread each
+// from kSellRowsP rows on (at 19,872 rows the CSR form is faster: 7.0 against 8.7 us with 6 x 6 blocks in FP32;
+// at 47,616 the sliced one: 3.5 against 4.1 in FP32, 11.5 against 17.1 in FP64); the longer rows of R four, or
+// eight where there are fewer, down to kSellRowsR.
+constexpr int kSellRowsP = 32768, kSellRowsR4 = 16384, kSellRowsR = 4096;
+
+int sell_lanes(const HostBsr& M, bool prolongation)
+{
+    if (prolongation) return M.nbr >= kSellRowsP ? 1 : 0;
+    return M.nbr >= kSellRowsR4 ? 4 : M.nbr >= kSellRowsR ? 8 : 0;
 }
 
 // The dictionary of a row-class view in T over classes and columns already on the device.
@@ -620,8 +642,10 @@ template <> struct LevelVecs<double> {
     static double* b(Level& L) { return L.b; }
     static double* r(Level& L) { return L.r; }
     static const BsrView<double>& A(Level& L) { return L.C64.vals ? L.C64.v : L.A.v; }
-    static const BsrView<double>& P(Level& L) { return L.P.v; }
-    static const BsrView<double>& R(Level& L) { return L.R.v; }
+    static const BsrView<double>& P(Level& L) { return L.p_sell[kPrec] && L.P64s.vals ? L.P64s.v : L.P.v; }
+    static const BsrView<double>& R(Level& L) { return L.r_sell[kPrec] && L.R64s.vals ? L.R64s.v : L.R.v; }
+    static const BsrView<double>* Psell(Level& L) { return L.P64s.vals ? &L.P64s.v : nullptr; }
+    static const BsrView<double>* Rsell(Level& L) { return L.R64s.vals ? &L.R64s.v : nullptr; }
     static const BsrView<double>& Pcsr(Level& L) { return L.P.v; }
     static const BsrView<double>& Rcsr(Level& L) { return L.R.v; }
     static const double* dinv(Level& L) { return L.dinv; }
@@ -641,10 +665,12 @@ template <> struct LevelVecs<float> {
         if (L.prod_slot[kPrec] && L.A32s.vals) return L.A32s.v;
         return L.A32p.vals ? L.A32p.v : L.A32.v;
     }
-    // transfers: the jagged view when setup kept it, else CSR (padded rows of P cost what the saved
+    // transfers: the sliced view when setup kept it, else CSR (padded rows of P cost what the saved
     // row-pointer load gains: its rows hold 1 to 7 blocks)
-    static const BsrView<float>& P(Level& L) { return L.p_jds[kPrec] && L.P32j.vals ? L.P32j.v : L.P32.v; }
-    static const BsrView<float>& R(Level& L) { return L.r_jds[kPrec] && L.R32j.vals ? L.R32j.v : L.R32.v; }
+    static const BsrView<float>& P(Level& L) { return L.p_sell[kPrec] && L.P32s.vals ? L.P32s.v : L.P32.v; }
+    static const BsrView<float>& R(Level& L) { return L.r_sell[kPrec] && L.R32s.vals ? L.R32s.v : L.R32.v; }
+    static const BsrView<float>* Psell(Level& L) { return L.P32s.vals ? &L.P32s.v : nullptr; }
+    static const BsrView<float>* Rsell(Level& L) { return L.R32s.vals ? &L.R32s.v : nullptr; }
     static const BsrView<float>& Pcsr(Level& L) { return L.P32.v; }
     static const BsrView<float>& Rcsr(Level& L) { return L.R32.v; }
     static const float* dinv(Level& L) { return L.dinv32; }
@@ -670,8 +696,10 @@ template <> struct LevelVecs<dfl> {
         if (L.prod_slot[kPrec] && L.A2s.vals) return L.A2s.v;
         return L.A2p.vals ? L.A2p.v : L.A2.v;
     }
-    static const BsrView<dfl>& P(Level& L) { return L.p_jds[kPrec] && L.P2j.vals ? L.P2j.v : L.P2.v; }
-    static const BsrView<dfl>& R(Level& L) { return L.r_jds[kPrec] && L.R2j.vals ? L.R2j.v : L.R2.v; }
+    static const BsrView<dfl>& P(Level& L) { return L.p_sell[kPrec] && L.P2s.vals ? L.P2s.v : L.P2.v; }
+    static const BsrView<dfl>& R(Level& L) { return L.r_sell[kPrec] && L.R2s.vals ? L.R2s.v : L.R2.v; }
+    static const BsrView<dfl>* Psell(Level& L) { return L.P2s.vals ? &L.P2s.v : nullptr; }
+    static const BsrView<dfl>* Rsell(Level& L) { return L.R2s.vals ? &L.R2s.v : nullptr; }
     static const BsrView<dfl>& Pcsr(Level& L) { return L.P2.v; }
     static const BsrView<dfl>& Rcsr(Level& L) { return L.R2.v; }
     static const dfl* dinv(Level& L) { return L.dinv2; }
@@ -1041,7 +1069,7 @@ void release_bsr(fhg_ctx* ctx, DevBsr<T>& D)
     if (D.owns_index) {
         dfree(ctx, D.rowptr);
         dfree(ctx, D.colidx);
-        dfree(ctx, D.jds_start);
+        dfree(ctx, D.slices);
     }
     D = DevBsr<T>();
 }
@@ -1058,10 +1086,12 @@ void release_unused_views(fhg_ctx* ctx)
         else if (L.G2s.vals) release_bsr(ctx, L.G2s);
         if (L.A2s.vals && L.prod_slot[FHG_PREC_DF]) release_bsr(ctx, L.A2p);
         else if (L.A2s.vals) release_bsr(ctx, L.A2s);
-        if (L.P32j.vals && !L.p_jds[FHG_PREC_FP32]) release_bsr(ctx, L.P32j);
-        if (L.R32j.vals && !L.r_jds[FHG_PREC_FP32]) release_bsr(ctx, L.R32j);
-        if (L.P2j.vals && !L.p_jds[FHG_PREC_DF]) release_bsr(ctx, L.P2j);
-        if (L.R2j.vals && !L.r_jds[FHG_PREC_DF]) release_bsr(ctx, L.R2j);
+        if (L.P64s.vals && !L.p_sell[FHG_PREC_FP64]) release_bsr(ctx, L.P64s);
+        if (L.R64s.vals && !L.r_sell[FHG_PREC_FP64]) release_bsr(ctx, L.R64s);
+        if (L.P32s.vals && !L.p_sell[FHG_PREC_FP32]) release_bsr(ctx, L.P32s);
+        if (L.R32s.vals && !L.r_sell[FHG_PREC_FP32]) release_bsr(ctx, L.R32s);
+        if (L.P2s.vals && !L.p_sell[FHG_PREC_DF]) release_bsr(ctx, L.P2s);
+        if (L.R2s.vals && !L.r_sell[FHG_PREC_DF]) release_bsr(ctx, L.R2s);
     }
     Level& L0 = ctx->levels[0];
     if (L0.Ahat2s.vals && L0.outer_slot && L0.ahat_lo) {
@@ -1449,7 +1479,7 @@ struct TuneKey {
 struct TuneShapes {
     int a_lanes, a_unroll, gs_lanes, gs_unroll, p_lanes, p_unroll, r_lanes, r_unroll;
     bool prod_slot, gs_slot;
-    bool p_jds = false, r_jds = false;
+    bool p_sell = false, r_sell = false;
 };
 std::mutex g_tune_mutex;
 std::map<TuneKey, TuneShapes> g_tune_cache;
@@ -1493,8 +1523,8 @@ int tune_level(fhg_ctx* ctx, int l)
                 BsrView<T>& R = const_cast<BsrView<T>&>(V::Rcsr(L));
                 P.lanes = t.p_lanes; P.unroll = t.p_unroll;
                 R.lanes = t.r_lanes; R.unroll = t.r_unroll;
-                L.p_jds[PR] = t.p_jds;
-                L.r_jds[PR] = t.r_jds;
+                L.p_sell[PR] = t.p_sell;
+                L.r_sell[PR] = t.r_sell;
             }
             return FHG_OK;
         }
@@ -1511,8 +1541,8 @@ int tune_level(fhg_ctx* ctx, int l)
     if (!coarsest) {
         t.p_lanes = V::Pcsr(L).lanes; t.p_unroll = V::Pcsr(L).unroll;
         t.r_lanes = V::Rcsr(L).lanes; t.r_unroll = V::Rcsr(L).unroll;
-        t.p_jds = L.p_jds[PR];
-        t.r_jds = L.r_jds[PR];
+        t.p_sell = L.p_sell[PR];
+        t.r_sell = L.r_sell[PR];
     }
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     g_tune_cache[key] = t;
@@ -1592,10 +1622,10 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
         if (L.inject) return FHG_OK;   // the natural injection has no launch shape
         BsrView<T>& P = const_cast<BsrView<T>&>(V::Pcsr(L));
         BsrView<T>& R = const_cast<BsrView<T>&>(V::Rcsr(L));
-        const bool forced_jds = ctx->opts.gs_layout == FHG_GS_SLOT;   // the jagged views, not compared
-        const bool pj0 = L.p_jds[V::kPrec], rj0 = L.r_jds[V::kPrec];
-        L.p_jds[V::kPrec] = false;
-        L.r_jds[V::kPrec] = false;
+        const bool forced_sell = ctx->opts.gs_layout == FHG_GS_SLOT;   // the sliced views, not compared
+        const bool pj0 = L.p_sell[V::kPrec], rj0 = L.r_sell[V::kPrec];
+        L.p_sell[V::kPrec] = false;
+        L.r_sell[V::kPrec] = false;
         CK(cudaMemsetAsync(V::x(C), 0, sizeof(T) * C.n, s));
         float p_ms = 0.f, r_ms = 0.f;
         if ((rc = tune(ctx, bs, P.lanes, P.unroll, [&](int G, int U) {
@@ -1608,30 +1638,23 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
                  fhg::launch_spmv<T>(v, fhg::kSpmvAssign, V::r(L), nullptr, V::b(C), s);
              }, &r_ms)))
             return rc;
-        // the jagged views against the best CSR shapes
-        if (forced_jds) {
-            L.p_jds[V::kPrec] = pj0;
-            L.r_jds[V::kPrec] = rj0;
-        } else if constexpr (!std::is_same<T, double>::value) {
-            const BsrView<T>* pj = nullptr;
-            const BsrView<T>* rj = nullptr;
-            if constexpr (std::is_same<T, float>::value) {
-                if (L.P32j.vals) pj = &L.P32j.v;
-                if (L.R32j.vals) rj = &L.R32j.v;
-            } else {
-                if (L.P2j.vals) pj = &L.P2j.v;
-                if (L.R2j.vals) rj = &L.R2j.v;
-            }
+        // the sliced views against the best CSR shapes
+        if (forced_sell) {
+            L.p_sell[V::kPrec] = pj0;
+            L.r_sell[V::kPrec] = rj0;
+        } else {
+            const BsrView<T>* pj = V::Psell(L);
+            const BsrView<T>* rj = V::Rsell(L);
             float ms = 0.f;
             if (pj) {
                 if ((rc = time_candidate(ctx, [&]() { fhg::launch_spmv<T>(*pj, fhg::kSpmvAddTo, V::x(C), V::r(L), V::r(L), s); }, &ms)))
                     return rc;
-                L.p_jds[V::kPrec] = ms < p_ms;
+                L.p_sell[V::kPrec] = ms < p_ms;
             }
             if (rj) {
                 if ((rc = time_candidate(ctx, [&]() { fhg::launch_spmv<T>(*rj, fhg::kSpmvAssign, V::r(L), nullptr, V::b(C), s); }, &ms)))
                     return rc;
-                L.r_jds[V::kPrec] = ms < r_ms;
+                L.r_sell[V::kPrec] = ms < r_ms;
             }
         }
     }
@@ -1663,6 +1686,8 @@ void reset_device_state(Level& L)
     L.A32p = DevBsr<float>();
     L.G32s = DevBsr<float>();
     L.A32s = DevBsr<float>();
+    L.P64s = DevBsr<double>();
+    L.R64s = DevBsr<double>();
     L.C64 = DevBsr<double>();
     L.Co64 = DevBsr<double>();
     L.C32 = DevBsr<float>();
@@ -1675,11 +1700,11 @@ void reset_device_state(Level& L)
     L.A2p = DevBsr<dfl>();
     L.G2s = DevBsr<dfl>();
     L.A2s = DevBsr<dfl>();
-    L.P32j = DevBsr<float>();
-    L.R32j = DevBsr<float>();
-    L.P2j = DevBsr<dfl>();
-    L.R2j = DevBsr<dfl>();
-    for (int i = 0; i < 3; i++) { L.p_jds[i] = false; L.r_jds[i] = false; }
+    L.P32s = DevBsr<float>();
+    L.R32s = DevBsr<float>();
+    L.P2s = DevBsr<dfl>();
+    L.R2s = DevBsr<dfl>();
+    for (int i = 0; i < 3; i++) { L.p_sell[i] = false; L.r_sell[i] = false; }
     L.dinv2 = nullptr;
     L.x2 = L.b2 = L.r2 = nullptr;
     for (int i = 0; i < 3; i++) { L.gs_slot[i] = false; L.prod_slot[i] = false; L.gs_lanes[i] = 0; L.gs_unroll[i] = 1; }
@@ -2221,18 +2246,20 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                     if ((rc = upload_bsr<dfl>(ctx, Pp, L.P2, &L.P))) return rc;
                     if ((rc = upload_bsr<dfl>(ctx, Rp, L.R2, &L.R))) return rc;
                 }
-                // the jagged transfer views of the two largest levels: compared by the autotuner, or used
-                // with FHG_GS_SLOT
-                const bool want_jds = o.gs_layout == FHG_GS_SLOT || (o.gs_layout == FHG_GS_AUTO && o.autotune);
-                if (want_jds && l <= 1) {
-                    if (fp32 && ((rc = upload_jds(ctx, Pp, L.P32j)) || (rc = upload_jds(ctx, Rp, L.R32j)))) return rc;
-                    if (pair && ((rc = upload_jds(ctx, Pp, L.P2j)) || (rc = upload_jds(ctx, Rp, L.R2j)))) return rc;
-                    if (o.gs_layout == FHG_GS_SLOT)
-                        for (int q : {FHG_PREC_FP32, FHG_PREC_DF}) {
-                            L.p_jds[q] = true;
-                            L.r_jds[q] = true;
-                        }
-                }
+                // Sliced views: where the rows fill the GPU (compared with CSR by the autotuner), or on levels 0
+                // and 1 with FHG_GS_SLOT (P with a thread per row, which adds; FP32 and pairs).
+                const bool slot = o.gs_layout == FHG_GS_SLOT;
+                auto sliced = [&](const HostBsr& M, bool prolongation, bool* use, auto& d64, auto& d32, auto& d2) -> int {
+                    const int lanes = slot ? (l <= 1 ? 1 : 0) : o.gs_layout == FHG_GS_ROW ? 0 : sell_lanes(M, prolongation);
+                    if (lanes == 0) return FHG_OK;
+                    if (o.vcycle_precision == FHG_PREC_FP64 && !slot && (rc = upload_sell(ctx, M, lanes, d64))) return rc;
+                    if (fp32 && (rc = upload_sell(ctx, M, lanes, d32))) return rc;
+                    if (pair && (rc = upload_sell(ctx, M, lanes, d2))) return rc;
+                    for (int q = 0; q < 3; q++) use[q] = true;
+                    return FHG_OK;
+                };
+                if ((rc = sliced(Pp, true, L.p_sell, L.P64s, L.P32s, L.P2s)) || (rc = sliced(Rp, false, L.r_sell, L.R64s, L.R32s, L.R2s)))
+                    return rc;
             }
         }
         if (l == 0 && fp32 && nlevels > 1 && fhg::learned_supports(L.bs)) {

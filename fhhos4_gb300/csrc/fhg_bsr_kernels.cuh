@@ -273,71 +273,66 @@ __global__ void __launch_bounds__(kThreads) k_bsr_spmv(int nbr, const int* __res
     }
 }
 
-// y = M x | y = y + M x on the jagged view (rows sorted by decreasing block count, slot s of sorted
-// row k at start[s] + k): one thread per row, every slot's load of a warp is 32 consecutive blocks with
-// no padding, the sorted order ends a row's walk at its own length. The output row is scattered by
-// the permutation (the vectors of one level stay in L2). The row's blocks are summed in column order.
-constexpr int kMaxJdsSlots = 64;
-
-template <class T, int BS, int MODE>
-__global__ void __launch_bounds__(kThreads) k_bsr_spmv_jds(int nbr, int nslots, const int* __restrict__ perm,
-                                                           const int* __restrict__ start,
-                                                           const int* __restrict__ colidx,
-                                                           const T* __restrict__ vals, long long ld,
-                                                           const T* __restrict__ x, const T* aux, T* y)
+// y = M x | y = y + M x on the sliced view: L lanes per row (1 for the short rows of P; 4 or 8 for those of
+// R, 25 to 50 blocks, of which there are too few for a thread each), a warp per slice of 32 / L rows, so every
+// load of the slice's columns and values is 32 consecutive words, with no padding but what the longest row of
+// a slice adds (a few percent, the rows being sorted by length in windows of kSellWindow; the windows keep a
+// slice's output rows within a few cache lines of each other). Few lanes: in FP64 a lane group's shuffle
+// adds cost the pipe as much as its products. The columns of the next kGroup blocks are loaded ahead of the
+// sums over the present ones. Against CSR rows of 8 (P) and 32 (R) lanes, or of the tuned lanes at 64^3: x += P e FP64
+// 32^3 124 -> 45 us, FP32 64^3 183 -> 125 us (0.9 of HBM), pairs 48^3 122 -> 96; R r FP64 32^3 118 -> 43,
+// FP32 64^3 148 -> 131, 32^3 23 -> 12, 24^3 k = 2 45 -> 30, pairs 48^3 113 -> 104.
+template <class T, int BS, int MODE, int L>
+__global__ void __launch_bounds__(kThreads) k_bsr_spmv_sell(int slices, const int* __restrict__ perm,
+                                                            const int* __restrict__ ptr,
+                                                            const int* __restrict__ colidx,
+                                                            const T* __restrict__ vals, long long ld,
+                                                            const T* __restrict__ x, const T* aux, T* y)
 {
-    // Slots go in groups of kJdsGroup with every load of a group issued before its sums (predicated on
-    // the row's length, the sorted order making the valid slots a prefix), so that a row's loads are in
-    // flight together instead of one slot's after the other's.
     constexpr int kBlockBytes = BS * BS * (int)sizeof(T);
-    constexpr int kJdsGroup = kBlockBytes <= 36 ? 4 : kBlockBytes <= 72 ? 2 : 1;   // registers: ~144 values
-    pdl_wait();
-    __shared__ int sh_start[kMaxJdsSlots + kJdsGroup + 1];
-    for (int i = threadIdx.x; i <= nslots + kJdsGroup; i += blockDim.x) sh_start[i] = start[i < nslots ? i : nslots];
-    __syncthreads();
-    const int k = (int)(blockIdx.x * kThreads + threadIdx.x);
-    if (k >= nbr) return;
-    const long long row = perm[k];
-    T av[BS];
-    if (MODE != kSpmvAssign)
+    constexpr int kGroup = kBlockBytes <= 36 ? 4 : kBlockBytes <= 72 ? 2 : 1;   // blocks in flight: ~144 bytes
+    const int slice = (int)((blockIdx.x * kThreads + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (slice >= slices) return;   // whole warps
+    const int row = perm[slice * (32 / L) + lane / L];
+    int p = ptr[slice] + lane;
+    const int p1 = ptr[slice + 1];
+    int col[kGroup];
 #pragma unroll
-        for (int r = 0; r < BS; r++) av[r] = aux[row * BS + r];
+    for (int g = 0; g < kGroup; g++) col[g] = p + 32 * g < p1 ? colidx[p + 32 * g] : -1;
+    pdl_wait();
     T acc[BS];
 #pragma unroll
-    for (int r = 0; r < BS; r++) acc[r] = T(0);
-    for (int s0 = 0; s0 < nslots; s0 += kJdsGroup) {
-        if (sh_start[s0] + k >= sh_start[s0 + 1]) break;   // the row has no slot s0
-        int col[kJdsGroup];
-        bool ok[kJdsGroup];
+    for (int r = 0; r < BS; r++) acc[r] = MODE == kSpmvAssign || row < 0 ? T(0) : aux[(long long)row * BS + r];
+    while (p < p1) {   // the same number of steps in every lane
+        T xv[kGroup][BS], v[kGroup][BS * BS];
 #pragma unroll
-        for (int g = 0; g < kJdsGroup; g++) {
-            const int p = sh_start[s0 + g] + k;
-            ok[g] = s0 + g < nslots && p < sh_start[s0 + g + 1];
-            col[g] = ok[g] ? colidx[p] : 0;
+        for (int g = 0; g < kGroup; g++) {
+#pragma unroll
+            for (int c = 0; c < BS; c++) xv[g][c] = col[g] >= 0 ? x[(long long)col[g] * BS + c] : T(0);
+#pragma unroll
+            for (int e = 0; e < BS * BS; e++) v[g][e] = col[g] >= 0 ? vals[(long long)e * ld + p + 32 * g] : T(0);
         }
-        T xv[kJdsGroup][BS], av2[kJdsGroup][BS * BS];
+        p += 32 * kGroup;
 #pragma unroll
-        for (int g = 0; g < kJdsGroup; g++) {
-            const long long p = (long long)sh_start[s0 + g] + k;
+        for (int g = 0; g < kGroup; g++) {
+            const int next = p + 32 * g < p1 ? colidx[p + 32 * g] : -1;
+            if (col[g] >= 0) {
 #pragma unroll
-            for (int c = 0; c < BS; c++) xv[g][c] = ok[g] ? x[(long long)col[g] * BS + c] : T(0);
+                for (int r = 0; r < BS; r++)
 #pragma unroll
-            for (int e = 0; e < BS * BS; e++) av2[g][e] = ok[g] ? vals[(long long)e * ld + p] : T(0);
-        }
-#pragma unroll
-        for (int g = 0; g < kJdsGroup; g++) {
-            if (!ok[g]) continue;
-#pragma unroll
-            for (int r = 0; r < BS; r++)
-#pragma unroll
-                for (int c = 0; c < BS; c++) acc[r] = fma(av2[g][r * BS + c], xv[g][c], acc[r]);
+                    for (int c = 0; c < BS; c++) acc[r] = fma(v[g][r * BS + c], xv[g][c], acc[r]);
+            }
+            col[g] = next;
         }
     }
+    if (L > 1) {
 #pragma unroll
-    for (int r = 0; r < BS; r++) {
-        if (MODE == kSpmvAssign) y[row * BS + r] = fin(acc[r]);
-        else y[row * BS + r] = av[r] + acc[r];
+        for (int r = 0; r < BS; r++) acc[r] = group_sum<L>(acc[r]);
     }
+    if (row < 0) return;
+#pragma unroll
+    for (int r = 0; r < BS; r++)
+        if (L == 1 || r % L == lane % L) y[(long long)row * BS + r] = fin(acc[r]);
 }
 
 // w = D^-1 (b - A x) (block-Jacobi-scaled residual, the learned step's input): the residual of a
@@ -1070,6 +1065,20 @@ void spmv_slot_w(const BsrView<T>& A, unsigned grid, int mode, const T* x, const
     default: break;                                                        \
     }
 
+template <class T, int BS>
+void sell_bs(const BsrView<T>& A, int mode, const T* x, const T* aux, T* y, cudaStream_t s)
+{
+    const int rows = 32 / A.sell_lanes, slices = (A.nbr + rows - 1) / rows;
+    const unsigned grid = grid_for(32LL * slices, kThreads);
+    auto go = [&](auto kernel) {
+        pdl_launch(kernel, grid, kThreads, 0, s, slices, A.sell_perm, A.sell_ptr, A.colidx, A.vals, A.ld, x, aux, y);
+    };
+    if (A.sell_lanes == 8) go(k_bsr_spmv_sell<T, BS, kSpmvAssign, 8>);
+    else if (A.sell_lanes == 4) go(k_bsr_spmv_sell<T, BS, kSpmvAssign, 4>);
+    else if (mode == kSpmvAssign) go(k_bsr_spmv_sell<T, BS, kSpmvAssign, 1>);
+    else go(k_bsr_spmv_sell<T, BS, kSpmvAddTo, 1>);
+}
+
 template <class T>
 void launch_spmv(const BsrView<T>& A, int mode, const T* x, const T* aux, T* y, cudaStream_t s)
 {
@@ -1087,26 +1096,16 @@ void launch_spmv(const BsrView<T>& A, int mode, const T* x, const T* aux, T* y, 
         g_kernel_launches++;
         return;
     }
-    if (A.jds_perm) {
-        // jagged views exist only for the transfers (assign, add-to) with at most kMaxJdsSlots blocks
-        // a row (setup builds no other); they have no row pointers to fall back on
-        if ((mode != kSpmvAssign && mode != kSpmvAddTo) || A.jds_slots > kMaxJdsSlots) return;
-        const unsigned grid = grid_for(A.nbr, kThreads);
-#define FHG_JDS_LAUNCH(BSV)                                                                                     \
-        if (mode == kSpmvAssign)                                                                                 \
-            pdl_launch(k_bsr_spmv_jds<T, BSV, kSpmvAssign>, grid, kThreads, 0, s, A.nbr, A.jds_slots, A.jds_perm, \
-                       A.jds_start, A.colidx, A.vals, A.ld, x, aux, y);                                          \
-        else                                                                                                     \
-            pdl_launch(k_bsr_spmv_jds<T, BSV, kSpmvAddTo>, grid, kThreads, 0, s, A.nbr, A.jds_slots, A.jds_perm,  \
-                       A.jds_start, A.colidx, A.vals, A.ld, x, aux, y);
+    if (A.sell_perm) {
+        // sliced views exist only for the transfers; they have no row pointers to fall back on
+        if (mode != kSpmvAssign && (mode != kSpmvAddTo || A.sell_lanes != 1)) return;
         switch (A.bs) {
-        case 2: FHG_JDS_LAUNCH(2) break;
-        case 3: FHG_JDS_LAUNCH(3) break;
-        case 4: FHG_JDS_LAUNCH(4) break;
-        case 6: FHG_JDS_LAUNCH(6) break;
+        case 2: sell_bs<T, 2>(A, mode, x, aux, y, s); break;
+        case 3: sell_bs<T, 3>(A, mode, x, aux, y, s); break;
+        case 4: sell_bs<T, 4>(A, mode, x, aux, y, s); break;
+        case 6: sell_bs<T, 6>(A, mode, x, aux, y, s); break;
         default: break;
         }
-#undef FHG_JDS_LAUNCH
         g_kernel_launches++;
         return;
     }

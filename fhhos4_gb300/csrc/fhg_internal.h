@@ -32,12 +32,13 @@ struct BsrView {
     const int* rowptr = nullptr;
     const int* colidx = nullptr;
     const T* vals = nullptr;
-    // Jagged view (JDS, the transfer operators): rows sorted by decreasing block count, row
-    // jds_perm[k] in sorted place k, its slot s at jds_start[s] + k (jds_start[s + 1] - jds_start[s]
-    // rows have more than s blocks); no padding, rowptr unused; products only (assign, add-to).
-    const int* jds_perm = nullptr;
-    const int* jds_start = nullptr;
-    int jds_slots = 0;
+    // Sliced view (the transfer operators): the rows sorted by decreasing block count within windows, then
+    // cut into slices of 32 / sell_lanes; lane t of slice q holds every sell_lanes-th block of row
+    // sell_perm[q * (32 / sell_lanes) + t / sell_lanes] (-1: none), its blocks at sell_ptr[q] + t, + 32, ...;
+    // empty places have column -1; rowptr unused; products only (assign; add-to with one lane).
+    int sell_lanes = 1;
+    const int* sell_perm = nullptr;
+    const int* sell_ptr = nullptr;
     // Row-class view (operators whose rows repeat): cls[i] is the class of row i, vals the dictionary of
     // the classes, entry e of class c at e * ld + c: the ell off-diagonal blocks in column order, D^-1, the
     // diagonal block; the off-diagonal columns of row i at s * nbr + i (the row itself in an empty slot);

@@ -105,7 +105,7 @@ class Multigrid(IterativeSolver):
         # smoothing steps on levels >= 1; -1: PreSmoothingIterations / PostSmoothingIterations
         self.CoarsePreSmoothingIterations = -1
         self.CoarsePostSmoothingIterations = -1
-        self.GsLayout = "auto"   # FP32 GS sweeps: "auto", "row" or "slot" (padded rows)
+        self.GsLayout = "auto"   # storage of sweeps and products: "auto", "row" or "slot" (padded rows)
         # further V-cycle precisions whose operator copies setup builds, to switch to later
         self.ExtraPrecisions: List[str] = []
         self._As: List[sp.csr_matrix] = []

@@ -118,12 +118,13 @@ typedef struct {
                                    default): pre_iterations, as the reference (one count for every level).
                                    No counterpart in the reference. */
     int coarse_post_iterations; /* the same after it; -1: post_iterations */
-    int gs_layout;              /* FP32 GS sweeps: FHG_GS_AUTO (the autotuner picks row- or slot-major padded
-                                   rows; row-major without autotuning), FHG_GS_ROW, FHG_GS_SLOT. Same
-                                   arithmetic, different storage order and launch shape; FHG_GS_SLOT also
-                                   makes the products with A use the slot-major view of all of A, and
-                                   the transfers of levels 0 and 1 their jagged views (rows sorted by
-                                   block count, one thread per row); the autotuner compares those too. */
+    int gs_layout;              /* Storage of the sweeps, products and transfers. FHG_GS_AUTO: row classes where
+                                   the rows of A repeat, else (FP32 and DF) row- or slot-major padded rows (the
+                                   autotuner picks; row-major without autotuning); the transfers in slices of
+                                   rows sorted by block count where their rows fill the GPU (the autotuner
+                                   compares them with CSR). FHG_GS_ROW: row-major padded rows, CSR transfers.
+                                   FHG_GS_SLOT: slot-major padded rows, the transfers of levels 0 and 1 sliced.
+                                   Same arithmetic, different storage order and launch shape. */
     int extra_precisions;       /* bit mask (1 << FHG_PREC_FP32, 1 << FHG_PREC_DF) of V-cycle precisions whose
                                    operator copies setup also builds, besides vcycle_precision's, so that
                                    fhg_set_vcycle_precision can switch to them (FP64 copies are always built) */

@@ -1,0 +1,60 @@
+"""Transfers on the sliced views (rows sorted by length in windows, slices of 32 rows or of 8 or 4 rows with
+several lanes each) against the scalar CSR products, in every value type and block size, where rows fill
+the GPU (P from 32,768 rows, R from 4,096 and 16,384): odd row counts, a last slice that is not full, rows of
+one to fifty blocks."""
+import numpy as np
+import pytest
+
+from fhhos4_gb300 import hho
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-14, "df": 1e-13, "fp32": 2e-6}   # of the largest |R||r| or |x| + |P||e|
+
+
+@pytest.mark.parametrize("precision", ["fp64", "df", "fp32"])
+@pytest.mark.parametrize("dim,n,k", [(2, 112, 1), (2, 112, 2), (2, 106, 3), (3, 16, 1), (3, 16, 2), (3, 28, 1)])
+def test_gpu_transfers_on_sliced_views(dim, n, k, precision):
+    torch = pytest.importorskip("torch")
+    from fhhos4_gb300 import _native as N
+    from fhhos4_gb300 import solver as S
+    from test_gpu_parity import scalar_perm
+    H = hho.Hierarchy(dim, n, k, max_levels=2)
+    A, P, bs = H.A(0), H.P(0), H.block_size
+    H.close()
+    # a coarse operator of the right size that is cheap to invert: the transfers do not see it
+    rng = np.random.default_rng(2)
+    import scipy.sparse as sp
+    top = P.shape[1]
+    As, Ps = [A, sp.identity(top, format="csr") + sp.csr_matrix((top, top))], [P]
+    # the dense limit of the coarsest level keeps large ones out: a third level of one block row
+    nb = top // bs
+    Q = sp.csr_matrix((np.ones(top), (np.arange(top), np.tile(np.arange(bs), nb))), shape=(top, bs))
+    As.append(sp.identity(bs, format="csr"))
+    Ps.append(Q)
+    ctx = S.fcg_mg(As, Ps, bs, precision=precision, fused=False).Context()
+    p0 = scalar_perm(ctx.permutation(0, A.shape[0] // bs), bs)
+    p1 = scalar_perm(ctx.permutation(1, nb), bs)
+    Pp = P.tocsr()[p0][:, p1]
+
+    def put(v):
+        if precision == "df":
+            hi = v.astype(np.float32)
+            return torch.tensor(np.stack([hi, (v - hi).astype(np.float32)], 1), device="cuda")
+        return torch.tensor(v, dtype=torch.float64 if precision == "fp64" else torch.float32, device="cuda")
+
+    def get(t):
+        a = t.cpu().numpy().astype(np.float64)
+        return a[:, 0] + a[:, 1] if precision == "df" else a
+
+    rd, ed = put(rng.standard_normal(A.shape[0])), put(rng.standard_normal(top))
+    r, e = get(rd), get(ed)
+    out = torch.full_like(ed, float("nan"))
+    ctx.apply_internal(0, N.OP_RESTRICT, precision, rd.data_ptr(), None, out.data_ptr())
+    scale = (abs(Pp).T @ np.abs(r)).max()
+    assert np.abs(get(out) - Pp.T @ r).max() <= TOL[precision] * scale
+    out = torch.full_like(rd, float("nan"))
+    ctx.apply_internal(0, N.OP_PROLONG_ADD, precision, ed.data_ptr(), rd.data_ptr(), out.data_ptr())
+    scale = np.abs(r).max() + (abs(Pp) @ np.abs(e)).max()
+    assert np.abs(get(out) - (r + Pp @ e)).max() <= TOL[precision] * scale
+    ctx.close()
