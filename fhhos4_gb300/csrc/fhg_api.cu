@@ -521,15 +521,17 @@ int upload_classes(fhg_ctx* ctx, const HostBsr& B, const RowClasses& C, const st
 // streamed operator) and at most kMaxClasses (its FP32 form, 258 KB at 3 x 3 blocks and 6 neighbours, stays
 // in L1 and L2). The operators of a 64^3 mesh with one tensor have 77 classes, of a 4 x 4 x 4
 // checkerboard about 200; one tensor per 4^3 cubes makes 25 to 30 rows to a class, which stay with the
-// stored-block views.
-constexpr int kClassRows = 64, kMaxClasses = 1024;
+// stored-block views. Levels of at most kClassSmall rows take the view however few rows a class has: their
+// launches are bound by latency, and the lanes of the class kernels have the shortest chains (24^3 k = 2 FP32,
+// 2,376 rows: a sweep 16.8 us on padded rows).
+constexpr int kClassRows = 64, kMaxClasses = 1024, kClassSmall = 8192;
 
 // Row-class views of B in FP64, FP32 (d32, nullable) and pairs; inv: the inverted diagonal blocks or null.
 int build_class_views(fhg_ctx* ctx, const HostBsr& B, const double* inv, DevBsr<double>& d64, DevBsr<float>* d32,
                       DevBsr<dfl>& d2)
 {
     RowClasses C;
-    if (!row_classes(B, kMaxClasses, kClassRows, C)) return FHG_OK;
+    if (!row_classes(B, kMaxClasses, B.nbr <= kClassSmall ? 1 : kClassRows, C)) return FHG_OK;
     std::vector<double> dict;
     class_dictionary(B, C, inv, dict);
     unsigned short* cls = nullptr;

@@ -805,6 +805,89 @@ __global__ void __launch_bounds__(kClsThreads, kClsBlocks<T, BS, W>)
     for (int r = 0; r < BS; r++) y[(long long)row * BS + r] = MODE == kSpmvAssign ? fin(acc[r]) : av[r] - acc[r];
 }
 
+// The same with one output per lane (BS lanes a row, 32 / BS rows a warp), for launches whose rows leave the
+// GPU's 608 schedulers a warp or less each: a thread per row is then one long chain (63 multiply-adds
+// with 3 x 3 blocks: 64 cycles each in FP64, 13 instructions in pairs), here a BS-th of it. The neighbours' x
+// entries are loaded by every lane of the row (one request); t = b - A x goes round by shuffles for D^-1.
+__device__ __forceinline__ float lane_value(float v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+__device__ __forceinline__ double lane_value(double v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+__device__ __forceinline__ dfl lane_value(dfl v, int lane)
+{
+    return dfl(__shfl_sync(0xffffffffu, v.h, lane), __shfl_sync(0xffffffffu, v.l, lane));
+}
+
+template <class T, int BS, int W>
+struct ClassLane {
+    static constexpr int kRows = 32 / BS;   // rows of a warp
+    int row, r, first;                      // row, output, first lane of the row
+    bool in;
+    int col[W];
+    const T* d;   // dictionary entry (0, r, 0) of the row's class
+
+    __device__ __forceinline__ ClassLane(int row0, int row1, int nbr, const unsigned short* __restrict__ cls,
+                                         const int* __restrict__ colidx, const T* __restrict__ dict, int ld)
+    {
+        const int lane = threadIdx.x & 31, q = lane / BS;
+        row = row0 + (int)((blockIdx.x * kClsThreads + threadIdx.x) >> 5) * kRows + q;
+        r = lane - q * BS;
+        first = q * BS;
+        in = q < kRows && row < row1;
+        d = dict + (in ? cls[row] : 0) + r * BS * ld;
+#pragma unroll
+        for (int s = 0; s < W; s++) col[s] = in ? colidx[(long long)s * nbr + row] : row;
+    }
+    // Output r of block `slot` times w.
+    __device__ __forceinline__ T block(int ld, int slot, const T (&w)[BS], T acc) const
+    {
+#pragma unroll
+        for (int c = 0; c < BS; c++) acc = fma(d[(slot * BS * BS + c) * ld], w[c], acc);
+        return acc;
+    }
+};
+
+template <class T, int BS, int W, bool ZERO>
+__global__ void __launch_bounds__(kClsThreads, kClsBlocks<T, BS, W>)
+    k_bsr_gs_cls_lanes(int row0, int row1, int nbr, const unsigned short* __restrict__ cls, const int* __restrict__ colidx,
+                       const T* __restrict__ dict, int ld, const T* __restrict__ b, T* x, int col_lo, int col_hi, T omega)
+{
+    const ClassLane<T, BS, W> L(row0, row1, nbr, cls, colidx, dict, ld);
+    pdl_wait();
+    const long long i = (long long)L.row * BS + L.r;
+    T xv[W][BS], t[BS], acc = T(0);
+    gather_slots<T, BS, W, ZERO>(L.col, L.row, col_lo, col_hi, x, xv);
+    const T bv = L.in ? b[i] : T(0);
+    if (L.in)
+#pragma unroll
+        for (int s = 0; s < W; s++) acc = L.block(ld, s, xv[s], acc);
+    acc = bv - acc;
+#pragma unroll
+    for (int c = 0; c < BS; c++) t[c] = lane_value(acc, L.first + c);
+    if (!L.in) return;
+    T v = L.block(ld, W, t, T(0));
+    if (omega != T(1)) v = fma(omega, v, (T(1) - omega) * x[i]);   // block SOR
+    x[i] = fin(v);
+}
+
+template <class T, int BS, int W, int MODE>
+__global__ void __launch_bounds__(kClsThreads, kClsBlocks<T, BS, W>)
+    k_bsr_spmv_cls_lanes(int nbr, const unsigned short* __restrict__ cls, const int* __restrict__ colidx,
+                         const T* __restrict__ dict, int ld, const T* __restrict__ x, const T* aux, T* y)
+{
+    const ClassLane<T, BS, W> L(0, nbr, nbr, cls, colidx, dict, ld);
+    pdl_wait();
+    if (!L.in) return;
+    const long long i = (long long)L.row * BS + L.r;
+    T xv[W][BS], xd[BS], acc = T(0);
+    gather_slots<T, BS, W, false>(L.col, L.row, 0, 0, x, xv);
+#pragma unroll
+    for (int c = 0; c < BS; c++) xd[c] = x[(long long)L.row * BS + c];
+    const T av = MODE == kSpmvAssign ? T(0) : aux[i];
+#pragma unroll
+    for (int s = 0; s < W; s++) acc = L.block(ld, s, xv[s], acc);
+    acc = L.block(ld, W + 1, xd, acc);
+    y[i] = MODE == kSpmvAssign ? fin(acc) : av - acc;
+}
+
 // Block Jacobi: xnew_i = D_i^{-1} (omega b_i + (1-omega) D_i xold_i - omega sum_{j!=i} A_ij xold_j)
 template <class T, int BS, int G>
 __global__ void __launch_bounds__(kThreads) k_bsr_jacobi(int nbr, const int* __restrict__ rowptr,
@@ -1079,14 +1162,32 @@ void sell_bs(const BsrView<T>& A, int mode, const T* x, const T* aux, T* y, cuda
     else go(k_bsr_spmv_sell<T, BS, kSpmvAddTo, 1>);
 }
 
+// Rows up to which a launch on a row-class view takes one output per lane: 24,576 in FP64 and pairs, 12,288
+// in FP32 (a thread per row gives the 608 schedulers 1.3 and 0.6 warps each there). us a sweep, a thread per row against
+// a lane per output, at rows a colour: FP64 3 x 3 1,150: 20 / 14, 9,500: 22 / 18, 77,000: 61 / 70; pairs 3 x 3
+// 4,000: 15 / 11, 32,000: 19 / 19; pairs 6 x 6 9,500: 40 / 23; FP32 3 x 3 9,500: 10.2 / 9.4, 77,000: 15 / 20;
+// FP32 6 x 6 4,000: 22 / 12, 32,000: 30 / 32.
+template <class T>
+constexpr int kClsLaneRows = sizeof(T) == 4 ? 12288 : 24576;
+
+template <int BS>
+unsigned class_lanes_grid(int rows) { return grid_for(rows, kClsThreads / 32 * (32 / BS)); }
+
 template <class T>
 void launch_spmv(const BsrView<T>& A, int mode, const T* x, const T* aux, T* y, cudaStream_t s)
 {
     if (A.nbr == 0) return;
     if (A.cls) {   // operators only (assign, residual)
-        const unsigned grid = grid_for(A.nbr, kClsThreads);
+        const bool lanes = A.nbr <= kClsLaneRows<T>;
         FHG_DISPATCH_CLS(A.bs, A.ell, {
-            if (mode == kSpmvAssign)
+            const unsigned grid = lanes ? class_lanes_grid<BS>(A.nbr) : grid_for(A.nbr, kClsThreads);
+            if (lanes && mode == kSpmvAssign)
+                pdl_launch(k_bsr_spmv_cls_lanes<T, BS, W, kSpmvAssign>, grid, kClsThreads, 0, s, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, x, aux, y);
+            else if (lanes)
+                pdl_launch(k_bsr_spmv_cls_lanes<T, BS, W, kSpmvResidual>, grid, kClsThreads, 0, s, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, x, aux, y);
+            else if (mode == kSpmvAssign)
                 pdl_launch(k_bsr_spmv_cls<T, BS, W, kSpmvAssign, false>, grid, kClsThreads, 0, s, A.nbr, A.cls, A.colidx,
                            A.vals, (int)A.ld, x, aux, y);
             else
@@ -1211,9 +1312,17 @@ void launch_gs(const BsrView<T>& A, int row0, int row1, const T* dinv, long long
 {
     if (row1 <= row0) return;
     if (A.cls) {
-        const unsigned grid = grid_for((long long)(row1 - row0), kClsThreads);
+        const int rows = row1 - row0;
+        const bool lanes = rows <= kClsLaneRows<T>, zero = col_lo > 0 || col_hi < 0x7fffffff;
         FHG_DISPATCH_CLS(A.bs, A.ell, {
-            if (col_lo > 0 || col_hi < 0x7fffffff)
+            const unsigned grid = lanes ? class_lanes_grid<BS>(rows) : grid_for(rows, kClsThreads);
+            if (lanes && zero)
+                pdl_launch(k_bsr_gs_cls_lanes<T, BS, W, true>, grid, kClsThreads, 0, s, row0, row1, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, b, x, col_lo, col_hi, omega);
+            else if (lanes)
+                pdl_launch(k_bsr_gs_cls_lanes<T, BS, W, false>, grid, kClsThreads, 0, s, row0, row1, A.nbr, A.cls, A.colidx,
+                           A.vals, (int)A.ld, b, x, col_lo, col_hi, omega);
+            else if (zero)
                 pdl_launch(k_bsr_gs_cls<T, BS, W, true>, grid, kClsThreads, 0, s, row0, row1, A.nbr, A.cls, A.colidx,
                            A.vals, (int)A.ld, b, x, col_lo, col_hi, omega);
             else

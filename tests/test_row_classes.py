@@ -90,7 +90,9 @@ PREC = {"fp64": (np.float64, 1e-13), "df": (None, 1e-12), "fp32": (np.float32, 1
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", ["fp64", "df", "fp32"])
 @pytest.mark.parametrize("dim,n,k,omega", [(2, 36, 1, 1.0), (2, 36, 2, 1.0), (2, 36, 3, 1.3), (3, 8, 1, 1.0), (3, 8, 1, 1.3),
-                                           (3, 8, 2, 1.0)])
+                                           (3, 8, 2, 1.0),
+                                           # colours and levels with a thread per row (above one output per lane)
+                                           (2, 160, 1, 1.3), (3, 24, 1, 1.3)])
 def test_gpu_sweeps_and_products_on_class_views(dim, n, k, omega, precision):
     """Level-0 sweeps, SpMV and residual against the oracle in FP64 and colour order. Tolerance: a row
     of up to 42 products in FP64 (2^-53), pairs (2^-47) or FP32 (2^-24), scaled by the operator."""
