@@ -91,29 +91,100 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// Sum over the CTA; result valid in every thread. `sh` holds >= 33 doubles.
-__device__ __forceinline__ double block_sum(double v, double* sh)
+// The warp of a kReduceThreads CTA that finishes its sums: one of four by the CTA's place in the grid, so that
+// the CTAs of an SM use its four schedulers.
+__device__ __forceinline__ int finishing_warp() { return (int)(blockIdx.x / (kReduceCtas / 4)) & 3; }
+
+// Not +-0, without an instruction of the FP64 pipe.
+__device__ __forceinline__ bool nonzero(double v) { return (__double_as_longlong(v) << 1) != 0; }
+
+// N sums over a kReduceThreads CTA in one fixed order, valid in every thread. A warp's FP64 addition holds its
+// scheduler for 64 cycles (2 lanes a clock on an SM), so what counts is the warp instructions of all CTAs of an
+// SM: one warp a sum, each lane adding eight of the threads' values and five shuffles (12 additions), where
+// a shuffle reduction of every warp and then of their results takes 45 (2.8 us for two sums with four CTAs on an
+// SM, against 0.8). Groups of zeros add nothing: a CTA without elements, and the partials of one, cost no
+// addition.
+template <int N>
+__device__ __forceinline__ void block_sums(double (&v)[N])
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    v = warp_sum(v);
+    constexpr int kWarps = kReduceThreads / 32;
+    __shared__ double sh[N * kReduceThreads + N];
+    const int lane = threadIdx.x & 31, k = ((int)(threadIdx.x >> 5) - finishing_warp()) & (kWarps - 1);
+    __syncthreads();   // the previous call's sums are read
+#pragma unroll
+    for (int q = 0; q < N; q++) sh[q * kReduceThreads + threadIdx.x] = v[q];
     __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        double t = lane < nw ? sh[lane] : 0.0;
-        t = warp_sum(t);
-        if (lane == 0) sh[32] = t;
+    if (k < N) {
+        const double* p = sh + k * kReduceThreads + lane;
+        double t = p[0];
+#pragma unroll
+        for (int q = 1; q < kWarps; q++) {
+            const double u = p[32 * q];
+            if (__any_sync(0xffffffffu, nonzero(u))) t += u;
+        }
+        if (__any_sync(0xffffffffu, nonzero(t))) t = warp_sum(t);
+        if (lane == 0) sh[N * kReduceThreads + k] = t;
     }
     __syncthreads();
-    return sh[32];
+#pragma unroll
+    for (int q = 0; q < N; q++) v[q] = sh[N * kReduceThreads + q];
 }
 
-// Fixed-order reduction of a kReduceCtas-long partial array by one CTA.
-__device__ __forceinline__ double reduce_partials(const double* __restrict__ p, double* sh)
+__device__ __forceinline__ double block_sum(double v)
 {
-    double v = 0.0;
-    for (int i = threadIdx.x; i < kReduceCtas; i += blockDim.x) v += p[i];
-    return block_sum(v, sh);
+    double s[1] = {v};
+    block_sums(s);
+    return s[0];
+}
+
+// Fixed-order sums of kReduceCtas-long partial arrays by one CTA.
+template <int N>
+__device__ __forceinline__ void reduce_partials(const double* const (&p)[N], double (&v)[N])
+{
+    constexpr int kRounds = (kReduceCtas + kReduceThreads - 1) / kReduceThreads;
+    double u[N][kRounds];
+#pragma unroll
+    for (int k = 0; k < N; k++)
+#pragma unroll
+        for (int q = 0; q < kRounds; q++) {
+            const int i = q * kReduceThreads + threadIdx.x;
+            u[k][q] = i < kReduceCtas ? p[k][i] : 0.0;
+        }
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        v[k] = u[k][0];
+#pragma unroll
+        for (int q = 1; q < kRounds; q++)
+            if (__any_sync(0xffffffffu, nonzero(u[k][q]))) v[k] += u[k][q];
+    }
+    block_sums(v);
+}
+
+__device__ __forceinline__ double reduce_partials(const double* __restrict__ p)
+{
+    const double* const ps[1] = {p};
+    double v[1];
+    reduce_partials(ps, v);
+    return v[0];
+}
+
+// A Krylov scalar num / den and its FP32 pair in every thread, divided by one warp: an FP64 division is about
+// ten instructions of the FP64 pipe, 2.5 us when all warps of four CTAs on an SM take it.
+struct Scalar {
+    double v;
+    float h, l;
+};
+__device__ __forceinline__ Scalar cta_ratio(double num, double den)
+{
+    __shared__ Scalar s;
+    if ((int)(threadIdx.x >> 5) == finishing_warp()) {
+        Scalar q;
+        q.v = num / den;
+        df_split(q.v, q.h, q.l);
+        if ((threadIdx.x & 31) == 0) s = q;
+    }
+    __syncthreads();
+    return s;
 }
 
 // Element loop of the fixed-grid vector kernels: thread t of CTA c visits
@@ -121,22 +192,39 @@ __device__ __forceinline__ double reduce_partials(const double* __restrict__ p, 
 // order, so every per-thread sum is taken in one fixed order. Four elements go per step with all
 // their loads issued before the first use: one element per thread per step leaves too few bytes
 // in flight for HBM (a quarter of what the copy rate needs at 152 x 4 CTAs of 256 threads).
-// `load(i)` returns the element's inputs, `use(i, v)` computes and stores.
+// `load(i)` returns the element's inputs, `use(i, v)` computes and stores; `ready()` runs once behind the
+// first loads and in front of their use, for what the uses need of the grid's scalars.
 constexpr long long kRedStride = (long long)kReduceCtas * kReduceThreads;
 constexpr int kRedUnroll = 4;
+
+// A CTA of those kernels without elements (the first one always works).
+__device__ __forceinline__ bool idle_cta(long long n) { return blockIdx.x > 0 && (long long)blockIdx.x * kReduceThreads >= n; }
+
+template <class Load, class Ready, class Use>
+__device__ __forceinline__ void for_each_element(long long n, Load load, Ready ready, Use use)
+{
+    long long i = (long long)blockIdx.x * kReduceThreads + threadIdx.x;
+    decltype(load(i)) v[kRedUnroll];
+    auto fetch = [&] {
+#pragma unroll
+        for (int u = 0; u < kRedUnroll; u++)
+            if (i + u * kRedStride < n) v[u] = load(i + u * kRedStride);
+    };
+    fetch();
+    ready();
+    while (i < n) {
+#pragma unroll
+        for (int u = 0; u < kRedUnroll; u++)
+            if (i + u * kRedStride < n) use(i + u * kRedStride, v[u]);
+        i += kRedUnroll * kRedStride;
+        fetch();
+    }
+}
 
 template <class Load, class Use>
 __device__ __forceinline__ void for_each_element(long long n, Load load, Use use)
 {
-    long long i = (long long)blockIdx.x * kReduceThreads + threadIdx.x;
-    for (; i + (kRedUnroll - 1) * kRedStride < n; i += kRedUnroll * kRedStride) {
-        decltype(load(i)) v[kRedUnroll];
-#pragma unroll
-        for (int u = 0; u < kRedUnroll; u++) v[u] = load(i + u * kRedStride);
-#pragma unroll
-        for (int u = 0; u < kRedUnroll; u++) use(i + u * kRedStride, v[u]);
-    }
-    for (; i < n; i += kRedStride) use(i, load(i));
+    for_each_element(n, load, [] {}, use);
 }
 
 template <class A, class B>
@@ -967,7 +1055,6 @@ __global__ void __launch_bounds__(kReduceThreads) k_dots3(long long n, int nq, c
                                                           const T* __restrict__ b2, double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh[33];
     double v0 = 0.0, v1 = 0.0, v2 = 0.0;
     struct E {
         T a0, b0, a1, b1, a2, b2;
@@ -985,16 +1072,9 @@ __global__ void __launch_bounds__(kReduceThreads) k_dots3(long long n, int nq, c
             if (nq > 1) v1 = fma((double)e.a1, (double)e.b1, v1);
             if (nq > 2) v2 = fma((double)e.a2, (double)e.b2, v2);
         });
-    v0 = block_sum(v0, sh);
-    if (threadIdx.x == 0) partials[blockIdx.x] = v0;
-    if (nq > 1) {
-        v1 = block_sum(v1, sh);
-        if (threadIdx.x == 0) partials[kReduceCtas + blockIdx.x] = v1;
-    }
-    if (nq > 2) {
-        v2 = block_sum(v2, sh);
-        if (threadIdx.x == 0) partials[2 * kReduceCtas + blockIdx.x] = v2;
-    }
+    double s[3] = {v0, v1, v2};
+    block_sums(s);
+    if (threadIdx.x < nq) partials[threadIdx.x * kReduceCtas + blockIdx.x] = threadIdx.x == 0 ? s[0] : threadIdx.x == 1 ? s[1] : s[2];
 }
 
 // y += alpha x; out = a c + b d (K-cycle updates, coefficients from the host).

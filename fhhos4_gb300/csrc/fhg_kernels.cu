@@ -38,7 +38,6 @@ __global__ void __launch_bounds__(kReduceThreads) k_bsr_spmv_dots(int nbr, const
                                                                   double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh[33];
     const int lane = threadIdx.x & (G - 1);
     // Loop bounds are uniform per warp (every lane runs the same shuffle rounds).
     constexpr int kGroupsPerWarp = 32 / G;
@@ -68,12 +67,9 @@ __global__ void __launch_bounds__(kReduceThreads) k_bsr_spmv_dots(int nbr, const
             }
         }
     }
-    const double s1 = block_sum(dad, sh);
-    const double s2 = block_sum(rd, sh);
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = s1;
-        partials[kReduceCtas + blockIdx.x] = s2;
-    }
+    double sums[2] = {dad, rd};
+    block_sums(sums);
+    if (threadIdx.x < 2) partials[threadIdx.x * kReduceCtas + blockIdx.x] = threadIdx.x ? sums[1] : sums[0];
 }
 
 
@@ -99,7 +95,6 @@ __global__ void __launch_bounds__(kReduceThreads) k_bsr_spmv_dots_df(int nbr, co
                                                                      double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh_red[33];
     const int lane = threadIdx.x & (G - 1);
     constexpr int kGroupsPerWarp = 32 / G;
     const long long warp_id = ((long long)blockIdx.x * kReduceThreads + threadIdx.x) >> 5;
@@ -167,12 +162,9 @@ __global__ void __launch_bounds__(kReduceThreads) k_bsr_spmv_dots_df(int nbr, co
             }
         }
     }
-    const double s1 = block_sum((double)dad_h + (double)dad_l, sh_red);
-    const double s2 = block_sum((double)rd_h + (double)rd_l, sh_red);
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = s1;
-        partials[kReduceCtas + blockIdx.x] = s2;
-    }
+    double sums[2] = {(double)dad_h + (double)dad_l, (double)rd_h + (double)rd_l};
+    block_sums(sums);
+    if (threadIdx.x < 2) partials[threadIdx.x * kReduceCtas + blockIdx.x] = threadIdx.x ? sums[1] : sums[0];
 }
 
 // The same on the slot-major pair view of Â (slot s of row i at s * nbr + i; values as interleaved
@@ -192,7 +184,6 @@ __global__ void __launch_bounds__(kReduceThreads, 2) k_bsr_spmv_dots_df_slot(int
                                                                           double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh_red[33];
     float dad_h = 0.f, dad_l = 0.f, rd_h = 0.f, rd_l = 0.f;
     const long long stride = (long long)kReduceCtas * kReduceThreads;
     for (long long row = (long long)blockIdx.x * kReduceThreads + threadIdx.x; row < nbr; row += stride) {
@@ -235,12 +226,9 @@ __global__ void __launch_bounds__(kReduceThreads, 2) k_bsr_spmv_dots_df_slot(int
             df_add(rd_h, rd_l, ph, pl);
         }
     }
-    const double s1 = block_sum((double)dad_h + (double)dad_l, sh_red);
-    const double s2 = block_sum((double)rd_h + (double)rd_l, sh_red);
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = s1;
-        partials[kReduceCtas + blockIdx.x] = s2;
-    }
+    double sums[2] = {(double)dad_h + (double)dad_l, (double)rd_h + (double)rd_l};
+    block_sums(sums);
+    if (threadIdx.x < 2) partials[threadIdx.x * kReduceCtas + blockIdx.x] = threadIdx.x ? sums[1] : sums[0];
 }
 
 // The outer products on the row-class view of Â (fhg_bsr_kernels.cuh): one thread per block row over the
@@ -259,7 +247,6 @@ __global__ void __launch_bounds__(kReduceThreads, BS <= 3 ? 4 : 2) k_bsr_spmv_do
                                                                          double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh_red[33];
     float dad_h = 0.f, dad_l = 0.f, rd_h = 0.f, rd_l = 0.f;
     for (long long row = (long long)blockIdx.x * kReduceThreads + threadIdx.x; row < nbr; row += kRedStride) {
         const dfl* t = dict + cls[row];
@@ -294,12 +281,9 @@ __global__ void __launch_bounds__(kReduceThreads, BS <= 3 ? 4 : 2) k_bsr_spmv_do
             df_add(rd_h, rd_l, ph, pl);
         }
     }
-    const double s1 = block_sum((double)dad_h + (double)dad_l, sh_red);
-    const double s2 = block_sum((double)rd_h + (double)rd_l, sh_red);
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = s1;
-        partials[kReduceCtas + blockIdx.x] = s2;
-    }
+    double sums[2] = {(double)dad_h + (double)dad_l, (double)rd_h + (double)rd_l};
+    block_sums(sums);
+    if (threadIdx.x < 2) partials[threadIdx.x * kReduceCtas + blockIdx.x] = threadIdx.x ? sums[1] : sums[0];
 }
 
 template <int BS, int W>
@@ -312,7 +296,6 @@ __global__ void __launch_bounds__(kReduceThreads, BS <= 3 ? 4 : 2) k_bsr_spmv_do
                                                                       double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh[33];
     double dad = 0.0, rd = 0.0;
     for (long long row = (long long)blockIdx.x * kReduceThreads + threadIdx.x; row < nbr; row += kRedStride) {
         const double* t = dict + cls[row];
@@ -336,12 +319,9 @@ __global__ void __launch_bounds__(kReduceThreads, BS <= 3 ? 4 : 2) k_bsr_spmv_do
             rd = fma(rvec[i], xd[r], rd);
         }
     }
-    const double s1 = block_sum(dad, sh);
-    const double s2 = block_sum(rd, sh);
-    if (threadIdx.x == 0) {
-        partials[blockIdx.x] = s1;
-        partials[kReduceCtas + blockIdx.x] = s2;
-    }
+    double sums[2] = {dad, rd};
+    block_sums(sums);
+    if (threadIdx.x < 2) partials[threadIdx.x * kReduceCtas + blockIdx.x] = threadIdx.x ? sums[1] : sums[0];
 }
 
 // r = b - A x with compensated summation (Ogita, Rump and Oishi 2005, "Accurate sum and dot
@@ -363,7 +343,6 @@ __global__ void __launch_bounds__(kReduceThreads) k_bsr_residual_comp(int nbr, c
 {
     pdl_wait();
     if (enable && *enable == 0) return;
-    __shared__ double sh[33];
     double rr = 0.0;
     for (long long row = (long long)blockIdx.x * kReduceThreads + threadIdx.x; row < nbr; row += kRedStride) {
         double sum[BS], err[BS];
@@ -395,7 +374,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_bsr_residual_comp(int nbr, c
             rr = fma(v, v, rr);
         }
     }
-    rr = block_sum(rr, sh);
+    rr = block_sum(rr);
     if (threadIdx.x == 0) partials[blockIdx.x] = rr;
 }
 
@@ -403,11 +382,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_dot(long long n, const doubl
                                                         const double* __restrict__ b, double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh[33];
     double v = 0.0;
     for_each_element(n, [&](long long i) { return Pair2<double, double>{a[i], b[i]}; },
                      [&](long long, const Pair2<double, double>& e) { v = fma(e.a, e.b, v); });
-    v = block_sum(v, sh);
+    v = block_sum(v);
     if (threadIdx.x == 0) partials[blockIdx.x] = v;
 }
 
@@ -415,11 +393,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_dot_mixed(long long n, const
                                                               const double* __restrict__ b, double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh[33];
     double v = 0.0;
     for_each_element(n, [&](long long i) { return Pair2<float, double>{a[i], b[i]}; },
                      [&](long long, const Pair2<float, double>& e) { v = fma((double)e.a, e.b, v); });
-    v = block_sum(v, sh);
+    v = block_sum(v);
     if (threadIdx.x == 0) partials[blockIdx.x] = v;
 }
 
@@ -430,9 +407,11 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_direction_mixed(long lon
                                                                         float* __restrict__ dhi, float* __restrict__ dlo)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double s = reduce_partials(partials, sh) / *dadp;
+    if (idle_cta(n)) return;
+    const double den = *dadp;
+    double s;
     for_each_element(n, [&](long long i) { return Pair2<float, double>{z[i], dp[i]}; },
+                     [&] { s = cta_ratio(reduce_partials(partials), den).v; },
                      [&](long long i, const Pair2<float, double>& e) {
                          const double v = (double)e.a - s * e.b;
                          d[i] = v;
@@ -449,9 +428,11 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_direction(long long n, c
                                                                   const double* __restrict__ dadp, double* d)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double s = reduce_partials(partials, sh) / *dadp;
+    if (idle_cta(n)) return;
+    const double den = *dadp;
+    double s;
     for_each_element(n, [&](long long i) { return Pair2<double, double>{z[i], dp[i]}; },
+                     [&] { s = cta_ratio(reduce_partials(partials), den).v; },
                      [&](long long i, const Pair2<double, double>& e) { d[i] = e.a - s * e.b; });
 }
 
@@ -462,13 +443,18 @@ __global__ void __launch_bounds__(kReduceThreads) k_krylov_step(long long n, dou
                                                                 float* __restrict__ r32)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double num = reduce_partials(pnum, sh);
-    const double den = reduce_partials(pden, sh);
-    const double alpha = num / den;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && den_out) *den_out = den;
-    double rr = 0.0;
+    if (idle_cta(n)) {
+        if (threadIdx.x == 0) prr[blockIdx.x] = 0.0;
+        return;
+    }
+    double alpha, rr = 0.0;
     for_each_element(n, [&](long long i) { return Quad4<double>{x[i], d[i], r[i], Ad[i]}; },
+                     [&] {
+                         double s[2];
+                         reduce_partials({pnum, pden}, s);
+                         if (blockIdx.x == 0 && threadIdx.x == 0 && den_out) *den_out = s[1];
+                         alpha = cta_ratio(s[0], s[1]).v;
+                     },
                      [&](long long i, const Quad4<double>& e) {
                          x[i] = e.a + alpha * e.b;
                          const double ri = e.c - alpha * e.d;
@@ -476,7 +462,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_krylov_step(long long n, dou
                          if (r32) r32[i] = (float)ri;
                          rr = fma(ri, ri, rr);
                      });
-    rr = block_sum(rr, sh);
+    rr = block_sum(rr);
     if (threadIdx.x == 0) prr[blockIdx.x] = rr;
 }
 
@@ -492,7 +478,6 @@ __global__ void __launch_bounds__(kReduceThreads) k_dot_df(long long n, const fl
                                                            double* __restrict__ partials)
 {
     pdl_wait();
-    __shared__ double sh[33];
     float vh = 0.f, vl = 0.f;
     struct E {
         float zh, zl, h, l;
@@ -510,7 +495,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_dot_df(long long n, const fl
                          df_mul(e.zh, e.zl, e.h, e.l, ph, pl);
                          df_add(vh, vl, ph, pl);
                      });
-    const double v = block_sum((double)vh + (double)vl, sh);
+    const double v = block_sum((double)vh + (double)vl);
     if (threadIdx.x == 0) partials[blockIdx.x] = v;
 }
 
@@ -524,9 +509,9 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_direction_df(long long n
                                                                      float* __restrict__ dh, float* __restrict__ dl)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    float sh_, sl_;
-    df_split(reduce_partials(partials, sh) / *dadp, sh_, sl_);
+    if (idle_cta(n)) return;
+    const double den = *dadp;
+    Scalar s;
     struct E {
         float zh, zl, h, l;
     };
@@ -538,9 +523,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_fcg_direction_df(long long n
                          }
                          return E{z[i], 0.f, dph[i], dpl[i]};
                      },
+                     [&] { s = cta_ratio(reduce_partials(partials), den); },
                      [&](long long i, const E& e) {
                          float ph, pl, h, l;
-                         df_mul(sh_, sl_, e.h, e.l, ph, pl);
+                         df_mul(s.h, s.l, e.h, e.l, ph, pl);
                          df_sum(e.zh, e.zl, -ph, -pl, h, l);
                          dh[i] = h;
                          dl[i] = l;
@@ -561,23 +547,27 @@ __global__ void __launch_bounds__(kReduceThreads) k_krylov_step_df(long long n, 
                                                                    dfl* __restrict__ r2)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double num = reduce_partials(pnum, sh);
-    const double den = reduce_partials(pden, sh);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && den_out) *den_out = den;
-    const double alpha = num / den;
-    float ah, al;
-    df_split(alpha, ah, al);
+    if (idle_cta(n)) {
+        if (threadIdx.x == 0) prr[blockIdx.x] = 0.0;
+        return;
+    }
+    Scalar alpha;
     float rrh = 0.f, rrl = 0.f;
     struct E {
         double x;
         float rh, rl, dh, dl, ah, al;
     };
     for_each_element(n, [&](long long i) { return E{x[i], rh[i], rl[i], dh[i], dl[i], Adh[i], Adl[i]}; },
+                     [&] {
+                         double s[2];
+                         reduce_partials({pnum, pden}, s);
+                         if (blockIdx.x == 0 && threadIdx.x == 0 && den_out) *den_out = s[1];
+                         alpha = cta_ratio(s[0], s[1]);
+                     },
                      [&](long long i, const E& e) {
                          float ph, pl, h, l;
-                         x[i] = fma(alpha, (double)e.dh + (double)e.dl, e.x);
-                         df_mul(ah, al, e.ah, e.al, ph, pl);
+                         x[i] = fma(alpha.v, (double)e.dh + (double)e.dl, e.x);
+                         df_mul(alpha.h, alpha.l, e.ah, e.al, ph, pl);
                          df_sum(e.rh, e.rl, -ph, -pl, h, l);
                          rh[i] = h;
                          rl[i] = l;
@@ -585,7 +575,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_krylov_step_df(long long n, 
                          df_mul(h, l, h, l, ph, pl);
                          df_add(rrh, rrl, ph, pl);
                      });
-    const double rr = block_sum((double)rrh + (double)rrl, sh);
+    const double rr = block_sum((double)rrh + (double)rrl);
     if (threadIdx.x == 0) prr[blockIdx.x] = rr;
 }
 
@@ -611,18 +601,21 @@ __global__ void __launch_bounds__(kReduceThreads) k_cg_step(long long n, double*
                                                             double* __restrict__ prr)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double den = reduce_partials(pden, sh);
-    const double alpha = *num / den;
-    double rr = 0.0;
+    if (idle_cta(n)) {
+        if (threadIdx.x == 0) prr[blockIdx.x] = 0.0;
+        return;
+    }
+    const double rz = *num;
+    double alpha, rr = 0.0;
     for_each_element(n, [&](long long i) { return Quad4<double>{x[i], d[i], r[i], Ad[i]}; },
+                     [&] { alpha = cta_ratio(rz, reduce_partials(pden)).v; },
                      [&](long long i, const Quad4<double>& e) {
                          x[i] = e.a + alpha * e.b;
                          const double ri = e.c - alpha * e.d;
                          r[i] = ri;
                          rr = fma(ri, ri, rr);
                      });
-    rr = block_sum(rr, sh);
+    rr = block_sum(rr);
     if (threadIdx.x == 0) prr[blockIdx.x] = rr;
 }
 
@@ -639,8 +632,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_finalize_norm(const double* 
                                                                   double* nr_out, double* hist, int* counter, int hist_len)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double rn = sqrt(reduce_partials(prr, sh));
+    const double rn = sqrt(reduce_partials(prr));
     if (threadIdx.x == 0) {
         const double bn = *bnorm;
         const double nr = bn > 0.0 ? rn / bn : rn;
@@ -654,24 +646,21 @@ __global__ void __launch_bounds__(kReduceThreads) k_finalize_norm(const double* 
 __global__ void __launch_bounds__(kReduceThreads) k_sqrt_sum(const double* __restrict__ p, double* out)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double v = reduce_partials(p, sh);
+    const double v = reduce_partials(p);
     if (threadIdx.x == 0) *out = sqrt(v);
 }
 
 __global__ void __launch_bounds__(kReduceThreads) k_sum(const double* __restrict__ p, double* out)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double v = reduce_partials(p, sh);
+    const double v = reduce_partials(p);
     if (threadIdx.x == 0) *out = v;
 }
 
 __global__ void __launch_bounds__(kReduceThreads) k_cg_beta(const double* __restrict__ p, double* rz, double* beta)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double v = reduce_partials(p, sh);
+    const double v = reduce_partials(p);
     if (threadIdx.x == 0) {
         *beta = v / *rz;
         *rz = v;
@@ -1012,8 +1001,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_check_fp64(const double* __r
                                                                int* state)
 {
     pdl_wait();
-    __shared__ double sh[33];
-    const double rn = sqrt(reduce_partials(p, sh));
+    const double rn = sqrt(reduce_partials(p));
     if (threadIdx.x == 0) {
         scal[5] = rn;
         const double bn = scal[0];
@@ -1030,8 +1018,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_check_comp(const double* __r
 {
     pdl_wait();
     if (state[kLoopNeedComp] == 0) return;
-    __shared__ double sh[33];
-    const double rn = sqrt(reduce_partials(p, sh));
+    const double rn = sqrt(reduce_partials(p));
     if (threadIdx.x == 0) {
         scal[5] = rn;
         const double bn = scal[0];
