@@ -137,13 +137,14 @@ struct Rows {
     unsigned ld;   // entries of the levels here fit 32 bits (fused_layout)
 };
 
-// The local rows [lo, hi) of a phase, and a lane's place in its first row: the row's bounds (p: the lane's
-// first block; it takes p, p + g, ...) and its first columns (-1: none).
+// The local rows [lo, hi) of a phase, a row's bounds, and the columns of a lane's first blocks in it (-1:
+// none); lane t of a row takes its blocks t, t + g, ... The bounds stay as loaded: an addition would wait for
+// them there.
 struct Span {
     int lo = 0, hi = 0;
 };
 struct Bounds {
-    int p = 0, p1 = 0;
+    int p0 = 0, p1 = 0;
 };
 template <int N>
 struct Columns {
@@ -151,23 +152,23 @@ struct Columns {
 };
 
 template <class T>
-__device__ __forceinline__ Bounds row_bounds(const Ctx<T>& C, const Rows<T>& M, int u, int hi, int g)
+__device__ __forceinline__ Bounds row_bounds(const Ctx<T>& C, const Rows<T>& M, int u, int hi)
 {
     Bounds b;
     if (u < hi) {
         const int i = C.row(u);
-        b.p = M.rowptr[i] + (C.lane & (g - 1));
+        b.p0 = M.rowptr[i];
         b.p1 = M.rowptr[i + 1];
     }
     return b;
 }
 
 template <int N, class T>
-__device__ __forceinline__ Columns<N> row_columns(const Rows<T>& M, const Bounds& b, int g)
+__device__ __forceinline__ Columns<N> row_columns(const Rows<T>& M, int p, int p1, int g)
 {
     Columns<N> c;
 #pragma unroll
-    for (int q = 0; q < N; q++) c.col[q] = b.p + q * g < b.p1 ? M.colidx[b.p + q * g] : -1;
+    for (int q = 0; q < N; q++) c.col[q] = p + q * g < p1 ? M.colidx[p + q * g] : -1;
     return c;
 }
 
@@ -175,8 +176,7 @@ __device__ __forceinline__ Columns<N> row_columns(const Rows<T>& M, const Bounds
 // bytes of a block: 128 registers of a 512-thread CTA, 64 of a 1024-thread one. kHold: the values in registers
 // (else as the sums reach them).
 template <class T, int BS, int TH>
-constexpr int kLaneBlocks = TH > kFusedThreads ? 1
-                            : BS * BS * (int)sizeof(T) <= 16 ? 4 : BS * BS * (int)sizeof(T) <= 36 ? 2 : 1;
+constexpr int kLaneBlocks = TH <= kFusedThreads && BS * BS * (int)sizeof(T) <= 16 ? 2 : 1;
 template <class T, int BS, int TH>
 constexpr bool kHold = BS * BS * (int)sizeof(T) <= (TH > kFusedThreads ? 16 : 36);
 
@@ -206,7 +206,8 @@ __device__ __forceinline__ void rows_phase(const Ctx<T>& C, Span span, int g, co
         const int u = base + C.lane / g;
         const bool in = u < span.hi;
         const int i = C.row(u);
-        Bounds at = bounds;
+        int p = bounds.p0 + lane;
+        const int p1 = bounds.p1;
         Columns<NB> now = cols;
         T acc[BS], dv[BS];
 #pragma unroll
@@ -236,7 +237,7 @@ __device__ __forceinline__ void rows_phase(const Ctx<T>& C, Span span, int g, co
                 for (int c = 0; c < BS; c++) xv[q][c] = T(0);
                 if (j >= 0) {
                     if (HOLD) {
-                        const T* vp = M.vals + (at.p + q * g);
+                        const T* vp = M.vals + (p + q * g);
 #pragma unroll
                         for (int e = 0; e < BS * BS; e++, vp += ld) v[q][e] = *vp;
                     }
@@ -246,12 +247,12 @@ __device__ __forceinline__ void rows_phase(const Ctx<T>& C, Span span, int g, co
             if (first) {   // behind the loads this row waits for
                 first = false;
                 if (base + stride < span.hi) {   // another pass of this phase
-                    bounds = row_bounds(C, M, u + stride, span.hi, g);
+                    bounds = row_bounds(C, M, u + stride, span.hi);
                 } else if (!ahead) {
                     ahead = true;
                     bounds = next_bounds;
-                    cols = row_columns<NB>(M, bounds, g);
-                    next_bounds = row_bounds(C, M, after.lo + group, after.hi, g);
+                    cols = row_columns<NB>(M, bounds.p0 + lane, bounds.p1, g);
+                    next_bounds = row_bounds(C, M, after.lo + group, after.hi);
                 }
             }
 #pragma unroll
@@ -261,16 +262,16 @@ __device__ __forceinline__ void rows_phase(const Ctx<T>& C, Span span, int g, co
                 for (int r = 0; r < BS; r++)
 #pragma unroll
                     for (int c = 0; c < BS; c++) {
-                        const T a = HOLD ? v[q][r * BS + c] : M.vals[(unsigned)(r * BS + c) * ld + (unsigned)(at.p + q * g)];
+                        const T a = HOLD ? v[q][r * BS + c] : M.vals[(unsigned)(r * BS + c) * ld + (unsigned)(p + q * g)];
                         acc[r] = fma(a, xv[q][c], acc[r]);
                     }
             }
-            at.p += NB * g;
-            if (at.p >= at.p1) break;   // per lane; no shuffle inside the loop
-            now = row_columns<NB>(M, at, g);
+            p += NB * g;
+            if (p >= p1) break;   // per lane; no shuffle inside the loop
+            now = row_columns<NB>(M, p, p1, g);
         }
         if (base >= span.hi) break;   // a warp without a row: only asked for the next phases' data
-        if (base + stride < span.hi) cols = row_columns<NB>(M, bounds, g);
+        if (base + stride < span.hi) cols = row_columns<NB>(M, bounds.p0 + lane, bounds.p1, g);
 #pragma unroll
         for (int r = 0; r < BS; r++) acc[r] = lanes_sum(acc[r], g);
         if (!in) continue;
@@ -279,13 +280,19 @@ __device__ __forceinline__ void rows_phase(const Ctx<T>& C, Span span, int g, co
             T t[BS];
 #pragma unroll
             for (int c = 0; c < BS; c++) t[c] = b[u * BS + c] - acc[c];
-            for (int r = lane; r < BS; r += g) {
+            auto output = [&](int r, const T (&d)[BS]) {
                 T y = T(0);
 #pragma unroll
-                for (int c = 0; c < BS; c++)
-                    y = fma(r == lane ? dv[c] : dinv[(unsigned)(r * BS + c) * (unsigned)nb + (unsigned)i], t[c], y);
+                for (int c = 0; c < BS; c++) y = fma(d[c], t[c], y);
                 if (w != T(1)) y = fma(w, y, (T(1) - w) * out[u * BS + r]);
                 out[u * BS + r] = fin(y);
+            };
+            if (lane < BS) output(lane, dv);
+            for (int r = lane + g; r < BS; r += g) {   // fewer lanes than outputs
+                T d[BS];
+#pragma unroll
+                for (int c = 0; c < BS; c++) d[c] = dinv[(unsigned)(r * BS + c) * (unsigned)nb + (unsigned)i];
+                output(r, d);
             }
         } else {
 #pragma unroll
@@ -313,8 +320,8 @@ __device__ __forceinline__ void product(const Ctx<T>& C, int rows, int g, const 
 {
     constexpr int NB = kLaneBlocks<T, BS, TH>;
     const Span span{0, C.local_rows(rows)};
-    Bounds bounds = row_bounds(C, M, C.warp * (32 / g) + C.lane / g, span.hi, g), none;
-    Columns<NB> cols = row_columns<NB>(M, bounds, g);
+    Bounds bounds = row_bounds(C, M, C.warp * (32 / g) + C.lane / g, span.hi), none;
+    Columns<NB> cols = row_columns<NB>(M, bounds.p0 + (C.lane & (g - 1)), bounds.p1, g);
     rows_phase<T, BS, TH, KIND>(C, span, g, M, bounds, cols, none, Span(), Span(), src, nullptr, 0, b, out, zero);
 }
 
@@ -342,9 +349,10 @@ __device__ void smooth(const Ctx<T>& C, const FusedLevel<T>& L, int code, int it
         return r;
     };
     Span now = next_span(), next = next_span(), after = next_span();
-    Bounds bounds = row_bounds(C, A, now.lo + group, now.hi, g);
-    Bounds next_bounds = row_bounds(C, A, next.lo + group, next.hi, g);
-    Columns<kLaneBlocks<T, BS, TH>> cols = row_columns<kLaneBlocks<T, BS, TH>>(A, bounds, g);
+    Bounds bounds = row_bounds(C, A, now.lo + group, now.hi);
+    Bounds next_bounds = row_bounds(C, A, next.lo + group, next.hi);
+    Columns<kLaneBlocks<T, BS, TH>> cols =
+        row_columns<kLaneBlocks<T, BS, TH>>(A, bounds.p0 + (C.lane & (g - 1)), bounds.p1, g);
     for (int phase = sweeps * L.ncol; phase > 0; phase--) {
         rows_phase<T, BS, TH, kRowSweep>(C, now, g, A, bounds, cols, next_bounds, next, after, L.x_off, L.dinv, L.nb,
                                          C.local(L.b_off), C.local(L.x_off), nullptr);

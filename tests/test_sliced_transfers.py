@@ -50,10 +50,12 @@ def test_gpu_transfers_on_sliced_views(dim, n, k, precision):
     rd, ed = put(rng.standard_normal(A.shape[0])), put(rng.standard_normal(top))
     r, e = get(rd), get(ed)
     out = torch.full_like(ed, float("nan"))
+    torch.cuda.synchronize()   # the context has a stream of its own
     ctx.apply_internal(0, N.OP_RESTRICT, precision, rd.data_ptr(), None, out.data_ptr())
     scale = (abs(Pp).T @ np.abs(r)).max()
     assert np.abs(get(out) - Pp.T @ r).max() <= TOL[precision] * scale
     out = torch.full_like(rd, float("nan"))
+    torch.cuda.synchronize()
     ctx.apply_internal(0, N.OP_PROLONG_ADD, precision, ed.data_ptr(), rd.data_ptr(), out.data_ptr())
     scale = np.abs(r).max() + (abs(Pp) @ np.abs(e)).max()
     assert np.abs(get(out) - (r + Pp @ e)).max() <= TOL[precision] * scale
