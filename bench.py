@@ -538,6 +538,7 @@ def run_ours(args, dist: Dist):
     # Dominant kernel of the headline (FP32 V-cycle) solve: GS sweeps on level 0.
     ncol = info0["colours"]
     gs_min_bytes = (nnzb0 - nb0) * (bs * bs * p32 + 4) + nb0 * bs * bs * p32 + 3 * n0 * p32
+    class_bytes = nb0 * (2 + 4 * 6) + 3 * n0 * p32
     dom = "bsr_gs_sweep_fp32"
     hbm, hbm_kind = measured_hbm_peak()
     traffic = committed_traffic().get(dom)
@@ -552,6 +553,11 @@ def run_ours(args, dist: Dist):
                 # and row pointers, which the sweep does not read).
                 "min_bytes_per_launch": gs_min_bytes / max(ncol, 1),
                 "frac_min_bytes": round(gs_min_bytes / (kernels[dom]["ms"] * 1e-3) / 1e9 / hbm, 4),
+                # Where block rows repeat, the sweep reads a 16-bit class and 6 columns per row instead of
+                # the blocks, so the byte counts above (and the captured traffic, of the stored-block
+                # sweep) are not moved and the fractions can exceed 1. What that sweep moves at least:
+                "class_view_bytes_per_launch": class_bytes / max(ncol, 1),
+                "frac_class_view": round(class_bytes / (kernels[dom]["ms"] * 1e-3) / 1e9 / hbm, 4),
                 "spmv_fp64_frac": round(kernels["bsr_spmv_fp64"]["gbs"] / hbm, 4),
         "spmv_fp64_native_frac": round(kernels["bsr_spmv_fp64_native"]["gbs"] / hbm, 4),
                 "spmv_fp32_frac": round(kernels["bsr_spmv_fp32"]["gbs"] / hbm, 4)}
