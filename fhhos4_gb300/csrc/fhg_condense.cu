@@ -215,7 +215,10 @@ __global__ void __launch_bounds__(kCondThreads) k_fill(CondData D, const long lo
         int col[kCondMaxRowBlocks];     // block columns
         unsigned lf0, lf1;              // 4 bits per column: its local face in element 1 / 2 (15: none)
         long long s0, s1;               // first entry of S of element 1 / 2 at the face's rows
-        int nb, start;                  // block columns; blocks before this row in the CTA
+        short nb;                       // block columns
+        short glued;                    // an element has a block on several faces (a periodic mesh one cell
+                                        // across): the 4 bits of lf0, lf1 are then a bit per local face
+        int start;                      // blocks before this row in the CTA
     };
     __shared__ Row rows[kCondThreads];
     __shared__ int warp_sum[kCondThreads / 32];
@@ -230,7 +233,8 @@ __global__ void __launch_bounds__(kCondThreads) k_fill(CondData D, const long lo
         nb = row_columns(D, I, cols);
 #pragma unroll
         for (int q = 0; q < kCondMaxRowBlocks; q++) R.col[q] = q < nb ? cols[q] : 0;
-        unsigned lfs[2] = {0xffffffffu, 0xffffffffu};
+        unsigned lfs[2] = {0xffffffffu, 0xffffffffu}, faces[2] = {0u, 0u};
+        R.glued = 0;
         long long first[2] = {0, 0};
         double acc[NF ? NF : kCondMaxFaceDofs];
         for (int a = 0; a < nf; a++) acc[a] = 0.0;
@@ -245,7 +249,9 @@ __global__ void __launch_bounds__(kCondThreads) k_fill(CondData D, const long lo
                 if (g < 0) continue;
                 int q = 0;
                 while (q < nb && cols[q] != g) q++;
+                if ((faces[side] >> (4 * q)) & 15u) R.glued = 1;
                 lfs[side] = (lfs[side] & ~(15u << (4 * q))) | ((unsigned)lf << (4 * q));
+                faces[side] |= 1u << (4 * q + lf);
             }
             const double* G = D.G + ((long long)c * nFF + lfi * nf) * nC;
             const double* bT = D.b_cell + (long long)e * nC;
@@ -256,10 +262,11 @@ __global__ void __launch_bounds__(kCondThreads) k_fill(CondData D, const long lo
             }
         }
         for (int a = 0; a < nf; a++) b[(long long)I * nf + a] = acc[a];
-        R.lf0 = lfs[0]; R.lf1 = lfs[1];
+        R.lf0 = R.glued ? faces[0] : lfs[0];
+        R.lf1 = R.glued ? faces[1] : lfs[1];
         R.s0 = first[0]; R.s1 = first[1];
     }
-    R.nb = nb;
+    R.nb = (short)nb;
     int run = nb;   // blocks of the CTA's rows up to this one
     for (int o = 1; o < 32; o <<= 1) {
         const int t = __shfl_up_sync(0xffffffffu, run, o);
@@ -285,10 +292,15 @@ __global__ void __launch_bounds__(kCondThreads) k_fill(CondData D, const long lo
         for (int e = lane; e < count; e += 32) {
             const int a = (int)(((unsigned)e * inv) >> 20), j = e - a * width;
             const int q = j / nf, cc = j - q * nf;
-            const unsigned f0 = (W.lf0 >> (4 * q)) & 15u, f1 = (W.lf1 >> (4 * q)) & 15u;
+            unsigned f0 = (W.lf0 >> (4 * q)) & 15u, f1 = (W.lf1 >> (4 * q)) & 15u;
             double v = 0.0;
-            if (f0 != 15u) v += D.S[W.s0 + a * nFF + (int)f0 * nf + cc];
-            if (f1 != 15u) v += D.S[W.s1 + a * nFF + (int)f1 * nf + cc];
+            if (!W.glued) {
+                if (f0 != 15u) v += D.S[W.s0 + a * nFF + (int)f0 * nf + cc];
+                if (f1 != 15u) v += D.S[W.s1 + a * nFF + (int)f1 * nf + cc];
+            } else {
+                for (; f0; f0 &= f0 - 1) v += D.S[W.s0 + a * nFF + (__ffs(f0) - 1) * nf + cc];
+                for (; f1; f1 &= f1 - 1) v += D.S[W.s1 + a * nFF + (__ffs(f1) - 1) * nf + cc];
+            }
             colidx[base + e] = W.col[q] * nf + cc;
             vals[base + e] = v;
         }

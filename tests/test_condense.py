@@ -191,3 +191,55 @@ def test_gpu_condensation_of_distinct_elements(dim, n, k):
     assert np.array_equal(A.indptr, A0.indptr) and np.array_equal(A.indices, A0.indices)
     assert np.abs(A.data - A0.data).max() <= 1e-12 * np.abs(A0.data).max()
     assert np.abs(b - b0).max() <= 1e-12 * np.abs(b0).max()
+
+
+def _glued(t):
+    """The tables with two faces of some elements identified: their unknown blocks become one, whose two sides are
+    that element (as in a periodic mesh one cell across). The neighbours' faces there become Dirichlet, the blocks
+    are renumbered. Also returns how many elements were glued."""
+    nF, nI = t["dim"] + 1, t["n_face_blocks"]
+    ef = t["elem_faces"].reshape(-1, nF).copy()
+    fe = t["face_elems"].reshape(nI, 4).copy()
+    glued = []
+    for e in range(ef.shape[0]):
+        lf = np.flatnonzero(ef[e] >= 0)
+        if len(lf) < 2 or any(set(ef[e]) & set(g) for g in glued):
+            continue
+        i, j = lf[0], lf[-1]
+        I, J = ef[e, i], ef[e, j]
+        glued.append(set(ef[e]) - {-1})
+        ef[(ef == I) | (ef == J)] = -1
+        ef[e, i] = ef[e, j] = I
+        fe[I] = (e, i, e, j)
+        fe[J] = (-1, 0, -1, 0)
+    keep = np.flatnonzero(fe[:, 0] >= 0)
+    new = np.full(nI + 1, -1, np.int32)
+    new[keep] = np.arange(len(keep))
+    ef = new[ef].astype(np.int32)
+    return dict(t, elem_faces=np.ascontiguousarray(ef.ravel()), n_face_blocks=len(keep),
+                face_elems=np.ascontiguousarray(fe[keep].astype(np.int32).ravel())), len(glued)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,n,k", [(2, 6, 1), (2, 6, 3), (3, 3, 1), (3, 3, 2), (3, 3, 3)])
+def test_gpu_condensation_of_an_element_glued_to_itself(dim, n, k):
+    """An element may hold one face block twice (its face row then gets four blocks of one local operator): every
+    contribution is added. Tolerance: as the host assembly's."""
+    from fhhos4_gb300 import _native as N
+    H = hho.Hierarchy(dim, n, k, max_levels=1)
+    try:
+        t, glued = _glued(H.condense_tables())
+    finally:
+        H.close()
+    assert glued > 3
+    A0, b0 = numpy_condense(t)
+    A0.sort_indices()
+    cond = N.Condense(t)
+    try:
+        nnz, _ = cond.run()
+        A, b = cond.result(nnz)
+    finally:
+        cond.close()
+    assert np.array_equal(A.indptr, A0.indptr) and np.array_equal(A.indices, A0.indices)
+    assert np.abs(A.data - A0.data).max() <= 1e-13 * np.abs(A0.data).max()
+    assert np.abs(b - b0).max() <= 1e-13 * np.abs(b0).max()
