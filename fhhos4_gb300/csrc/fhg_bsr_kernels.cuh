@@ -389,9 +389,12 @@ __global__ void __launch_bounds__(kThreads) k_bsr_spmv_sell(int slices, const in
 #pragma unroll
     for (int g = 0; g < kGroup; g++) col[g] = p + 32 * g < p1 ? colidx[p + 32 * g] : -1;
     pdl_wait();
-    T acc[BS];
+    T acc[BS], av[BS];   // M x is summed from zero and added once: from y on, every product would round at y's size
 #pragma unroll
-    for (int r = 0; r < BS; r++) acc[r] = MODE == kSpmvAssign || row < 0 ? T(0) : aux[(long long)row * BS + r];
+    for (int r = 0; r < BS; r++) {
+        av[r] = MODE == kSpmvAssign || row < 0 ? T(0) : aux[(long long)row * BS + r];
+        acc[r] = T(0);
+    }
     while (p < p1) {   // the same number of steps in every lane
         T xv[kGroup][BS], v[kGroup][BS * BS];
 #pragma unroll
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(kThreads) k_bsr_spmv_sell(int slices, const in
     if (row < 0) return;
 #pragma unroll
     for (int r = 0; r < BS; r++)
-        if (L == 1 || r % L == lane % L) y[(long long)row * BS + r] = fin(acc[r]);
+        if (L == 1 || r % L == lane % L) y[(long long)row * BS + r] = MODE == kSpmvAssign ? fin(acc[r]) : av[r] + acc[r];
 }
 
 // w = D^-1 (b - A x) (block-Jacobi-scaled residual, the learned step's input): the residual of a

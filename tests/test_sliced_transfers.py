@@ -60,3 +60,50 @@ def test_gpu_transfers_on_sliced_views(dim, n, k, precision):
     scale = np.abs(r).max() + (abs(Pp) @ np.abs(e)).max()
     assert np.abs(get(out) - (r + Pp @ e)).max() <= TOL[precision] * scale
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("dim,n,k", [(2, 112, 1), (2, 106, 3), (3, 16, 1), (3, 16, 2)])
+def test_gpu_prolongation_rounds_once_at_the_size_of_x(dim, n, k, precision):
+    """x + P e with e a hundredth of x: P e is summed from zero and x added once, so an entry is off by half a unit
+    in the last place of the result and the rounding of the row's m products, m u |P||e|, where summing from x on
+    rounds m times at the size of x."""
+    torch = pytest.importorskip("torch")
+    from fhhos4_gb300 import _native as N
+    from fhhos4_gb300 import solver as S
+    from test_gpu_parity import scalar_perm
+    import scipy.sparse as sp
+    H = hho.Hierarchy(dim, n, k, max_levels=2)
+    A, P, bs = H.A(0), H.P(0).tocsr(), H.block_size
+    H.close()
+    top = P.shape[1]
+    nb = top // bs
+    Q = sp.csr_matrix((np.ones(top), (np.arange(top), np.tile(np.arange(bs), nb))), shape=(top, bs))
+    ctx = S.fcg_mg([A, sp.identity(top, format="csr"), sp.identity(bs, format="csr")], [P, Q], bs, precision=precision,
+                   fused=False).Context()
+    p0 = scalar_perm(ctx.permutation(0, A.shape[0] // bs), bs)
+    p1 = scalar_perm(ctx.permutation(1, nb), bs)
+    rng = np.random.default_rng(4)
+    dt = np.float64 if precision == "fp64" else np.float32
+    x, e = rng.standard_normal(A.shape[0]).astype(dt), (0.01 * rng.standard_normal(top)).astype(dt)
+    xd, ed = torch.tensor(x, device="cuda"), torch.tensor(e, device="cuda")
+    out = torch.full_like(xd, float("nan"))
+    torch.cuda.synchronize()
+    ctx.apply_internal(0, N.OP_PROLONG_ADD, precision, ed.data_ptr(), xd.data_ptr(), out.data_ptr())
+    Pp = P[p0][:, p1].tocsr()
+    vals = Pp.data.astype(dt).astype(np.longdouble)   # the values as the view stores them
+    terms = vals * e.astype(np.longdouble)[Pp.indices]
+    full = np.diff(Pp.indptr) > 0
+
+    def rows(t):
+        s = np.zeros(Pp.shape[0], np.longdouble)
+        s[full] = np.add.reduceat(t, Pp.indptr[:-1][full])
+        return s
+
+    ref, size = x.astype(np.longdouble) + rows(terms), rows(np.abs(terms))
+    u = np.longdouble(2.0) ** (-53 if precision == "fp64" else -24)
+    # a row's block columns hold bs products each, zeros of the blocks among them
+    m = bs * 7
+    err = np.abs(out.cpu().numpy().astype(np.longdouble) - ref)
+    assert np.all(err <= (1 + u) * u * (np.abs(ref) + (m + 1) * size)), float((err / (u * np.abs(ref) + m * u * size)).max())
+    ctx.close()
