@@ -45,7 +45,7 @@ EXPORTS = ["fhg_default_options", "fhg_create", "fhg_destroy", "fhg_last_error",
            "fhg_learned_reference_rate", "fhg_learned_features", "fhg_apply_internal", "fhg_net_num_params",
            "fhg_net_create", "fhg_net_destroy", "fhg_net_last_error", "fhg_net_set_params", "fhg_net_get_params",
            "fhg_net_train_step", "fhg_io_buffers", "fhg_io_upload", "fhg_io_download", "fhg_batch_create", "fhg_batch_destroy", "fhg_batch_last_error",
-           "fhg_batch_add", "fhg_batch_solve", "fhg_post_create", "fhg_post_run", "fhg_post_last_error",
+           "fhg_batch_add", "fhg_batch_solve", "fhg_post_create", "fhg_post_run", "fhg_post_factors", "fhg_post_last_error",
            "fhg_post_destroy", "fhg_cond_create", "fhg_cond_run", "fhg_cond_result", "fhg_cond_download", "fhg_cond_last_error",
            "fhg_cond_destroy"]
 
@@ -140,6 +140,7 @@ def load(path: str = LIB):
     lib.fhg_batch_solve.argtypes = [C.c_void_p, C.c_void_p, P(C.c_double)]
     lib.fhg_post_create.argtypes = [P(C.c_void_p)] + [C.c_int] * 8 + [C.c_void_p] * 9
     lib.fhg_post_run.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, P(C.c_double), P(C.c_double)]
+    lib.fhg_post_factors.argtypes = [C.c_void_p]
     lib.fhg_post_last_error.argtypes = [C.c_void_p]
     lib.fhg_post_last_error.restype = C.c_char_p
     lib.fhg_post_destroy.argtypes = [C.c_void_p]
@@ -381,6 +382,10 @@ class Post:
         self._check(self.lib.fhg_post_run(self.h, C.c_void_p(x_faces_dev), C.c_void_p(x_cells_dev) if x_cells_dev else None,
                                           EXACT[exact], C.byref(err), C.byref(ms)))
         return (err.value if exact != "none" else None), ms.value
+
+    def factors(self) -> int:
+        """Quadrature tables factorised so far (0: none asked for yet, or the sums go over the points)."""
+        return int(self.lib.fhg_post_factors(self.h))
 
     def close(self):
         if self.h:

@@ -19,7 +19,7 @@
 // cos(pi c) sin(pi o), so u at the points of an element is Phi t: 2^dim class functions Phi (products of
 // cos / sin of pi o) times 2^dim element coefficients t. With u_h = B c_h there, sum_q w_q (u_h - u)^2 is
 // the squared 2-norm of sqrt(W) [Phi B] (t, -c_h), and a QR factorisation of that matrix per distinct
-// table (at setup) leaves the same number as |R (t, -c_h)|^2 with R of 2^dim + n_recon rows: 171 multiply-adds
+// table (on the first run that asks) leaves the same number as |R (t, -c_h)|^2 with R of 2^dim + n_recon rows: 171 multiply-adds
 // per element in 3D, k = 1, instead of 216 points with three sines each on the FP64 pipe (2 per clock and
 // SM), and the differences u_h - u are formed before they are squared, as at the points. A 32^3, k = 1
 // solution takes 0.23 ms, 7.09 ms with the points. One thread per element in FP64, bound by the FP64 pipe; the L2
@@ -50,6 +50,12 @@ constexpr int kPostMaxRecon = 35;      // reconstruction basis functions (3D, de
 constexpr int kPostMaxPoints = 512;
 
 constexpr int kPostMaxGeometries = 256;   // distinct quadrature tables that are factorised (else: the points)
+// Tables that are factorised however few elements share them, and elements to a table above that. A table takes
+// 0.34 ms of one core in 3D, k = 1 (0.03 in 2D), on the first run with an exact solution; the points take 1.1 ms
+// there for 1,300 elements (a thread's 216 points one after another), 7.1 ms for 197,000, and the factors 0.05 and
+// 0.21 ms. So 32 tables on 16 cores repay themselves within that run, more of them from 500 elements each on: 13
+// tables of 10,368 elements: first run and set-up 1.31 ms against 1.43 at the points.
+constexpr int kPostFewTables = 32, kPostFactorElements = 512;
 
 struct PostData {
     int dim, ne, ncls, ngeo, nC, nFF, nF, nf, nR, nq;
@@ -181,48 +187,107 @@ __global__ void __launch_bounds__(kPostThreads) k_post_finish(const double* part
     }
 }
 
-// R of the QR factorisation (Householder) of sqrt(W) [Phi B] of one quadrature table, in extended
-// precision so that R adds no more than its own rounding to FP64; column m < 2^dim of Phi is the product
+// Numbers of 106 bits as a sum of two doubles (Dekker 1971), on the host: the same results on every machine,
+// and ten times faster than a long double where that is emulated.
+struct Dd {
+    double h, l;
+};
+inline Dd dd_fast(double a, double b) { const double s = a + b; return {s, b - (s - a)}; }   // |a| >= |b|
+inline Dd operator+(Dd a, Dd b)
+{
+    const double s = a.h + b.h, t = s - a.h;
+    return dd_fast(s, ((a.h - (s - t)) + (b.h - t)) + (a.l + b.l));
+}
+inline Dd operator-(Dd a, Dd b) { return a + Dd{-b.h, -b.l}; }
+inline Dd operator*(Dd a, Dd b)
+{
+    const double p = a.h * b.h;
+    return dd_fast(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+inline Dd operator/(Dd a, Dd b)
+{
+    const double q = a.h / b.h;
+    return dd_fast(q, (a - b * Dd{q, 0.0}).h / b.h);
+}
+inline Dd dd_sqrt(double a)
+{
+    const double s = std::sqrt(a);
+    return s > 0.0 ? dd_fast(s, (Dd{a, 0.0} - Dd{s, 0.0} * Dd{s, 0.0}).h / (2.0 * s)) : Dd{s, 0.0};
+}
+
+// sin(pi o) and cos(pi o): o = 2 m + n / 2 + f exactly, |f| <= 1/4, and the Taylor series of pi f to
+// y^22 / 22! (5e-24).
+void dd_sincospi(double o, Dd& sn, Dd& cs)
+{
+    constexpr int kTerms = 11;
+    const Dd pi = {3.141592653589793, 1.2246467991473532e-16};
+    const double r = o - 2.0 * std::round(0.5 * o), n = std::round(2.0 * r), f = r - 0.5 * n;
+    const Dd y = pi * Dd{f, 0.0}, y2 = y * y;
+    Dd s = {1.0, 0.0}, c = {1.0, 0.0};   // Horner: 1 - y^2 / ((k - 1) k) (1 - ...)
+    for (int k = 2 * kTerms; k > 0; k -= 2) {
+        c = Dd{1.0, 0.0} - y2 * c / Dd{(double)(k - 1) * k, 0.0};
+        s = Dd{1.0, 0.0} - y2 * s / Dd{(double)k * (k + 1), 0.0};
+    }
+    s = s * y;
+    const Dd ms = {-s.h, -s.l}, mc = {-c.h, -c.l};
+    switch ((int)n & 3) {
+    case 0: sn = s; cs = c; break;
+    case 1: sn = c; cs = ms; break;
+    case 2: sn = ms; cs = mc; break;
+    default: sn = mc; cs = s; break;
+    }
+}
+
+// sum over q of a[q] b[q], four sums side by side.
+inline Dd dd_dot(const Dd* a, const Dd* b, int n)
+{
+    Dd t[4] = {};
+    int q = 0;
+    for (; q + 4 <= n; q += 4)
+        for (int u = 0; u < 4; u++) t[u] = t[u] + a[q + u] * b[q + u];
+    for (; q < n; q++) t[0] = t[0] + a[q] * b[q];
+    return (t[0] + t[1]) + (t[2] + t[3]);
+}
+
+// R of the QR factorisation (Householder) of sqrt(W) [Phi B] of one quadrature table, in pairs of doubles
+// so that R adds no more than its own rounding to FP64; column m < 2^dim of Phi is the product
 // over d of sin(pi o_d) (bit d of m set) or cos(pi o_d). Rows past the number of points are zero.
 void factor_table(int dim, int nq, int nR, const double* w, const double* off, const double* basis, double* R)
 {
-    typedef long double ld;
-    const ld pi = 3.14159265358979323846264338327950288L;
     const int M = 1 << dim, nv = M + nR;
-    std::vector<ld> A((size_t)nv * nq);   // column-major
+    std::vector<Dd> A((size_t)nv * nq);   // column-major
     for (int q = 0; q < nq; q++) {
-        const ld sw = std::sqrt((ld)w[q]);
-        ld s[3], c[3];
-        for (int d = 0; d < dim; d++) {
-            s[d] = std::sin(pi * (ld)off[q * 3 + d]);
-            c[d] = std::cos(pi * (ld)off[q * 3 + d]);
-        }
+        const Dd sw = dd_sqrt(w[q]);
+        Dd s[3], c[3];
+        for (int d = 0; d < dim; d++) dd_sincospi(off[q * 3 + d], s[d], c[d]);
         for (int m = 0; m < M; m++) {
-            ld v = sw;
-            for (int d = 0; d < dim; d++) v *= (m >> d & 1) ? s[d] : c[d];
+            Dd v = sw;
+            for (int d = 0; d < dim; d++) v = v * ((m >> d & 1) ? s[d] : c[d]);
             A[(size_t)m * nq + q] = v;
         }
-        for (int i = 0; i < nR; i++) A[(size_t)(M + i) * nq + q] = sw * (ld)basis[(size_t)q * nR + i];
+        for (int i = 0; i < nR; i++) A[(size_t)(M + i) * nq + q] = sw * Dd{basis[(size_t)q * nR + i], 0.0};
     }
     for (int k = 0; k < std::min(nv, nq); k++) {
-        ld* a = &A[(size_t)k * nq];
-        ld nn = 0;
-        for (int q = k; q < nq; q++) nn += a[q] * a[q];
-        const ld alpha = a[k] > 0 ? -std::sqrt(nn) : std::sqrt(nn);
-        const ld v0 = a[k] - alpha, vv = nn - alpha * a[k];   // v = a - alpha e_k, v.v / 2 = nn - alpha a_k
-        if (vv > 0)
+        Dd* a = &A[(size_t)k * nq];
+        const Dd nn = dd_dot(a + k, a + k, nq - k);
+        Dd alpha = {0.0, 0.0};
+        if (!(nn.h <= 0.0)) {
+            const Dd root = dd_sqrt(nn.h);   // of the pair: one Newton step more
+            alpha = root + (nn - root * root) / Dd{2.0 * root.h, 0.0};
+            if (a[k].h > 0.0) alpha = Dd{-alpha.h, -alpha.l};
+        }
+        const Dd vv = nn - alpha * a[k];   // v = a - alpha e_k, v.v / 2 = nn - alpha a_k
+        a[k] = a[k] - alpha;
+        if (!(vv.h <= 0.0))
             for (int j = k + 1; j < nv; j++) {
-                ld* b = &A[(size_t)j * nq];
-                ld dot = v0 * b[k];
-                for (int q = k + 1; q < nq; q++) dot += a[q] * b[q];
-                dot /= vv;
-                b[k] -= dot * v0;
-                for (int q = k + 1; q < nq; q++) b[q] -= dot * a[q];
+                Dd* b = &A[(size_t)j * nq];
+                const Dd dot = dd_dot(a + k, b + k, nq - k) / vv;
+                for (int q = k; q < nq; q++) b[q] = b[q] - dot * a[q];
             }
         a[k] = alpha;
     }
     for (int r = 0; r < nv; r++)
-        for (int m = 0; m < nv; m++) R[(size_t)r * nv + m] = r < nq && m >= r ? (double)A[(size_t)m * nq + r] : 0.0;
+        for (int m = 0; m < nv; m++) R[(size_t)r * nv + m] = r < nq && m >= r ? A[(size_t)m * nq + r].h : 0.0;
 }
 
 }  // namespace
@@ -236,6 +301,10 @@ struct fhg_post {
     double* sums = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    // The distinct quadrature tables (weights, offsets, basis values) and each class's, held until the first
+    // run with an exact solution factorises them; empty when the points are used.
+    std::vector<double> w, off, basis;
+    std::vector<int> geo;
 };
 
 namespace {
@@ -268,30 +337,40 @@ int upload(fhg_post* p, const T* host, size_t n, const T** dev)
     return FHG_OK;
 }
 
-// A table of n entries per class, given class by class, entry by entry (entry e of class c at
-// e * classes + c).
-int upload_interleaved(fhg_post* p, const double* host, size_t classes, size_t n, const double** dev)
+// A table of n entries per class, given class by class (of = null) or table by table (class c's is of[c]),
+// entry by entry (entry e of class c at e * classes + c).
+int upload_interleaved(fhg_post* p, const double* host, size_t classes, size_t n, const double** dev, const int* of = nullptr)
 {
     std::vector<double> t(classes * n);
     for (size_t c = 0; c < classes; c++)
-        for (size_t e = 0; e < n; e++) t[e * classes + c] = host[c * n + e];
+        for (size_t e = 0; e < n; e++) t[e * classes + c] = host[(of ? (size_t)of[c] : c) * n + e];
     return upload(p, t.data(), t.size(), dev);
 }
 
-// The factorised quadrature tables: classes with the same weights, offsets and basis values share one
-// (coefficients change an element's operators, not its quadrature), found by hashing. Leaves D.R null
-// (evaluation at the points) when there are more than kPostMaxGeometries or a weight is negative: a
-// factorisation takes about 5 ms of one core in 3D, k = 1, more than the points of a few hundred elements.
-int upload_factors(fhg_post* p, int nc, const double* weights, const double* offsets, const double* basis)
+int upload_points(fhg_post* p, const double* weights, const double* offsets, const double* basis, const int* of = nullptr)
 {
     PostData& D = p->D;
-    const size_t nq = D.nq, nR = D.nR;
-    for (size_t i = 0; i < (size_t)nc * nq; i++)
-        if (!(weights[i] >= 0.0)) return FHG_OK;
-    std::vector<int> geo(nc), rep;
-    std::vector<size_t> hash;
+    const size_t nc = D.ncls, nq = D.nq;
+    int rc;
+    if ((rc = upload_interleaved(p, weights, nc, nq, &D.w, of)) || (rc = upload_interleaved(p, offsets, nc, nq * 3, &D.off, of)))
+        return rc;
+    return upload_interleaved(p, basis, nc, nq * D.nR, &D.basis, of);
+}
+
+// The distinct quadrature tables: classes with the same weights, offsets and basis values share one
+// (coefficients change an element's operators, not its quadrature), found by hashing. Left in p for factorise
+// where they repay it (kPostFewTables) and no weight is negative; false: the points are used.
+bool distinct_tables(fhg_post* p, const double* weights, const double* offsets, const double* basis)
+{
+    const PostData& D = p->D;
+    const size_t nc = D.ncls, nq = D.nq, nR = D.nR;
+    const size_t limit = std::min(kPostMaxGeometries, std::max(kPostFewTables, D.ne / kPostFactorElements));
+    for (size_t i = 0; i < nc * nq; i++)
+        if (!(weights[i] >= 0.0)) return false;
+    std::vector<int> geo(nc);
+    std::vector<size_t> hash, rep;
     auto same = [](const double* a, const double* b, size_t n) { return std::memcmp(a, b, sizeof(double) * n) == 0; };
-    for (int c = 0; c < nc; c++) {
+    for (size_t c = 0; c < nc; c++) {
         const double *w = weights + c * nq, *o = offsets + c * nq * 3, *B = basis + c * nq * nR;
         size_t h = 1469598103934665603ull;
         for (const auto& [t, n] : {std::pair<const double*, size_t>{w, nq}, {o, nq * 3}, {B, nq * nR}})
@@ -307,41 +386,63 @@ int upload_factors(fhg_post* p, int nc, const double* weights, const double* off
                 same(basis + rep[k] * nq * nR, B, nq * nR))
                 g = (int)k;
         if (g < 0) {
-            if ((int)rep.size() == kPostMaxGeometries) return FHG_OK;
+            if (rep.size() == limit) return false;
             g = (int)rep.size();
             rep.push_back(c);
             hash.push_back(h);
         }
         geo[c] = g;
     }
-    const size_t nv = (size_t)(1 << D.dim) + nR;
-    std::vector<double> R(rep.size() * nv * nv);
+    for (size_t c : rep) {
+        p->w.insert(p->w.end(), weights + c * nq, weights + (c + 1) * nq);
+        p->off.insert(p->off.end(), offsets + c * nq * 3, offsets + (c + 1) * nq * 3);
+        p->basis.insert(p->basis.end(), basis + c * nq * nR, basis + (c + 1) * nq * nR);
+    }
+    p->geo = std::move(geo);
+    return true;
+}
+
+// The factors of the distinct tables, on the host's threads; where one is not finite, the points. The tables held
+// for it are given back.
+int factorise(fhg_post* p)
+{
+    PostData& D = p->D;
+    const size_t nq = D.nq, nR = D.nR, nv = (size_t)(1 << D.dim) + nR, tables = p->w.size() / nq;
+    std::vector<double> R(tables * nv * nv);
     std::atomic<size_t> next{0};
-    std::atomic<bool> no_memory{false};
+    std::atomic<bool> bad{false};
     auto work = [&]() {
         try {
-            for (size_t k = next++; k < rep.size(); k = next++)
-                factor_table(D.dim, (int)nq, (int)nR, weights + rep[k] * nq, offsets + rep[k] * nq * 3,
-                             basis + rep[k] * nq * nR, &R[k * nv * nv]);
+            for (size_t k = next++; k < tables; k = next++)
+                factor_table(D.dim, (int)nq, (int)nR, &p->w[k * nq], &p->off[k * nq * 3], &p->basis[k * nq * nR], &R[k * nv * nv]);
         } catch (const std::bad_alloc&) {
-            no_memory = true;
+            bad = true;
         }
     };
     std::vector<std::thread> th;
-    const size_t nt = std::min<size_t>(rep.size(), std::max(1u, std::min(32u, std::thread::hardware_concurrency())));
+    const size_t nt = std::min<size_t>(tables, std::max(1u, std::min(32u, std::thread::hardware_concurrency())));
+    th.reserve(nt);   // no allocation between the first thread and the joins
     try {
         for (size_t t = 1; t < nt; t++) th.emplace_back(work);
-    } catch (const std::system_error&) {
+    } catch (...) {
         // no more threads to be had: those that run and this one share the tables
     }
     work();
     for (auto& t : th) t.join();
-    if (no_memory) return FHG_OK;
-    for (double v : R)
-        if (!std::isfinite(v)) return FHG_OK;
-    D.ngeo = (int)rep.size();
-    int rc = upload(p, geo.data(), geo.size(), &D.geo);
-    return rc ? rc : upload_interleaved(p, R.data(), rep.size(), nv * nv, &D.R);
+    for (double v : R) bad = bad || !std::isfinite(v);
+    int rc;
+    if (bad) {
+        if ((rc = upload_points(p, p->w.data(), p->off.data(), p->basis.data(), p->geo.data()))) return rc;
+    } else {
+        const double* dev = nullptr;
+        if ((rc = upload(p, p->geo.data(), p->geo.size(), &D.geo)) || (rc = upload_interleaved(p, R.data(), tables, nv * nv, &dev)))
+            return rc;
+        D.ngeo = (int)tables;
+        D.R = dev;
+    }
+    for (auto* t : {&p->w, &p->off, &p->basis}) std::vector<double>().swap(*t);
+    std::vector<int>().swap(p->geo);
+    return FHG_OK;
 }
 
 typedef void (*PostKernel)(PostData, const double*, double*, int, double*);
@@ -400,13 +501,9 @@ int fhg_post_create(fhg_post** out, int device, int dim, int n_elements, int n_c
         if ((rc = upload(p, elem_class, ne, &D.cls)) || (rc = upload(p, elem_faces, ne * D.nF, &D.faces)) ||
             (rc = upload(p, elem_centre, ne * 3, &D.centre)) || (rc = upload(p, cell_rhs, ne * n_cell, &D.cell_rhs)) ||
             (rc = upload_interleaved(p, solve_cells, nc, (size_t)n_cell * n_face_dofs, &D.sc)) ||
-            (rc = upload_interleaved(p, recon, nc, (size_t)n_recon * (n_cell + n_face_dofs), &D.rc)) ||
-            (rc = upload_factors(p, n_classes, weights, offsets, basis)))
+            (rc = upload_interleaved(p, recon, nc, (size_t)n_recon * (n_cell + n_face_dofs), &D.rc)))
             return rc;
-        if (!D.R && ((rc = upload_interleaved(p, weights, nc, n_points, &D.w)) ||
-                     (rc = upload_interleaved(p, offsets, nc, (size_t)n_points * 3, &D.off)) ||
-                     (rc = upload_interleaved(p, basis, nc, (size_t)n_points * n_recon, &D.basis))))
-            return rc;
+        if (!distinct_tables(p, weights, offsets, basis) && (rc = upload_points(p, weights, offsets, basis))) return rc;
     } catch (const std::bad_alloc&) {
         return post_fail(p, FHG_ERR_TOO_LARGE, "out of host memory for the element tables");
     }
@@ -428,6 +525,14 @@ int fhg_post_run(fhg_post* p, const double* x_faces, double* x_cells, int exact,
     if (exact != FHG_EXACT_NONE && exact != FHG_EXACT_SINE) return post_fail(p, FHG_ERR_INVALID_ARG, "unknown exact solution %d", exact);
     if (exact == FHG_EXACT_SINE && !rel_l2_error) return post_fail(p, FHG_ERR_INVALID_ARG, "null error output");
     PCK(cudaSetDevice(p->device));
+    if (exact == FHG_EXACT_SINE && !p->geo.empty()) {
+        try {
+            const int rc = factorise(p);
+            if (rc) return rc;
+        } catch (const std::bad_alloc&) {
+            return post_fail(p, FHG_ERR_TOO_LARGE, "out of host memory for the element tables");
+        }
+    }
     const int grid = (int)std::min<long long>(kPostMaxCtas, ((long long)p->D.ne + kPostThreads - 1) / kPostThreads);
     PCK(cudaEventRecord(p->ev0, p->stream));
     post_kernel(p->D)<<<grid, kPostThreads, 0, p->stream>>>(p->D, x_faces, x_cells, exact, p->partials);
@@ -448,6 +553,8 @@ int fhg_post_run(fhg_post* p, const double* x_faces, double* x_cells, int exact,
     }
     return FHG_OK;
 }
+
+int fhg_post_factors(const fhg_post* p) { return p ? p->D.ngeo : 0; }
 
 const char* fhg_post_last_error(const fhg_post* p) { return p ? p->err.c_str() : "null post-processing handle"; }
 

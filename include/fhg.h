@@ -374,6 +374,9 @@ int fhg_post_create(fhg_post** post, int device, int dim, int n_elements, int n_
  * time (CUDA events) or null. */
 int fhg_post_run(fhg_post* post, const double* x_faces, double* x_cells, int exact, double* rel_l2_error,
                  double* elapsed_ms);
+/* Quadrature tables factorised so far: 0 before the first run with an exact solution, and where the sums go over
+ * the quadrature points. */
+int fhg_post_factors(const fhg_post* post);
 const char* fhg_post_last_error(const fhg_post* post);
 void fhg_post_destroy(fhg_post* post);
 

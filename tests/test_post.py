@@ -168,3 +168,46 @@ def test_gpu_post_with_factorised_and_pointwise_tables(dim, n, k, tables):
         post.close()
     assert np.abs(cells.cpu().numpy().reshape(xc_ref.shape) - xc_ref).max() <= 1e-12 * np.abs(xc_ref).max()
     assert err == pytest.approx(err_ref, rel=1e-12)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,n,k,tables", [(2, 16, 1, None), (3, 6, 1, None), (3, 6, 2, None), (3, 2, 3, 31), (3, 2, 1, 32),
+                                            (3, 3, 1, 33), (2, 12, 1, 288), (2, 96, 2, 33), (2, 96, 1, 200)])
+def test_gpu_post_factorises_on_the_first_exact_run_where_that_repays(dim, n, k, tables):
+    """Quadrature tables are factorised by the first run with an exact solution, not at set-up and not for the cell
+    unknowns alone, and only where they are few (32) or have 512 elements each; both forms against numpy at the
+    points. `tables`: that many rules of weights in turn (None: the mesh's own few). 1e-12: sums of positive terms."""
+    import torch
+    from fhhos4_gb300 import _native as N
+    H = hho.Hierarchy(dim, n, k, max_levels=1)
+    try:
+        t = H.post_tables()
+        rows = H.A_rows(0)
+    finally:
+        H.close()
+    ne, nq = t["n_elements"], t["n_points"]
+    if tables:   # every element of one geometry, so that the weights alone tell the tables apart
+        cls = np.zeros(ne, np.int32)
+        for name, m in (("solve_cells", t["n_cell"] * t["n_face_dofs"]), ("recon", t["n_recon"] * (t["n_cell"] + t["n_face_dofs"])),
+                        ("offsets", nq * 3), ("basis", nq * t["n_recon"]), ("weights", nq)):
+            t[name] = np.repeat(t[name].reshape(-1, m)[:1], tables, axis=0)
+        t["weights"] *= 1.0 + 1e-3 * np.arange(tables)[:, None]
+        t["n_classes"], t["elem_class"] = tables, (cls + np.arange(ne) % tables).astype(np.int32)
+    expect = (tables or t["n_classes"]) if not tables or tables <= 32 or ne >= 512 * tables else 0
+    x = np.random.default_rng(3).standard_normal(rows)
+    xc_ref, err_ref = numpy_post(t, x)
+    post = N.Post({k_: (v.ravel() if isinstance(v, np.ndarray) else v) for k_, v in t.items()})
+    try:
+        assert post.factors() == 0
+        xd = torch.tensor(x, device="cuda")
+        cells = torch.zeros(ne * t["n_cell"], dtype=torch.float64, device="cuda")
+        post.run(xd.data_ptr(), cells.data_ptr(), "none")
+        assert post.factors() == 0
+        assert np.abs(cells.cpu().numpy().reshape(xc_ref.shape) - xc_ref).max() <= 1e-12 * np.abs(xc_ref).max()
+        err, _ = post.run(xd.data_ptr(), 0, "sine")
+        assert 0 < post.factors() <= expect if expect else post.factors() == 0
+        assert tables is None or post.factors() == expect
+        assert err == pytest.approx(err_ref, rel=1e-12)
+        assert post.run(xd.data_ptr(), 0, "sine")[0] == err
+    finally:
+        post.close()
