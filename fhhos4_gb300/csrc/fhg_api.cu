@@ -997,13 +997,15 @@ int choose_fused(fhg_ctx* ctx)
     const int bs = ctx->levels[first].bs;
     FusedKey key;
     key.sig = {PR, ctx->levels[0].bs, bs, nlevels, o.pre_smoother, o.post_smoother, o.pre_iterations, o.post_iterations,
-               o.coarse_pre_iterations, o.coarse_post_iterations, o.w_loops, o.omega == 1.0 ? 1 : 0};
+               o.coarse_pre_iterations, o.coarse_post_iterations, o.w_loops, o.omega == 1.0 ? 1 : 0, o.gs_layout};
+    // and the forms that the launch-by-launch cycle runs on: row classes depend on values, not on structure
     for (int l = 1; l < nlevels; l++) {
-        const Level& L = ctx->levels[l];
-        key.sig.push_back(L.nb);
-        key.sig.push_back(L.bs);
-        key.sig.push_back(L.ncolours);
-        key.sig.push_back(V::Acsr(const_cast<Level&>(L)).nnzb);
+        Level& L = ctx->levels[l];
+        const bool transfers = l + 1 < nlevels && !L.inject;
+        for (long long v : {(long long)L.nb, (long long)L.bs, (long long)L.ncolours, V::Acsr(L).nnzb,
+                            (long long)(V::gs(L).cls != nullptr), (long long)L.gs_slot[PR], (long long)L.prod_slot[PR],
+                            (long long)(transfers && V::P(L).sell_perm), (long long)(transfers && V::R(L).sell_perm)})
+            key.sig.push_back(v);
     }
     {
         std::lock_guard<std::mutex> lock(g_fused_mutex);
@@ -2787,6 +2789,25 @@ int fhg_fused_coarse_info(const fhg_ctx* ctx, int precision, int* first_level, i
     if (first_level) *first_level = ctx->fused_from[precision];
     if (cluster_ctas) *cluster_ctas = ctx->fused_ctas[precision];
     if (cta_threads) *cta_threads = ctx->fused_threads[precision];
+    return FHG_OK;
+}
+
+int fhg_view_info(const fhg_ctx* ctx, int level, int precision, int* classes, int* slots, int* p_lanes, int* r_lanes)
+{
+    if (!ctx || !ctx->ready || level < 0 || level >= ctx->nlevels || precision < 0 || precision > 2) return FHG_ERR_INVALID_ARG;
+    Level& L = const_cast<Level&>(ctx->levels[level]);
+    auto info = [&](auto t) {
+        using V = LevelVecs<decltype(t)>;
+        const auto& A = V::gs(L);
+        const bool transfers = level + 1 < ctx->nlevels && !L.inject;
+        if (classes) *classes = A.cls ? (int)A.ld : 0;
+        if (slots) *slots = A.cls ? A.ell : 0;
+        if (p_lanes) *p_lanes = transfers && V::P(L).sell_perm ? V::P(L).sell_lanes : 0;
+        if (r_lanes) *r_lanes = transfers && V::R(L).sell_perm ? V::R(L).sell_lanes : 0;
+    };
+    if (precision == FHG_PREC_FP32) info(float());
+    else if (precision == FHG_PREC_DF) info(dfl());
+    else info(double());
     return FHG_OK;
 }
 

@@ -244,6 +244,10 @@ int fhg_level_info(const fhg_ctx* ctx, int level, int* n_block_rows, long long* 
  * cluster and the threads of each CTA. Any pointer may be NULL. No counterpart in the reference. */
 int fhg_fused_coarse_info(const fhg_ctx* ctx, int precision, int* first_level, int* cluster_ctas,
                           int* cta_threads);
+/* The storage that a V-cycle in `precision` reads on a level: the row classes of its sweeps and products (0: stored
+ * blocks) and their off-diagonal slots, and the threads per row of the sliced transfers to the next level (0: CSR or
+ * none). Any pointer may be NULL. */
+int fhg_view_info(const fhg_ctx* ctx, int level, int precision, int* classes, int* slots, int* p_lanes, int* r_lanes);
 
 /* The colour permutation of `level` after setup: perm[new_block_row] = given_block_row. */
 int fhg_get_permutation(const fhg_ctx* ctx, int level, int* perm);
