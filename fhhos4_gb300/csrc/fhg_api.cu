@@ -1013,7 +1013,9 @@ int choose_fused(fhg_ctx* ctx)
     {
         std::lock_guard<std::mutex> lock(g_fused_mutex);
         auto it = g_fused_cache.find(key);
-        if (it != g_fused_cache.end()) {
+        // the kernel's opt-ins (cluster size, shared memory) hold for a device: made on this one too
+        if (it != g_fused_cache.end() &&
+            (it->second.from < 0 || fused_clusters<T>(ctx, it->second.from, it->second.ctas, it->second.threads) > 0)) {
             ctx->fused_from[PR] = it->second.from;
             ctx->fused_ctas[PR] = it->second.ctas;
             ctx->fused_threads[PR] = it->second.threads;
