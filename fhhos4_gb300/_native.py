@@ -40,7 +40,7 @@ LEARNED_PARAMS = 24848
 # Every symbol include/fhg.h declares.
 EXPORTS = ["fhg_default_options", "fhg_create", "fhg_destroy", "fhg_last_error", "fhg_set_level",
            "fhg_set_prolongation", "fhg_setup", "fhg_solve", "fhg_solve_device", "fhg_apply",
-           "fhg_time_op", "fhg_set_cycle", "fhg_set_coarse_smoothing", "fhg_set_vcycle_precision", "fhg_level_info", "fhg_fused_coarse_info", "fhg_view_info",
+           "fhg_time_op", "fhg_set_cycle", "fhg_set_coarse_smoothing", "fhg_set_vcycle_precision", "fhg_level_info", "fhg_fused_coarse_info", "fhg_set_fused_coarse", "fhg_view_info",
            "fhg_device_bytes", "fhg_get_permutation",
            "fhg_kernel_launches", "fhg_residual_norm_noalloc", "fhg_set_face_tensors", "fhg_set_learned",
            "fhg_learned_reference_rate", "fhg_learned_features", "fhg_apply_internal", "fhg_net_num_params",
@@ -105,6 +105,7 @@ def load(path: str = LIB):
     lib.fhg_set_cycle.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]
     lib.fhg_set_coarse_smoothing.argtypes = [C.c_void_p, C.c_int, C.c_int]
     lib.fhg_view_info.argtypes = [C.c_void_p, C.c_int, C.c_int] + [P(C.c_int)] * 4
+    lib.fhg_set_fused_coarse.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int]
     lib.fhg_fused_coarse_info.argtypes = [C.c_void_p, C.c_int, P(C.c_int), P(C.c_int), P(C.c_int)]
     lib.fhg_device_bytes.argtypes = [C.c_void_p]
     lib.fhg_device_bytes.restype = C.c_longlong
@@ -266,6 +267,11 @@ class Context:
         v = [C.c_int() for _ in range(4)]
         self._check(self.lib.fhg_view_info(self.h, level, PRECISION[precision], *map(C.byref, v)))
         return dict(zip(("classes", "slots", "p_lanes", "r_lanes"), (q.value for q in v)))
+
+    def set_fused_coarse(self, precision: str, first_level: int, cluster_ctas: int = 8, cta_threads: int = 512):
+        """Run the coarse sub-cycle from first_level down as one launch (-1: launch by launch) until setup or a
+        change of the cycle chooses again."""
+        self._check(self.lib.fhg_set_fused_coarse(self.h, PRECISION[precision], first_level, cluster_ctas, cta_threads))
 
     def permutation(self, level: int, nb: int) -> np.ndarray:
         perm = np.empty(nb, dtype=np.int32)

@@ -833,14 +833,23 @@ void kcycle_fcg(fhg_ctx* ctx, int m, T* r, T* x)
     fhg::launch_lincomb<T>(n, alpha1 / rho1 - gamma * alpha2 / (rho1 * rho2), c, alpha2 / rho2, d, x, s);
 }
 
-// Threads per block row of a phase of the one-launch sub-cycle: `each` blocks of the average row to a thread
-// (2 to 32 threads), but no more threads than leave the phase's rows in one pass of the cluster.
-int fused_lanes(double blocks_per_row, int each, int rows, int threads)
+// Threads per row of a phase of the one-launch sub-cycle: `each` of the average row's entries to a thread
+// (2 to 32 threads), but no more than leave the phase's rows in one pass of the cluster, and no fewer than `least`.
+int fused_lanes(double per_row, int each, int rows, int threads, int least)
 {
     int g = 2;
-    while (g < 32 && g * each < blocks_per_row) g *= 2;
-    while (g > 2 && (long long)rows * g > threads) g /= 2;
+    while (g < 32 && g * each < per_row) g *= 2;
+    while (g > least && (long long)rows * g > threads) g /= 2;
     return g;
+}
+
+// The least of a block row: a lane's blocks are summed one after another and the lanes' sums as a tree, so few
+// lanes on a long row round more. In pairs with the 40 blocks of a 2D Galerkin row on 2 lanes a cycle from 12,160
+// rows down was 1.5 times further from FP64 (2.4e-14) than launch by launch; on 16 lanes it is as near (1.5e-14),
+// for 564 us instead of 511 with 2 x 2 blocks in FP32, 1,028 instead of 1,431 with 4 x 4. Below 3,000 rows the same time.
+int fused_block_lanes(double blocks_per_row, int rows, int threads)
+{
+    return fused_lanes(blocks_per_row, 1, rows, threads, blocks_per_row <= 5.0 ? 4 : blocks_per_row <= 12.0 ? 8 : 16);
 }
 
 int largest_colour(const Level& L)
@@ -896,7 +905,7 @@ bool fused_cycle(fhg_ctx* ctx, int l, const T* b, T* x, bool x_zero)
             if (l + k == ctx->nlevels - 1) {
                 P.n_coarse = L.n;
                 P.cinv = L.cinv;
-                P.c_lanes = fused_lanes(L.n, 16, L.n, threads);
+                P.c_lanes = fused_lanes(L.n, 16, L.n, threads, 2);
                 continue;
             }
             F.ncol = L.ncolours;
@@ -908,10 +917,10 @@ bool fused_cycle(fhg_ctx* ctx, int l, const T* b, T* x, bool x_zero)
             F.p_rowptr = Pv.rowptr; F.p_colidx = Pv.colidx; F.p_vals = Pv.vals; F.p_ld = Pv.ld;
             const BsrView<T>& Rv = V::Rcsr(L);
             F.r_rowptr = Rv.rowptr; F.r_colidx = Rv.colidx; F.r_vals = Rv.vals; F.r_ld = Rv.ld;
-            F.lanes = fused_lanes(mean(A), 1, largest_colour(L), threads);
-            F.a_lanes = fused_lanes(mean(A), 1, L.nb, threads);
-            F.p_lanes = fused_lanes(mean(Pv), 1, L.nb, threads);
-            F.r_lanes = fused_lanes(mean(Rv), 1, Rv.nbr, threads);
+            F.lanes = fused_block_lanes(mean(A), largest_colour(L), threads);
+            F.a_lanes = fused_block_lanes(mean(A), L.nb, threads);
+            F.p_lanes = fused_block_lanes(mean(Pv), L.nb, threads);
+            F.r_lanes = fused_block_lanes(mean(Rv), Rv.nbr, threads);
         }
         const int smem = fhg::fused_layout<T>(P, ctx->levels[l].bs, ctas);
         if (smem < 0 || fhg::launch_fused_cycle<T>(P, ctx->levels[l].bs, ctas, cta_threads, smem, ctx->stream) != cudaSuccess)
@@ -2813,6 +2822,37 @@ int fhg_view_info(const fhg_ctx* ctx, int level, int precision, int* classes, in
     if (precision == FHG_PREC_FP32) info(float());
     else if (precision == FHG_PREC_DF) info(dfl());
     else info(double());
+    return FHG_OK;
+}
+
+// The sub-cycle of one precision from first_level (-1: launch by launch) with the given cluster, in place of what
+// setup chose, until setup or a change of the cycle chooses again.
+int fhg_set_fused_coarse(fhg_ctx* ctx, int precision, int first_level, int cluster_ctas, int cta_threads)
+{
+    if (!ctx) return FHG_ERR_INVALID_ARG;
+    if (!ctx->ready) return fail(ctx, FHG_ERR_NOT_READY, "fhg_setup has not completed");
+    if (precision != FHG_PREC_FP32 && precision != FHG_PREC_DF)
+        return fail(ctx, FHG_ERR_INVALID_ARG, "the coarse sub-cycle runs in FP32 and in pairs");
+    const fhg_options& o = ctx->opts;
+    const bool pair = precision == FHG_PREC_DF;
+    if (first_level >= 0) {
+        if (pair ? !ctx->levels[0].A2.vals : !ctx->levels[0].A32.vals)
+            return fail(ctx, FHG_ERR_NOT_READY, "operators of precision %d were not built", precision);
+        if (!o.fused_coarse || o.w_loops == FHG_CYCLE_K || !is_gs(o.pre_smoother) || !is_gs(o.post_smoother) ||
+            first_level < 1 || !fused_eligible(ctx, first_level))
+            return fail(ctx, FHG_ERR_UNSUPPORTED, "the coarse sub-cycle cannot start from level %d", first_level);
+        CK(cudaSetDevice(ctx->device));
+        if ((pair ? fused_clusters<dfl>(ctx, first_level, cluster_ctas, cta_threads)
+                  : fused_clusters<float>(ctx, first_level, cluster_ctas, cta_threads)) < 1)
+            return fail(ctx, FHG_ERR_UNSUPPORTED, "no cluster of %d CTAs of %d threads for level %d and below", cluster_ctas,
+                        cta_threads, first_level);
+        ctx->fused_ctas[precision] = cluster_ctas;
+        ctx->fused_threads[precision] = cta_threads;
+    }
+    free_graphs(ctx);
+    ctx->epoch++;
+    ctx->rho_plain = 0.0;
+    ctx->fused_from[precision] = first_level < 0 ? -1 : first_level;
     return FHG_OK;
 }
 

@@ -248,6 +248,10 @@ int fhg_fused_coarse_info(const fhg_ctx* ctx, int precision, int* first_level, i
  * blocks) and their off-diagonal slots, and the threads per row of the sliced transfers to the next level (0: CSR or
  * none). Any pointer may be NULL. */
 int fhg_view_info(const fhg_ctx* ctx, int level, int precision, int* classes, int* slots, int* p_lanes, int* r_lanes);
+/* Run the coarse sub-cycle of one precision (FP32 or DF) as one cluster launch of cluster_ctas (8, 16) CTAs of
+ * cta_threads (512, 1024) threads from first_level (>= 1) down, or launch by launch (-1), in place of what setup
+ * chose; holds until setup or a change of the cycle chooses again. FHG_ERR_UNSUPPORTED where it cannot run. */
+int fhg_set_fused_coarse(fhg_ctx* ctx, int precision, int first_level, int cluster_ctas, int cta_threads);
 
 /* The colour permutation of `level` after setup: perm[new_block_row] = given_block_row. */
 int fhg_get_permutation(const fhg_ctx* ctx, int level, int* perm);
