@@ -107,3 +107,54 @@ def test_gpu_prolongation_rounds_once_at_the_size_of_x(dim, n, k, precision):
     err = np.abs(out.cpu().numpy().astype(np.longdouble) - ref)
     assert np.all(err <= (1 + u) * u * (np.abs(ref) + (m + 1) * size)), float((err / (u * np.abs(ref) + m * u * size)).max())
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "df", "fp32"])
+@pytest.mark.parametrize("dim,n,k,p_lanes,r_lanes",
+                         [(2, 96, 1, 0, 8), (2, 112, 1, 1, 8), (2, 112, 2, 1, 8), (2, 106, 3, 1, 8), (2, 160, 1, 1, 4),
+                          (2, 160, 3, 1, 4), (3, 16, 1, 1, 8), (3, 24, 2, 1, 4), (3, 28, 1, 1, 4)])
+def test_gpu_transfers_run_on_the_sliced_views_of_their_sizes(dim, n, k, p_lanes, r_lanes, precision):
+    """The view that each size takes (P a thread per row from 32,768 rows, R four from 16,384 and eight from 4,096,
+    CSR below), and R r, x + P e on it."""
+    torch = pytest.importorskip("torch")
+    from fhhos4_gb300 import _native as N
+    from fhhos4_gb300 import solver as S
+    from test_gpu_parity import scalar_perm
+    import scipy.sparse as sp
+    H = hho.Hierarchy(dim, n, k, max_levels=2)
+    A, P, bs = H.A(0), H.P(0).tocsr(), H.block_size
+    H.close()
+    top = P.shape[1]
+    nb = top // bs
+    Q = sp.csr_matrix((np.ones(top), (np.arange(top), np.tile(np.arange(bs), nb))), shape=(top, bs))
+    ctx = S.fcg_mg([A, sp.identity(top, format="csr"), sp.identity(bs, format="csr")], [P, Q], bs, precision=precision,
+                   fused=False).Context()
+    info = ctx.view_info(0, precision)
+    assert (info["p_lanes"], info["r_lanes"]) == (p_lanes, r_lanes)
+    row = S.fcg_mg([A, sp.identity(top, format="csr"), sp.identity(bs, format="csr")], [P, Q], bs, precision=precision,
+                   fused=False, gs_layout="row").Context()
+    assert (row.view_info(0, precision)["p_lanes"], row.view_info(0, precision)["r_lanes"]) == (0, 0)
+    rng = np.random.default_rng(2)
+    pair = precision == "df"
+    dt = torch.float64 if precision == "fp64" else torch.float32
+
+    def put(v):
+        return torch.tensor(np.stack([v.astype(np.float32), 0 * v.astype(np.float32)], 1) if pair else v, dtype=dt, device="cuda")
+
+    def get(t):
+        a = t.cpu().numpy().astype(np.float64)
+        return a[:, 0] + a[:, 1] if pair else a
+
+    p0 = scalar_perm(ctx.permutation(0, A.shape[0] // bs), bs)
+    p1 = scalar_perm(ctx.permutation(1, nb), bs)
+    Pp = P[p0][:, p1]
+    rd, ed = put(rng.standard_normal(A.shape[0])), put(rng.standard_normal(top))
+    out, aux = torch.full_like(ed, float("nan")), torch.full_like(rd, float("nan"))
+    torch.cuda.synchronize()
+    ctx.apply_internal(0, N.OP_RESTRICT, precision, rd.data_ptr(), None, out.data_ptr())
+    ctx.apply_internal(0, N.OP_PROLONG_ADD, precision, ed.data_ptr(), rd.data_ptr(), aux.data_ptr())
+    r, e = get(rd), get(ed)
+    assert np.abs(get(out) - Pp.T @ r).max() <= TOL[precision] * (abs(Pp).T @ np.abs(r)).max()
+    assert np.abs(get(aux) - (r + Pp @ e)).max() <= TOL[precision] * (np.abs(r).max() + (abs(Pp) @ np.abs(e)).max())
+    ctx.close()
+    row.close()
