@@ -493,10 +493,14 @@ int upload_sell(fhg_ctx* ctx, const HostBsr& B, int lanes, DevBsr<T>& D)
 // at 47,616 the sliced one: 3.5 against 4.1 in FP32, 11.5 against 17.1 in FP64); the longer rows of R four, or
 // eight where there are fewer, down to kSellRowsR.
 constexpr int kSellRowsP = 32768, kSellRowsR4 = 16384, kSellRowsR = 4096;
+// In pairs with blocks of up to 3 x 3 the rows of R take a thread each where they are many: 64^3, k = 1, 387,072
+// rows, 239 us against 246 with four lanes (FP32 134 against 131; 48^3, 162,432 rows, pairs 108 against 104).
+constexpr int kSellRowsR1 = 262144;
 
-int sell_lanes(const HostBsr& M, bool prolongation)
+int sell_lanes(const HostBsr& M, bool prolongation, bool pair)
 {
     if (prolongation) return M.nbr >= kSellRowsP ? 1 : 0;
+    if (pair && M.bs <= 3 && M.nbr >= kSellRowsR1) return 1;
     return M.nbr >= kSellRowsR4 ? 4 : M.nbr >= kSellRowsR ? 8 : 0;
 }
 
@@ -2268,11 +2272,14 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                 // and 1 with FHG_GS_SLOT (P with a thread per row, which adds; FP32 and pairs).
                 const bool slot = o.gs_layout == FHG_GS_SLOT;
                 auto sliced = [&](const HostBsr& M, bool prolongation, bool* use, auto& d64, auto& d32, auto& d2) -> int {
-                    const int lanes = slot ? (l <= 1 ? 1 : 0) : o.gs_layout == FHG_GS_ROW ? 0 : sell_lanes(M, prolongation);
+                    auto by_rule = [&](bool in_pairs) {
+                        return slot ? (l <= 1 ? 1 : 0) : o.gs_layout == FHG_GS_ROW ? 0 : sell_lanes(M, prolongation, in_pairs);
+                    };
+                    const int lanes = by_rule(false);
                     if (lanes == 0) return FHG_OK;
                     if (o.vcycle_precision == FHG_PREC_FP64 && !slot && (rc = upload_sell(ctx, M, lanes, d64))) return rc;
                     if (fp32 && (rc = upload_sell(ctx, M, lanes, d32))) return rc;
-                    if (pair && (rc = upload_sell(ctx, M, lanes, d2))) return rc;
+                    if (pair && (rc = upload_sell(ctx, M, by_rule(true), d2))) return rc;
                     for (int q = 0; q < 3; q++) use[q] = true;
                     return FHG_OK;
                 };

@@ -368,9 +368,11 @@ __global__ void __launch_bounds__(kThreads) k_bsr_spmv(int nbr, const int* __res
 // a slice adds (a few percent, the rows being sorted by length in windows of kSellWindow; the windows keep a
 // slice's output rows within a few cache lines of each other). Few lanes: in FP64 a lane group's shuffle
 // adds cost the pipe as much as its products. The columns of the next kGroup blocks are loaded ahead of the
-// sums over the present ones. Against CSR rows of 8 (P) and 32 (R) lanes, or of the tuned lanes at 64^3: x += P e FP64
-// 32^3 124 -> 45 us, FP32 64^3 183 -> 125 us (0.9 of HBM), pairs 48^3 122 -> 96; R r FP64 32^3 118 -> 43,
-// FP32 64^3 148 -> 131, 32^3 23 -> 12, 24^3 k = 2 45 -> 30, pairs 48^3 113 -> 104.
+// sums over the present ones. A lane's running sum in pairs is normalised every second product: left as it is, its
+// low part gathers the errors of a dozen blocks and rounds at their size (R r 1.4 to 3 times further off than with a
+// warp a row; so, 0.9 to 1.1 times). Against CSR rows of 8 (P) and 32 (R) lanes, or of the tuned lanes at 64^3: x += P e
+// FP64 32^3 124 -> 47 us, FP32 64^3 183 -> 128 us (0.9 of HBM), pairs 48^3 122 -> 96; R r FP64 32^3 118 -> 43,
+// FP32 64^3 148 -> 130, 32^3 23 -> 12, 24^3 k = 2 45 -> 30, pairs 48^3 113 -> 104.
 template <class T, int BS, int MODE, int L>
 __global__ void __launch_bounds__(kThreads) k_bsr_spmv_sell(int slices, const int* __restrict__ perm,
                                                             const int* __restrict__ ptr,
@@ -379,7 +381,10 @@ __global__ void __launch_bounds__(kThreads) k_bsr_spmv_sell(int slices, const in
                                                             const T* __restrict__ x, const T* aux, T* y)
 {
     constexpr int kBlockBytes = BS * BS * (int)sizeof(T);
-    constexpr int kGroup = kBlockBytes <= 36 ? 4 : kBlockBytes <= 72 ? 2 : 1;   // blocks in flight: ~144 bytes
+    // blocks in flight: ~144 bytes; a thread a row of R, whose rows are long, takes twice that (pairs 64^3, 387,072
+    // rows: 246 -> 239 us)
+    constexpr bool kLong = L == 1 && MODE == kSpmvAssign;
+    constexpr int kGroup = kBlockBytes <= (kLong ? 72 : 36) ? 4 : kBlockBytes <= 72 ? 2 : 1;
     const int slice = (int)((blockIdx.x * kThreads + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (slice >= slices) return;   // whole warps
     const int row = perm[slice * (32 / L) + lane / L];
@@ -412,7 +417,10 @@ __global__ void __launch_bounds__(kThreads) k_bsr_spmv_sell(int slices, const in
 #pragma unroll
                 for (int r = 0; r < BS; r++)
 #pragma unroll
-                    for (int c = 0; c < BS; c++) acc[r] = fma(v[g][r * BS + c], xv[g][c], acc[r]);
+                    for (int c = 0; c < BS; c++) {
+                        acc[r] = fma(v[g][r * BS + c], xv[g][c], acc[r]);
+                        if (c % 2 || c + 1 == BS) acc[r] = fin(acc[r]);
+                    }
             }
             col[g] = next;
         }
