@@ -165,6 +165,79 @@ def test_gpu_solves_on_class_views_track_stored_blocks(dim, n, k, precision):
         s.Context().close()
 
 
+def _grid(dims, m, bs):
+    """A block operator on a grid of m points a side: one block per direction, a dominant diagonal block (equal
+    rows but at the boundary)."""
+    rng = np.random.default_rng(9)
+    nb = m ** dims
+    ids = np.arange(nb).reshape((m,) * dims)
+    A = sp.kron(sp.identity(nb), np.eye(bs) * 2.0 * dims + 0.5 * np.diag(rng.random(bs))).tocsr()
+    for d in range(dims):
+        B = -np.eye(bs) + 0.3 * rng.uniform(-1, 1, (bs, bs))
+        lo, hi = np.take(ids, range(m - 1), d).ravel(), np.take(ids, range(1, m), d).ravel()
+        E = sp.csr_matrix((np.ones(len(lo)), (lo, hi)), shape=(nb, nb))
+        A = A + 0.9 * (sp.kron(E, B) + sp.kron(E.T, B.T))
+    A = A.tocsr()
+    A.sort_indices()
+    return A
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "df", "fp32"])
+@pytest.mark.parametrize("dims,m,bs", [(3, 11, 2), (3, 38, 2), (3, 11, 4), (3, 38, 4), (2, 37, 6), (2, 230, 6),
+                                       (3, 11, 3), (3, 11, 6), (2, 37, 2)])
+def test_gpu_class_kernels_of_every_block_size_and_width(dims, m, bs, precision):
+    """Block sizes and slot counts that no generated mesh brings (2 and 4 with 6 neighbours, 6 with 4), with one output
+    per lane and with a thread per row: products, sweeps, the outer product, and a sweep from zero (through the
+    cycle; P of zeros, so the coarse correction vanishes) against the oracle."""
+    torch = pytest.importorskip("torch")
+    from fhhos4_gb300 import _native as N
+    from fhhos4_gb300 import solver as S
+    from test_gpu_parity import scalar_perm
+    A = _grid(dims, m, bs)
+    nb, n = m ** dims, A.shape[0]
+    P = sp.csr_matrix((np.zeros(n), (np.arange(n), np.tile(np.arange(bs), nb))), shape=(n, bs))
+    rng = np.random.default_rng(21)
+
+    def put(v):
+        if precision == "df":
+            hi = v.astype(np.float32)
+            return torch.tensor(np.stack([hi, (v - hi).astype(np.float32)], 1), device="cuda")
+        return torch.tensor(v.astype(PREC[precision][0]), device="cuda")
+
+    def get(t):
+        a = t.cpu().numpy().astype(np.float64)
+        return a[:, 0] + a[:, 1] if precision == "df" else a
+
+    tol = PREC[precision][1]
+    for pre, op in (("bgs", N.OP_GS_FORWARD), ("rbgs", N.OP_GS_BACKWARD)):
+        ctx = S.fcg_mg([A, sp.identity(bs, format="csr")], [P], bs, precision=precision, pre=pre, nu=(1, 0)).Context()
+        info = ctx.view_info(0, precision)
+        assert info["classes"] == 3 ** dims and info["slots"] == 2 * dims
+        s = scalar_perm(ctx.permutation(0, nb), bs)
+        Ap = O.as_csr(A[s][:, s])
+        xd, bd = put(rng.standard_normal(n)), put(rng.standard_normal(n))
+        x, b = get(xd), get(bd)
+        scale = abs(Ap).sum(axis=1).max() * np.abs(x).max() + np.abs(b).max()
+        out = torch.empty_like(xd)
+        ctx.apply_internal(0, N.OP_SPMV, precision, xd.data_ptr(), None, out.data_ptr())
+        assert np.abs(get(out) - Ap @ x).max() <= tol * scale
+        ctx.apply_internal(0, N.OP_RESIDUAL, precision, xd.data_ptr(), bd.data_ptr(), out.data_ptr())
+        assert np.abs(get(out) - (b - Ap @ x)).max() <= tol * scale
+        ctx.apply_internal(0, op, precision, xd.data_ptr(), bd.data_ptr(), out.data_ptr())
+        ref = O.block_gs(Ap, bs, b, x, backward=pre == "rbgs")
+        assert np.abs(get(out) - ref).max() <= 50 * tol * np.abs(ref).max()
+        r = np.empty(n)
+        r[s] = b
+        ref = O.block_gs(Ap, bs, b, np.zeros(n), backward=pre == "rbgs")
+        assert np.abs(ctx.apply(0, N.OP_VCYCLE, r, None, n)[s] - ref).max() <= 50 * tol * np.abs(ref).max()
+        y = np.empty(n)
+        y[s] = x
+        sym = ctx.apply(0, N.OP_SYM_SPMV, y, None, n)
+        assert np.abs(sym - A @ y).max() <= 1e-13 * scale
+        ctx.close()
+
+
 @pytest.mark.gpu
 def test_gpu_jacobi_beside_class_views_keeps_its_speed():
     """Block Jacobi walks A's own rows whatever the sweeps read: in FP64, with and without class views, the same
