@@ -70,6 +70,10 @@ class Options(C.Structure):
                 ("fused_coarse", C.c_int)]
 
 
+class View(C.Structure):
+    _fields_ = [(f, C.c_int) for f in ("classes", "sweep_classes", "outer_classes", "slots", "p_lanes", "r_lanes")]
+
+
 class SolveInfo(C.Structure):
     _fields_ = [("iterations", C.c_int), ("status", C.c_int), ("normalized_residual", C.c_double),
                 ("solve_ms", C.c_double), ("learned_iterations", C.c_int), ("true_relative_residual", C.c_double)]
@@ -104,7 +108,7 @@ def load(path: str = LIB):
     lib.fhg_set_vcycle_precision.argtypes = [C.c_void_p, C.c_int]
     lib.fhg_set_cycle.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]
     lib.fhg_set_coarse_smoothing.argtypes = [C.c_void_p, C.c_int, C.c_int]
-    lib.fhg_view_info.argtypes = [C.c_void_p, C.c_int, C.c_int] + [P(C.c_int)] * 4
+    lib.fhg_view_info.argtypes = [C.c_void_p, C.c_int, C.c_int, P(View)]
     lib.fhg_set_fused_coarse.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int]
     lib.fhg_fused_coarse_info.argtypes = [C.c_void_p, C.c_int, P(C.c_int), P(C.c_int), P(C.c_int)]
     lib.fhg_device_bytes.argtypes = [C.c_void_p]
@@ -262,11 +266,11 @@ class Context:
         return first.value, ctas.value, threads.value
 
     def view_info(self, level: int, precision: str):
-        """Storage read by a V-cycle in `precision`: row classes (0: stored blocks), their slots, threads per row
-        of the sliced P and R (0: CSR)."""
-        v = [C.c_int() for _ in range(4)]
-        self._check(self.lib.fhg_view_info(self.h, level, PRECISION[precision], *map(C.byref, v)))
-        return dict(zip(("classes", "slots", "p_lanes", "r_lanes"), (q.value for q in v)))
+        """Storage that a level is read from in `precision`: row classes of its products, sweeps and outer product
+        (0: stored blocks), their slots, threads per row of the sliced P and R (0: CSR)."""
+        v = View()
+        self._check(self.lib.fhg_view_info(self.h, level, PRECISION[precision], C.byref(v)))
+        return {f: getattr(v, f) for f, _ in v._fields_}
 
     def set_fused_coarse(self, precision: str, first_level: int, cluster_ctas: int = 8, cta_threads: int = 512):
         """Run the coarse sub-cycle from first_level down as one launch (-1: launch by launch) until setup or a

@@ -74,6 +74,9 @@ struct Level {
     DevBsr<double> C64, Co64;
     DevBsr<float> C32;
     DevBsr<dfl> C2, Co2;
+    // and whether the sweeps, the products with A and the outer product read them (per precision: by rule, or chosen
+    // by timing against the stored blocks at setup)
+    bool gs_cls[3] = {true, true, true}, prod_cls[3] = {true, true, true}, outer_cls[3] = {true, true, true};
     // sliced views of the transfers, and whether the products use them (per V-cycle precision: by rule, or
     // chosen by timing at setup)
     DevBsr<double> P64s, R64s;
@@ -522,13 +525,37 @@ int upload_classes(fhg_ctx* ctx, const HostBsr& B, const RowClasses& C, const st
 }
 
 // Where rows repeat: at least kClassRows rows to a class (the dictionary is then a small part of the
-// streamed operator) and at most kMaxClasses (its FP32 form, 258 KB at 3 x 3 blocks and 6 neighbours, stays
-// in L1 and L2). The operators of a 64^3 mesh with one tensor have 77 classes, of a 4 x 4 x 4
-// checkerboard about 200; one tensor per 4^3 cubes makes 25 to 30 rows to a class, which stay with the
+// streamed operator) and at most kMaxClasses. How many there are does not show: 24^3, k = 2 takes 30 us a sweep in
+// FP32 and 48 to 50 in pairs with 77 classes (87 and 173 KB of dictionary) as with 605 (681 and 1,361 KB),
+// neighbouring rows all of different ones. The operators of a 64^3 mesh with one tensor have 77 classes, of a
+// 4 x 4 x 4 checkerboard about 200; one tensor per 4^3 cubes makes 25 to 30 rows to a class, which stay with the
 // stored-block views. Levels of at most kClassSmall rows take the view however few rows a class has: their
-// launches are bound by latency, and the lanes of the class kernels have the shortest chains (24^3 k = 2 FP32,
-// 2,376 rows: a sweep 16.8 us on padded rows).
+// launches are bound by latency, and the lanes of the class kernels have the shortest chains (672 rows of 6 x 6,
+// a class each: a sweep 14.9 -> 12.8 us in FP32, 36 -> 16 in pairs, 35 -> 21 in FP64; 3 x 3 8.8 -> 10.0, 11.4 -> 12.0,
+// 16.7 -> 15.3).
 constexpr int kClassRows = 64, kMaxClasses = 1024, kClassSmall = 8192;
+
+// Up to here the autotuner holds the stored blocks beside class views and compares them: above, the bytes decide
+// (387,072 rows of 3 x 3: a sweep 29 -> 16 us in FP32, 51 -> 26 in pairs; the autotuned stored blocks first). Below,
+// either may win: FP32 sweeps of 27,456 rows of 2 x 2 5.2 -> 6.3, of 129,376 5.9 -> 6.2, of 2,376 rows of 6 x 6 17 -> 12.
+constexpr int kCompareRows = 262144;
+
+// Without autotuning: the FP32 sweeps of 2 x 2 blocks stay on stored blocks (row-major) between these rows, where a
+// row's 16 multiply-adds are too few to pay for a scattered dictionary: 6,816 rows 5.5 us, on classes 6.0, 27,456
+// 5.6 and 6.3; 61,920 6.1 and 5.7, and every other block size is as fast or faster on classes.
+bool stored_sweeps(int bs, int rows) { return bs == 2 && rows >= 4096 && rows < 49152; }
+
+// And the outer product of rows with more than four neighbours: a thread per row of a class view is then one chain of
+// 7 blocks, stored blocks give a row eight lanes. us, stored -> classes: pairs 3 x 3 5,760 rows 4.6 -> 7.3,
+// 47,616 6.2 -> 8.6, 93,600 9.4 -> 10.2, 387,072 39 -> 24; 6 x 6 5,760 10.3 -> 10.3, 47,616 18.1 -> 16.4; FP64
+// 3 x 3 5,760 5.2 -> 7.6, 19,872 11.5 -> 7.6; 6 x 6 5,760 12.4 -> 19.7, 11,400 17.7 -> 19.9, 19,872 27 -> 20. With
+// four neighbours classes win or lose 0.3 us in pairs; FP64 1,680 rows of 4 x 4 6.0 -> 8.7, 6,816 8.1 -> 8.8, 27,456 20 -> 9.
+bool stored_outer(const HostBsr& B, bool pair)
+{
+    const bool many = B.nnzb() > 5LL * B.nbr;
+    if (pair) return many && B.bs <= 4 && B.nbr < 131072;
+    return B.nbr < (many ? 14336 : 6144);
+}
 
 // Row-class views of B in FP64, FP32 (d32, nullable) and pairs; inv: the inverted diagonal blocks or null.
 int build_class_views(fhg_ctx* ctx, const HostBsr& B, const double* inv, DevBsr<double>& d64, DevBsr<float>* d32,
@@ -658,6 +685,9 @@ template <> struct LevelVecs<double> {
     static double* k(Level& L, int i) { return L.kv64[i]; }
     static const BsrView<double>& gs(Level& L) { return L.C64.vals ? L.C64.v : L.A.v; }
     static const BsrView<double>& Acsr(Level& L) { return L.A.v; }
+    static const BsrView<double>* cls(Level& L) { return L.C64.vals ? &L.C64.v : nullptr; }
+    static bool stored_gs(Level&) { return false; }   // in FP64 the class views are the faster at every size
+    static bool stored_prod(Level&) { return false; }
 };
 template <> struct LevelVecs<float> {
     static constexpr int kPrec = FHG_PREC_FP32;
@@ -667,7 +697,7 @@ template <> struct LevelVecs<float> {
     // products with A: the row-class, slot-major or row-major padded view when setup built one
     static const BsrView<float>& A(Level& L)
     {
-        if (L.C32.vals) return L.C32.v;
+        if (L.C32.vals && L.prod_cls[kPrec]) return L.C32.v;
         if (L.prod_slot[kPrec] && L.A32s.vals) return L.A32s.v;
         return L.A32p.vals ? L.A32p.v : L.A32.v;
     }
@@ -684,11 +714,15 @@ template <> struct LevelVecs<float> {
     // GS sweeps: the row-class, slot-major or padded off-diagonal view when setup built one
     static const BsrView<float>& gs(Level& L)
     {
-        if (L.C32.vals) return L.C32.v;
+        if (L.C32.vals && L.gs_cls[kPrec]) return L.C32.v;
         if (L.gs_slot[kPrec] && L.G32s.vals) return L.G32s.v;
         return L.G32.vals ? L.G32.v : L.A32.v;
     }
     static const BsrView<float>& Acsr(Level& L) { return L.A32.v; }   // Jacobi: row pointers
+    // the row-class view, and whether setup also holds the stored blocks in the form of the sweeps and products
+    static const BsrView<float>* cls(Level& L) { return L.C32.vals ? &L.C32.v : nullptr; }
+    static bool stored_gs(Level& L) { return L.G32.vals; }
+    static bool stored_prod(Level& L) { return L.A32p.vals; }
 };
 // FP32 pairs: the FP32 V-cycle's views with 8-byte pair values (FP64-class arithmetic on the FP32 pipe).
 template <> struct LevelVecs<dfl> {
@@ -698,7 +732,7 @@ template <> struct LevelVecs<dfl> {
     static dfl* r(Level& L) { return L.r2; }
     static const BsrView<dfl>& A(Level& L)
     {
-        if (L.C2.vals) return L.C2.v;
+        if (L.C2.vals && L.prod_cls[kPrec]) return L.C2.v;
         if (L.prod_slot[kPrec] && L.A2s.vals) return L.A2s.v;
         return L.A2p.vals ? L.A2p.v : L.A2.v;
     }
@@ -712,11 +746,15 @@ template <> struct LevelVecs<dfl> {
     static dfl* k(Level& L, int i) { return L.kv2[i]; }
     static const BsrView<dfl>& gs(Level& L)
     {
-        if (L.C2.vals) return L.C2.v;
+        if (L.C2.vals && L.gs_cls[kPrec]) return L.C2.v;
         if (L.gs_slot[kPrec] && L.G2s.vals) return L.G2s.v;
         return L.G2.vals ? L.G2.v : L.A2.v;
     }
     static const BsrView<dfl>& Acsr(Level& L) { return L.A2.v; }
+    // the row-class view, and whether setup also holds the stored blocks in the form of the sweeps and products
+    static const BsrView<dfl>* cls(Level& L) { return L.C2.vals ? &L.C2.v : nullptr; }
+    static bool stored_gs(Level& L) { return L.G2.vals; }
+    static bool stored_prod(Level& L) { return L.A2p.vals; }
 };
 
 // `from_zero`: x holds zeros on entry (the pre-smoothing of a V-cycle), so the first GS sweep
@@ -1019,7 +1057,7 @@ int choose_fused(fhg_ctx* ctx)
         Level& L = ctx->levels[l];
         const bool transfers = l + 1 < nlevels && !L.inject;
         for (long long v : {(long long)L.nb, (long long)L.bs, (long long)L.ncolours, V::Acsr(L).nnzb,
-                            (long long)(V::gs(L).cls != nullptr), (long long)L.gs_slot[PR], (long long)L.prod_slot[PR],
+                            (long long)(V::gs(L).cls != nullptr), (long long)(V::A(L).cls != nullptr), (long long)L.gs_slot[PR], (long long)L.prod_slot[PR],
                             (long long)(transfers && V::P(L).sell_perm), (long long)(transfers && V::R(L).sell_perm)})
             key.sig.push_back(v);
     }
@@ -1100,6 +1138,17 @@ void release_unused_views(fhg_ctx* ctx)
 {
     for (int l = 0; l + 1 < ctx->nlevels; l++) {
         Level& L = ctx->levels[l];
+        // stored blocks beside class views that serve the sweeps, the products
+        auto drop = [&](const auto& cls, bool use, auto& row, auto& slot) {
+            if (cls.vals && use) {
+                if (row.vals) release_bsr(ctx, row);
+                if (slot.vals) release_bsr(ctx, slot);
+            }
+        };
+        drop(L.C32, L.gs_cls[FHG_PREC_FP32], L.G32, L.G32s);
+        drop(L.C32, L.prod_cls[FHG_PREC_FP32], L.A32p, L.A32s);
+        drop(L.C2, L.gs_cls[FHG_PREC_DF], L.G2, L.G2s);
+        drop(L.C2, L.prod_cls[FHG_PREC_DF], L.A2p, L.A2s);
         if (L.G32s.vals && L.gs_slot[FHG_PREC_FP32]) release_bsr(ctx, L.G32);
         else if (L.G32s.vals) release_bsr(ctx, L.G32s);
         if (L.A32s.vals && L.prod_slot[FHG_PREC_FP32]) release_bsr(ctx, L.A32p);
@@ -1116,7 +1165,15 @@ void release_unused_views(fhg_ctx* ctx)
         if (L.R2s.vals && !L.r_sell[FHG_PREC_DF]) release_bsr(ctx, L.R2s);
     }
     Level& L0 = ctx->levels[0];
-    if (L0.Ahat2s.vals && L0.outer_slot && L0.ahat_lo) {
+    if (L0.Co2.vals && L0.outer_cls[FHG_PREC_DF]) {
+        if (L0.Ahat2s.vals) release_bsr(ctx, L0.Ahat2s);
+        if (L0.ahat_lo) {
+            dfree(ctx, L0.Ahat_hi.vals);
+            dfree(ctx, L0.ahat_lo);
+        }
+        L0.Ahat_hi = DevBsr<float>();
+        L0.ahat_lo = nullptr;
+    } else if (L0.Ahat2s.vals && L0.outer_slot && L0.ahat_lo) {
         dfree(ctx, L0.Ahat_hi.vals);
         dfree(ctx, L0.ahat_lo);
         L0.Ahat_hi = DevBsr<float>();
@@ -1264,7 +1321,7 @@ double* part(fhg_ctx* ctx, int i) { return ctx->partials + (size_t)i * fhg::kRed
 // The FP64 outer operator Â: its row-class view, else CSR with the tuned lanes.
 BsrView<double> outer_operator(const Level& L)
 {
-    if (L.Co64.vals) return L.Co64.v;
+    if (L.Co64.vals && L.outer_cls[FHG_PREC_FP64]) return L.Co64.v;
     BsrView<double> Ah = L.ahat_is_a ? L.A.v : L.Ahat.v;
     if (L.outer_lanes) Ah.lanes = L.outer_lanes;
     return Ah;
@@ -1277,7 +1334,7 @@ void outer_product_df(fhg_ctx* ctx, const float* dh, const float* dl, const floa
                       float* Adl, double* partials)
 {
     Level& L0 = ctx->levels[0];
-    if (L0.Co2.vals)
+    if (L0.Co2.vals && L0.outer_cls[FHG_PREC_DF])
         fhg::launch_spmv_dots_df_slot(L0.Co2.v, dh, dl, rh, rl, Adh, Adl, partials, ctx->stream);
     else if (L0.Ahat2s.vals && (L0.outer_slot || !L0.ahat_lo))
         fhg::launch_spmv_dots_df_slot(L0.Ahat2s.v, dh, dl, rh, rl, Adh, Adl, partials, ctx->stream);
@@ -1500,14 +1557,14 @@ struct TuneKey {
 };
 struct TuneShapes {
     int a_lanes, a_unroll, gs_lanes, gs_unroll, p_lanes, p_unroll, r_lanes, r_unroll;
-    bool prod_slot, gs_slot;
+    bool prod_slot, gs_slot, prod_cls, gs_cls;
     bool p_sell = false, r_sell = false;
 };
 std::mutex g_tune_mutex;
 std::map<TuneKey, TuneShapes> g_tune_cache;
 struct OuterChoice {
     int lanes, df_lanes;
-    bool slot;
+    bool slot, cls, df_cls;
 };
 std::map<std::vector<long long>, OuterChoice> g_outer_cache;   // the outer operator's, per structure
 
@@ -1526,17 +1583,22 @@ int tune_level(fhg_ctx* ctx, int l)
     const bool ps0 = L.prod_slot[PR], gs0 = L.gs_slot[PR];
     L.prod_slot[PR] = false;
     L.gs_slot[PR] = false;
-    BsrView<T>& A = const_cast<BsrView<T>&>(V::A(L));
+    L.prod_cls[PR] = !V::stored_prod(L);
+    L.gs_cls[PR] = !V::stored_gs(L);
+    const BsrView<T>& A = V::A(L);
     TuneKey key{PR, L.bs, L.nb, L.ncolours, V::gs(L).ell, A.ell, coarsest ? 0 : V::Pcsr(L).nbr,
-                coarsest ? 0 : V::Rcsr(L).nbr, A.cls ? 1 : 0, A.nnzb, coarsest ? 0 : V::Pcsr(L).nnzb};
+                coarsest ? 0 : V::Rcsr(L).nbr, (A.cls ? 1 : 0) + (V::cls(L) ? 2 : 0), A.nnzb, coarsest ? 0 : V::Pcsr(L).nnzb};
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
             const TuneShapes& t = it->second;
-            A.lanes = t.a_lanes;
-            A.unroll = t.a_unroll;
+            BsrView<T>& Ar = const_cast<BsrView<T>&>(A);   // the row-major view, where there is one
+            Ar.lanes = t.a_lanes;
+            Ar.unroll = t.a_unroll;
             L.prod_slot[PR] = t.prod_slot;
+            L.prod_cls[PR] = t.prod_cls;
+            L.gs_cls[PR] = t.gs_cls;
             L.gs_lanes[PR] = t.gs_lanes;
             L.gs_unroll[PR] = t.gs_unroll;
             L.gs_slot[PR] = t.gs_slot;
@@ -1555,11 +1617,8 @@ int tune_level(fhg_ctx* ctx, int l)
     L.gs_slot[PR] = gs0;
     int rc = tune_level_uncached<T>(ctx, l);
     if (rc) return rc;
-    const bool ps = L.prod_slot[PR];
-    L.prod_slot[PR] = false;
-    const BsrView<T>& Ar = V::A(L);
-    TuneShapes t{Ar.lanes, Ar.unroll, L.gs_lanes[PR], L.gs_unroll[PR], 0, 1, 0, 1, ps, L.gs_slot[PR]};
-    L.prod_slot[PR] = ps;
+    TuneShapes t{A.lanes, A.unroll, L.gs_lanes[PR], L.gs_unroll[PR], 0, 1, 0, 1, L.prod_slot[PR], L.gs_slot[PR],
+                 L.prod_cls[PR], L.gs_cls[PR]};
     if (!coarsest) {
         t.p_lanes = V::Pcsr(L).lanes; t.p_unroll = V::Pcsr(L).unroll;
         t.r_lanes = V::Rcsr(L).lanes; t.r_unroll = V::Rcsr(L).unroll;
@@ -1584,8 +1643,13 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
     // against it.
     const bool forced_prod_slot = L.prod_slot[V::kPrec];
     L.prod_slot[V::kPrec] = false;
+    // Row-class views have no launch shape to choose; where the stored blocks are held beside them, the shapes of
+    // those first, then the better of the two.
+    const BsrView<T>* cls = V::cls(L);
+    L.prod_cls[V::kPrec] = !V::stored_prod(L);
+    L.gs_cls[V::kPrec] = !V::stored_gs(L);
     BsrView<T>& A = const_cast<BsrView<T>&>(V::A(L));
-    const bool classes = A.cls != nullptr;   // row-class views have no launch shape to choose
+    const bool classes = A.cls != nullptr;
     float row_prod_ms = 0.f;
     int rc = classes ? FHG_OK : tune(ctx, bs, A.lanes, A.unroll, [&](int G, int U) {
         BsrView<T> v = A; v.lanes = G; v.unroll = U;
@@ -1603,7 +1667,14 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
                                 &slot_ms);
             if (rc) return rc;
             L.prod_slot[V::kPrec] = slot_ms < row_prod_ms;
+            row_prod_ms = std::min(row_prod_ms, slot_ms);
         }
+    }
+    if (cls && !classes) {
+        float cls_ms = 0.f;
+        rc = time_candidate(ctx, [&]() { fhg::launch_spmv<T>(*cls, fhg::kSpmvResidual, V::x(L), V::b(L), V::r(L), s); }, &cls_ms);
+        if (rc) return rc;
+        L.prod_cls[V::kPrec] = cls_ms <= row_prod_ms;
     }
     if (l < ctx->nlevels - 1) {
         Level& C = ctx->levels[l + 1];
@@ -1614,14 +1685,15 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
         const bool forced_slot = L.gs_slot[PR];
         L.gs_slot[PR] = false;
         float row_ms = 0.f;
+        const bool gs_classes = V::gs(L).cls != nullptr;
         if (V::gs(L).ell > 0) { g = V::gs(L).lanes; gu = 1; }
-        rc = classes ? FHG_OK : tune(ctx, bs, g, gu, [&](int G, int U) {
+        rc = gs_classes ? FHG_OK : tune(ctx, bs, g, gu, [&](int G, int U) {
             BsrView<T> v = V::gs(L); v.lanes = G; v.unroll = U;
             for (int c = 0; c < L.ncolours; c++)
                 fhg::launch_gs<T>(v, L.colour_start[c], L.colour_start[c + 1], V::dinv(L), L.nb, V::b(L), V::x(L), s);
         }, &row_ms);
         if (rc) return rc;
-        if (!classes) {
+        if (!gs_classes) {
             L.gs_lanes[PR] = g;
             L.gs_unroll[PR] = gu;
         }
@@ -1639,7 +1711,17 @@ int tune_level_uncached(fhg_ctx* ctx, int l)
                 }, &slot_ms);
                 if (rc) return rc;
                 L.gs_slot[PR] = slot_ms < row_ms;
+                row_ms = std::min(row_ms, slot_ms);
             }
+        }
+        if (cls && !gs_classes) {
+            float cls_ms = 0.f;
+            rc = time_candidate(ctx, [&]() {
+                for (int c = 0; c < L.ncolours; c++)
+                    fhg::launch_gs<T>(*cls, L.colour_start[c], L.colour_start[c + 1], V::dinv(L), L.nb, V::b(L), V::x(L), s);
+            }, &cls_ms);
+            if (rc) return rc;
+            L.gs_cls[PR] = cls_ms <= row_ms;
         }
         if (L.inject) return FHG_OK;   // the natural injection has no launch shape
         BsrView<T>& P = const_cast<BsrView<T>&>(V::Pcsr(L));
@@ -1729,6 +1811,7 @@ void reset_device_state(Level& L)
     for (int i = 0; i < 3; i++) { L.p_sell[i] = false; L.r_sell[i] = false; }
     L.dinv2 = nullptr;
     L.x2 = L.b2 = L.r2 = nullptr;
+    for (int i = 0; i < 3; i++) { L.gs_cls[i] = L.prod_cls[i] = L.outer_cls[i] = true; }
     for (int i = 0; i < 3; i++) { L.gs_slot[i] = false; L.prod_slot[i] = false; L.gs_lanes[i] = 0; L.gs_unroll[i] = 1; }
     L.Ahat_hi = DevBsr<float>();
     L.Ahat2s = DevBsr<dfl>();
@@ -2222,21 +2305,25 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                 (rc = build_class_views(ctx, Ap, inv.data(), L.C64, &L.C32, L.C2)))
                 return rc;
         }
-        // The row- and slot-major views of stored blocks: not beside class views.
+        // The row- and slot-major views of stored blocks: instead of class views, or beside them for the autotuner to
+        // compare (up to kCompareRows rows), or for the FP32 sweeps where those are the faster (stored_sweeps).
         const bool classes = L.C64.vals != nullptr;
+        const bool stored = !classes || (o.autotune && L.nb <= kCompareRows);
         // slot-major views (GS sweeps and products): when forced, or for the autotuner to compare
-        const bool want_slot = o.colouring && !classes && (o.gs_layout == FHG_GS_SLOT || (o.gs_layout == FHG_GS_AUTO && o.autotune));
+        const bool want_slot = o.colouring && stored && (o.gs_layout == FHG_GS_SLOT || (o.gs_layout == FHG_GS_AUTO && o.autotune));
         if (fp32 && l < nlevels - 1) {
-            if (o.colouring && !classes && (rc = upload_padded(ctx, Ap, L.G32, true, 8))) return rc;
-            if (!classes && (rc = upload_padded(ctx, Ap, L.A32p, false, 8))) return rc;
+            const bool sweeps = stored || stored_sweeps(L.bs, L.nb);
+            if (o.colouring && sweeps && (rc = upload_padded(ctx, Ap, L.G32, true, 8))) return rc;
+            if (stored && (rc = upload_padded(ctx, Ap, L.A32p, false, 8))) return rc;
             if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G32s))) return rc;
             if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A32s))) return rc;
             L.gs_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.G32s.vals;
             L.prod_slot[FHG_PREC_FP32] = o.gs_layout == FHG_GS_SLOT && L.A32s.vals;
+            L.gs_cls[FHG_PREC_FP32] = !(L.G32.vals && stored_sweeps(L.bs, L.nb));
         }
         if (pair && l < nlevels - 1) {
-            if (o.colouring && !classes && (rc = upload_padded(ctx, Ap, L.G2, true, 8))) return rc;
-            if (!classes && (rc = upload_padded(ctx, Ap, L.A2p, false, 8))) return rc;
+            if (o.colouring && stored && (rc = upload_padded(ctx, Ap, L.G2, true, 8))) return rc;
+            if (stored && (rc = upload_padded(ctx, Ap, L.A2p, false, 8))) return rc;
             if (want_slot && (rc = upload_offdiag_slot_major(ctx, Ap, L.colour_start, L.G2s))) return rc;
             if (want_slot && (rc = upload_slot_major_all(ctx, Ap, L.A2s))) return rc;
             L.gs_slot[FHG_PREC_DF] = o.gs_layout == FHG_GS_SLOT && L.G2s.vals;
@@ -2308,12 +2395,23 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                 csr_to_bsr(S, L.bs, Sb);
                 permute_bsr(Sb, L.perm, iperm[0], Sp);
                 if (L.C64.vals && (rc = build_class_views(ctx, Sp, nullptr, L.Co64, nullptr, L.Co2))) return rc;
-                if (!L.Co64.vals && (rc = upload_bsr<double>(ctx, Sp, L.Ahat, nullptr))) return rc;
-                if (split && !L.Co64.vals && (rc = upload_bsr_split(ctx, Sp, L.Ahat_hi, &L.ahat_lo, L.Ahat))) return rc;
-                if (split && !L.Co64.vals && (rc = upload_slot_major_all(ctx, Sp, L.Ahat2s))) return rc;
+                const bool stored = !L.Co64.vals || (o.autotune && L.nb <= kCompareRows);
+                if ((stored || stored_outer(Sp, false) || (split && stored_outer(Sp, true))) &&
+                    (rc = upload_bsr<double>(ctx, Sp, L.Ahat, nullptr)))
+                    return rc;
+                if (split && (stored || stored_outer(Sp, true)) &&
+                    ((rc = upload_bsr_split(ctx, Sp, L.Ahat_hi, &L.ahat_lo, L.Ahat)) || (rc = upload_slot_major_all(ctx, Sp, L.Ahat2s))))
+                    return rc;
+                L.outer_cls[FHG_PREC_FP64] = !stored_outer(Sp, false);
+                L.outer_cls[FHG_PREC_DF] = !stored_outer(Sp, true);
             } else if (L.C64.vals) {   // Â = A: its views
                 L.Co64 = L.C64;
                 L.Co2 = L.C2;
+                if (split && (stored_outer(Ap, true) || (o.autotune && L.nb <= kCompareRows)) &&
+                    ((rc = upload_bsr_split(ctx, Ap, L.Ahat_hi, &L.ahat_lo, L.A)) || (rc = upload_slot_major_all(ctx, Ap, L.Ahat2s))))
+                    return rc;
+                L.outer_cls[FHG_PREC_FP64] = !stored_outer(Ap, false);
+                L.outer_cls[FHG_PREC_DF] = !stored_outer(Ap, true);
             } else if (split) {
                 if ((rc = upload_bsr_split(ctx, Ap, L.Ahat_hi, &L.ahat_lo, L.A))) return rc;
                 if ((rc = upload_slot_major_all(ctx, Ap, L.Ahat2s))) return rc;
@@ -2388,8 +2486,9 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
         BsrView<double>& Ah = L0.ahat_is_a ? L0.A.v : L0.Ahat.v;
         // the outer operator's choices, kept per structure like the levels' shapes
         const std::vector<long long> okey = {L0.bs, L0.nb, (long long)Ah.nnzb, L0.ahat_is_a ? 1 : 0,
-                                             L0.ahat_lo ? 1 : 0, L0.Ahat2s.vals ? 1 : 0, o.gs_layout};
-        bool cached = L0.Co64.vals != nullptr;   // a row-class view has no launch shape
+                                             L0.ahat_lo ? 1 : 0, L0.Ahat2s.vals ? 1 : 0, o.gs_layout, L0.Co64.vals ? 1 : 0};
+        // a row-class view has no launch shape: only compared where the stored blocks are held too
+        bool cached = L0.Co64.vals && L0.nb > kCompareRows;
         if (!cached && o.gs_layout == FHG_GS_AUTO) {
             std::lock_guard<std::mutex> lock(g_tune_mutex);
             auto it = g_outer_cache.find(okey);
@@ -2397,18 +2496,29 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                 L0.outer_lanes = it->second.lanes;
                 if (L0.ahat_lo) L0.Ahat_hi.v.lanes = it->second.df_lanes;
                 L0.outer_slot = it->second.slot;
+                L0.outer_cls[FHG_PREC_FP64] = it->second.cls;
+                L0.outer_cls[FHG_PREC_DF] = it->second.df_cls;
                 cached = true;
             }
         }
         if (!cached) {
             int g = Ah.lanes, gu = 1;
+            float fp64_ms = 0.f;
             CK(cudaMemsetAsync(ctx->kz[0], 0, sizeof(double) * L0.n, ctx->stream));
             if ((rc = tune(ctx, 9, g, gu, [&](int G, int) {
                      BsrView<double> v = Ah; v.lanes = G;
                      fhg::launch_spmv_dots(v, ctx->kz[0], ctx->kz[0], ctx->kAd[0], part(ctx, 5), ctx->stream);
-                 })))
+                 }, &fp64_ms)))
                 return rc;
             L0.outer_lanes = g;
+            if (L0.Co64.vals) {
+                float cls_ms = 0.f;
+                if ((rc = time_candidate(ctx, [&]() {
+                         fhg::launch_spmv_dots(L0.Co64.v, ctx->kz[0], ctx->kz[0], ctx->kAd[0], part(ctx, 5), ctx->stream);
+                     }, &cls_ms)))
+                    return rc;
+                L0.outer_cls[FHG_PREC_FP64] = cls_ms <= fp64_ms;
+            }
             if (L0.ahat_lo) {
                 int gd = g, gdu = 1;
                 const long long n = L0.n;
@@ -2430,12 +2540,24 @@ int fhg_setup(fhg_ctx* ctx, int nlevels, const fhg_options* opts)
                          }, &slot_ms)))
                         return rc;
                     L0.outer_slot = slot_ms < row_ms;
+                    row_ms = std::min(row_ms, slot_ms);
+                }
+                if (L0.Co2.vals) {
+                    float cls_ms = 0.f;
+                    if ((rc = time_candidate(ctx, [&]() {
+                             fhg::launch_spmv_dots_df_slot(L0.Co2.v, pair_hi(ctx->kz[0]), pair_lo(ctx->kz[0], n),
+                                                           pair_hi(ctx->kz[0]), pair_lo(ctx->kz[0], n), pair_hi(ctx->kAd[0]),
+                                                           pair_lo(ctx->kAd[0], n), part(ctx, 5), ctx->stream);
+                         }, &cls_ms)))
+                        return rc;
+                    L0.outer_cls[FHG_PREC_DF] = cls_ms <= row_ms;
                 }
                 L0.Ahat_hi.v.lanes = gd;
             }
             if (o.gs_layout == FHG_GS_AUTO) {
                 std::lock_guard<std::mutex> lock(g_tune_mutex);
-                g_outer_cache[okey] = OuterChoice{L0.outer_lanes, L0.ahat_lo ? L0.Ahat_hi.v.lanes : 0, L0.outer_slot};
+                g_outer_cache[okey] = OuterChoice{L0.outer_lanes, L0.ahat_lo ? L0.Ahat_hi.v.lanes : 0, L0.outer_slot,
+                                                  L0.outer_cls[FHG_PREC_FP64], L0.outer_cls[FHG_PREC_DF]};
             }
         }
     }
@@ -2813,22 +2935,28 @@ int fhg_fused_coarse_info(const fhg_ctx* ctx, int precision, int* first_level, i
     return FHG_OK;
 }
 
-int fhg_view_info(const fhg_ctx* ctx, int level, int precision, int* classes, int* slots, int* p_lanes, int* r_lanes)
+int fhg_view_info(const fhg_ctx* ctx, int level, int precision, fhg_view* view)
 {
-    if (!ctx || !ctx->ready || level < 0 || level >= ctx->nlevels || precision < 0 || precision > 2) return FHG_ERR_INVALID_ARG;
+    if (!ctx || !ctx->ready || level < 0 || level >= ctx->nlevels || precision < 0 || precision > 2 || !view)
+        return FHG_ERR_INVALID_ARG;
     Level& L = const_cast<Level&>(ctx->levels[level]);
+    auto classes = [](const auto& A) { return A.cls ? (int)A.ld : 0; };
     auto info = [&](auto t) {
         using V = LevelVecs<decltype(t)>;
-        const auto& A = V::gs(L);
         const bool transfers = level + 1 < ctx->nlevels && !L.inject;
-        if (classes) *classes = A.cls ? (int)A.ld : 0;
-        if (slots) *slots = A.cls ? A.ell : 0;
-        if (p_lanes) *p_lanes = transfers && V::P(L).sell_perm ? V::P(L).sell_lanes : 0;
-        if (r_lanes) *r_lanes = transfers && V::R(L).sell_perm ? V::R(L).sell_lanes : 0;
+        const auto* C = V::cls(L);
+        view->classes = classes(V::A(L));
+        view->sweep_classes = classes(V::gs(L));
+        view->slots = C ? C->ell : 0;
+        view->p_lanes = transfers && V::P(L).sell_perm ? V::P(L).sell_lanes : 0;
+        view->r_lanes = transfers && V::R(L).sell_perm ? V::R(L).sell_lanes : 0;
     };
     if (precision == FHG_PREC_FP32) info(float());
     else if (precision == FHG_PREC_DF) info(dfl());
     else info(double());
+    view->outer_classes = 0;
+    if (precision == FHG_PREC_FP64) view->outer_classes = level == 0 ? classes(outer_operator(L)) : 0;
+    else if (level == 0 && L.Co2.vals && L.outer_cls[FHG_PREC_DF]) view->outer_classes = classes(L.Co2.v);
     return FHG_OK;
 }
 

@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_bsr_residual_dinv_slot(int nbr,
 constexpr int kClsThreads = 128;
 
 // CTAs per SM of a class kernel: 64, 80 or 128 registers, what W x BS gathered values in flight and
-// 2 BS sums take without spills.
+// 2 BS sums take (FP32 6 x 6 spills up to 40 bytes of 80 registers).
 template <class T, int BS, int W>
 constexpr int kClsBlocks = BS <= 3 ? 8 : sizeof(T) == 4 ? 6 : 4;
 

@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(kReduceThreads, 2) k_bsr_spmv_dots_df_slot(int
 // The outer products on the row-class view of Â (fhg_bsr_kernels.cuh): one thread per block row over the
 // fixed grid, the values from the class dictionary. In pairs the 64^3, k = 1 product is bound by its FP32
 // pair arithmetic (13 instructions a term) instead of the 1.6 GB of stored pairs.
+// The FP64 form of 3 x 3 blocks with six slots spills 64 bytes at its 64 registers.
 template <int BS, int W>
 __global__ void __launch_bounds__(kReduceThreads, BS <= 3 ? 4 : 2) k_bsr_spmv_dots_df_cls(int nbr, const unsigned short* __restrict__ cls,
                                                                          const int* __restrict__ colidx,

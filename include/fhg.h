@@ -244,10 +244,13 @@ int fhg_level_info(const fhg_ctx* ctx, int level, int* n_block_rows, long long* 
  * cluster and the threads of each CTA. Any pointer may be NULL. No counterpart in the reference. */
 int fhg_fused_coarse_info(const fhg_ctx* ctx, int precision, int* first_level, int* cluster_ctas,
                           int* cta_threads);
-/* The storage that a V-cycle in `precision` reads on a level: the row classes of its sweeps and products (0: stored
- * blocks) and their off-diagonal slots, and the threads per row of the sliced transfers to the next level (0: CSR or
- * none). Any pointer may be NULL. */
-int fhg_view_info(const fhg_ctx* ctx, int level, int precision, int* classes, int* slots, int* p_lanes, int* r_lanes);
+/* The storage that a level is read from in one precision: the row classes of its products with A, of its sweeps and
+ * (level 0; FP32: the pair product it shares with DF) of the outer product, 0 where those run on stored blocks; the
+ * classes' off-diagonal slots; the threads per row of the sliced transfers to the next level (0: CSR or none). */
+typedef struct {
+    int classes, sweep_classes, outer_classes, slots, p_lanes, r_lanes;
+} fhg_view;
+int fhg_view_info(const fhg_ctx* ctx, int level, int precision, fhg_view* view);
 /* Run the coarse sub-cycle of one precision (FP32 or DF) as one cluster launch of cluster_ctas (8, 16) CTAs of
  * cta_threads (512, 1024) threads from first_level (>= 1) down, or launch by launch (-1), in place of what setup
  * chose; holds until setup or a change of the cycle chooses again. FHG_ERR_UNSUPPORTED where it cannot run. */
@@ -398,8 +401,8 @@ void fhg_post_destroy(fhg_post* post);
  * order their contributions are added. fhg_cond_run condenses and assembles on the device and
  * returns the number of stored entries; fhg_cond_result gives device pointers to the scalar CSR
  * (rows face block * face DOFs + a: rowptr, colidx, vals) and b, valid until the next run or destroy,
- * in the layout fhg_set_level takes. Every row is written by one thread in a fixed order (the result
- * is bitwise reproducible). No counterpart in the reference's API: it replaces the host assembly. */
+ * in the layout fhg_set_level takes. Every entry is written once, its contributions added in a fixed order (the
+ * result is bitwise reproducible). No counterpart in the reference's API: it replaces the host assembly. */
 typedef struct fhg_cond fhg_cond;
 int fhg_cond_create(fhg_cond** cond, int device, int dim, int n_elements, int n_classes, int n_cell,
                     int n_face_dofs, int n_face_blocks, const int* elem_class, const int* elem_faces,

@@ -256,3 +256,76 @@ def test_gpu_jacobi_beside_class_views_keeps_its_speed():
         c.close()
     assert np.linalg.norm(out[0] - out[1]) <= 1e-13 * np.linalg.norm(out[1])
     assert ms[0] <= 1.3 * ms[1]
+
+
+def _two_levels(A, bs):
+    """A over a coarsest level of one block: sizes and storage of level 0 alone matter."""
+    n = A.shape[0]
+    P = sp.csr_matrix((np.ones(n), (np.arange(n), np.tile(np.arange(bs), n // bs))), shape=(n, bs))
+    return [A, sp.identity(bs, format="csr")], [P]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,n,k,sweeps,outer_df,outer_fp64", [
+    (2, 30, 1, True, True, False), (2, 40, 1, False, True, False), (2, 96, 1, False, True, True), (2, 144, 1, True, True, True),
+    (2, 96, 2, True, True, True), (3, 8, 1, True, False, False), (3, 20, 1, True, False, True), (3, 24, 1, True, True, True),
+    (3, 8, 2, True, True, False), (3, 12, 2, True, True, True)])
+def test_gpu_stored_blocks_serve_where_they_are_faster(dim, n, k, sweeps, outer_df, outer_fp64):
+    """Without autotuning: the FP32 sweeps of 2 x 2 blocks between 4,096 and 49,152 rows and the outer products of
+    small levels run on stored blocks beside the class views; everything else on classes. Outer products and sweeps
+    on either against the operator and the oracle."""
+    torch = pytest.importorskip("torch")
+    from fhhos4_gb300 import _native as N
+    from fhhos4_gb300 import solver as S
+    from test_gpu_parity import scalar_perm
+    H = hho.Hierarchy(dim, n, k, max_levels=1)
+    A, bs = H.A(0).tocsr(), H.block_size
+    H.close()
+    As, Ps = _two_levels(A, bs)
+    ctx = S.fcg_mg(As, Ps, bs, precision="fp32", extra=["df"]).Context()
+    f32, df, f64 = (ctx.view_info(0, p) for p in ("fp32", "df", "fp64"))
+    assert f32["classes"] > 0 and df["classes"] > 0 and f64["classes"] > 0
+    assert (f32["sweep_classes"] > 0) == sweeps and df["sweep_classes"] > 0 and f64["sweep_classes"] > 0
+    assert (f32["outer_classes"] > 0) == outer_df and (df["outer_classes"] > 0) == outer_df
+    assert (f64["outer_classes"] > 0) == outer_fp64
+    rng = np.random.default_rng(4)
+    y, b = rng.standard_normal((2, A.shape[0]))
+    scale = abs(A).sum(axis=1).max() * np.abs(y).max()
+    assert np.abs(ctx.apply(0, N.OP_SYM_SPMV, y, None, len(y)) - A @ y).max() <= 1e-13 * scale
+    s = scalar_perm(ctx.permutation(0, A.shape[0] // bs), bs)
+    Ap = O.as_csr(A[s][:, s])
+    xd, bd = (torch.tensor(v[s].astype(np.float32), device="cuda") for v in (y, b))
+    out = torch.empty_like(xd)
+    torch.cuda.synchronize()
+    ctx.apply_internal(0, N.OP_GS_FORWARD, "fp32", xd.data_ptr(), bd.data_ptr(), out.data_ptr())
+    ref = O.block_gs(Ap, bs, bd.cpu().numpy().astype(np.float64), xd.cpu().numpy().astype(np.float64))
+    assert np.abs(out.cpu().numpy() - ref).max() <= 50 * PREC["fp32"][1] * np.abs(ref).max()
+    ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,n,k", [(3, 8, 1), (3, 8, 2), (2, 96, 1)])
+def test_gpu_autotuning_compares_class_views_with_stored_blocks(dim, n, k):
+    """With autotuning no use of a level is slower than on stored blocks alone (within 25%, of launches of 4 to 20 us;
+    the outer product of 8^3 took 1.7 to 2 times as long on classes), and the second context of a structure takes the
+    same forms."""
+    from fhhos4_gb300 import _native as N
+    from fhhos4_gb300 import solver as S
+    H = hho.Hierarchy(dim, n, k, max_levels=1)
+    A, bs = H.A(0).tocsr(), H.block_size
+    H.close()
+    As, Ps = _two_levels(A, bs)
+    noisy = A.copy()
+    noisy.data = noisy.data * (1.0 + 1e-13 * np.random.default_rng(8).integers(0, 64, A.nnz))
+    for precision in ("fp32", "df", "fp64"):
+        kw = dict(precision=precision, autotune=True, fused=False)
+        a = S.fcg_mg(As, Ps, bs, **kw).Context()
+        again = S.fcg_mg(As, Ps, bs, **kw).Context()
+        stored = S.fcg_mg([noisy, As[1]], Ps, bs, **kw).Context()
+        assert stored.view_info(0, precision)["classes"] == 0 and a.view_info(0, precision) == again.view_info(0, precision)
+        assert a.view_info(0, precision)["slots"] > 0
+        for op in (N.OP_GS_FORWARD, N.OP_RESIDUAL, N.OP_SYM_SPMV):
+            ms = [min(c.time_op(0, op, precision, 10, 50) for _ in range(6)) for c in (a, stored)]
+            assert ms[0] <= 1.25 * ms[1], (precision, op, ms)
+        for c in (a, again, stored):
+            c.close()
