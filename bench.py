@@ -511,14 +511,20 @@ def run_ours(args, dist: Dist):
 
     # outer FCG operator: double-FP32 (values as FP32 pairs, d as an FP32 pair, r.d, d.Ad; the product
     # of both the FP32 and the FP64-class methods) and native FP64
-    outer_bytes = bytes_spmv(nnzb0, nb0, n0, n0, bs, 8) + n0 * 8 * 2   # + d (own rows) and r for the dots
-    add_kernel("bsr_outer_dots_fp64", N.OP_SYM_SPMV, "df", outer_bytes)
-    add_kernel("bsr_outer_dots_fp64_native", N.OP_SYM_SPMV, "fp64", outer_bytes)
+    # Where block rows repeat, a product reads a 16-bit class and `slots` columns per row instead of the blocks
+    # (their dictionary stays in cache); otherwise the stored blocks, columns and row pointers.
+    def a_bytes(prec, p, use="classes"):
+        view = ctx.view_info(0, prec)
+        return nb0 * (2 + 4 * view["slots"]) + 2 * n0 * p if view[use] else bytes_spmv(nnzb0, nb0, n0, n0, bs, p)
+
+    add_kernel("bsr_outer_dots_fp64", N.OP_SYM_SPMV, "df", a_bytes("df", 8, "outer_classes") + n0 * 8 * 2)   # + d and r for the dots
+    add_kernel("bsr_outer_dots_fp64_native", N.OP_SYM_SPMV, "fp64", a_bytes("fp64", 8, "outer_classes") + n0 * 8 * 2)
     # FP64 operators: "fp64" = the FP64-class pair kernels the plain method runs (8-byte values);
     # "fp64_native" = the same products in native FP64 arithmetic
     for name, prec, p in (("fp32", "fp32", p32), ("fp64", "df", p64), ("fp64_native", "fp64", p64)):
-        add_kernel(f"bsr_spmv_{name}", N.OP_SPMV, prec, bytes_spmv(nnzb0, nb0, n0, n0, bs, p))
-        gs_bytes = bytes_spmv(nnzb0, nb0, n0, n0, bs, p) + nb0 * bs * bs * p + n0 * p   # + D^-1 + b
+        add_kernel(f"bsr_spmv_{name}", N.OP_SPMV, prec, a_bytes(prec, p))
+        # + b, and D^-1 where it is not a part of the dictionary
+        gs_bytes = a_bytes(prec, p, "sweep_classes") + n0 * p + (0 if ctx.view_info(0, prec)["sweep_classes"] else nb0 * bs * bs * p)
         add_kernel(f"bsr_gs_sweep_{name}", N.OP_GS_FORWARD, prec, gs_bytes)
         if info1:
             pb = info0["p_blocks"]
@@ -538,26 +544,21 @@ def run_ours(args, dist: Dist):
     # Dominant kernel of the headline (FP32 V-cycle) solve: GS sweeps on level 0.
     ncol = info0["colours"]
     gs_min_bytes = (nnzb0 - nb0) * (bs * bs * p32 + 4) + nb0 * bs * bs * p32 + 3 * n0 * p32
-    class_bytes = nb0 * (2 + 4 * 6) + 3 * n0 * p32
+    view = ctx.view_info(0, "fp32")
     dom = "bsr_gs_sweep_fp32"
     hbm, hbm_kind = measured_hbm_peak()
-    traffic = committed_traffic().get(dom)
+    # the committed capture is of the sweep over stored blocks
+    form = f"row classes ({view['sweep_classes']}, {view['slots']} slots)" if view["sweep_classes"] else "stored blocks"
+    traffic = None if view["sweep_classes"] else committed_traffic().get(dom)
     ach = kernels[dom]["gbs"]
-    roofline = {"bound": "hbm", "kernel": dom, "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s",
+    roofline = {"bound": "hbm", "kernel": dom, "form": form, "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s",
                 "frac": round(ach / hbm, 4), "peak_kind": f"of {hbm_kind}",
                 "traffic": traffic,
                 "algorithmic_bytes_per_launch": kernels[dom]["bytes"] / max(ncol, 1),
                 "launches_per_sweep": ncol,
-                # The sweep's own minimum: off-diagonal blocks with their column indices, D^-1, b,
-                # x read once and written once (the formula above also counts the diagonal blocks
-                # and row pointers, which the sweep does not read).
-                "min_bytes_per_launch": gs_min_bytes / max(ncol, 1),
-                "frac_min_bytes": round(gs_min_bytes / (kernels[dom]["ms"] * 1e-3) / 1e9 / hbm, 4),
-                # Where block rows repeat, the sweep reads a 16-bit class and 6 columns per row instead of
-                # the blocks, so the byte counts above (and the captured traffic, of the stored-block
-                # sweep) are not moved and the fractions can exceed 1. What that sweep moves at least:
-                "class_view_bytes_per_launch": class_bytes / max(ncol, 1),
-                "frac_class_view": round(class_bytes / (kernels[dom]["ms"] * 1e-3) / 1e9 / hbm, 4),
+                # What a sweep over stored blocks needs at least: off-diagonal blocks with their column
+                # indices, D^-1, b, x read once and written once.
+                "stored_block_min_bytes_per_launch": gs_min_bytes / max(ncol, 1),
                 "spmv_fp64_frac": round(kernels["bsr_spmv_fp64"]["gbs"] / hbm, 4),
         "spmv_fp64_native_frac": round(kernels["bsr_spmv_fp64_native"]["gbs"] / hbm, 4),
                 "spmv_fp32_frac": round(kernels["bsr_spmv_fp32"]["gbs"] / hbm, 4)}
