@@ -1181,6 +1181,8 @@ void release_unused_views(fhg_ctx* ctx)
     } else if (L0.Ahat2s.vals && !L0.outer_slot) {
         release_bsr(ctx, L0.Ahat2s);
     }
+    // the FP64 form of Â, whose columns the row-major pairs share
+    if (L0.Co64.vals && L0.outer_cls[FHG_PREC_FP64] && !L0.ahat_is_a && !L0.ahat_lo && L0.Ahat.vals) release_bsr(ctx, L0.Ahat);
 }
 
 // Timing at setup (launch shapes, the coarse sub-cycle) runs one context at a time, so contexts set up
