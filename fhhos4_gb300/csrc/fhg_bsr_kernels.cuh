@@ -787,7 +787,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_bsr_residual_dinv_slot(int nbr,
 // takes twice as long). The sums run over the off-diagonal blocks in column order. What bounds a sweep now
 // is the L1's rate of gathered lines (a warp's x loads of one slot touch 7 lines) and L2; FP64 stays bound
 // by its pipe. 64^3, k = 1 (3.1 M rows, 77 classes), one sweep of stored blocks against classes:
-// FP32 171 -> 73 us, pairs 326 -> 139 us, FP64 777 -> 413 us.
+// FP32 171 -> 73 us, pairs 326 -> 148 us, FP64 777 -> 413 us.
 constexpr int kClsThreads = 128;
 
 // CTAs per SM of a class kernel: 64, 80 or 128 registers, what W x BS gathered values in flight and
